@@ -1004,15 +1004,16 @@ int bx_prefill_attention(const int32_t* q, const int64_t* sh, const int64_t* pos
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return BX_ELAUNCH;
-  const int smem32 = 2 * PF_STAGE + PfCfg<32>::QTILE + PfCfg<32>::PTILE + (int)sizeof(PrefillSmall) + 1024;
-  const int smem16 = 2 * PF_STAGE + PfCfg<16>::QTILE + PfCfg<16>::PTILE + (int)sizeof(PrefillSmall) + 1024;
+  const bool exact = !ptab;
+  const int sms = device_sms();
+  if (sms <= 0) return BX_ELAUNCH;
   static PerDevice configured;
-  if (once_per_device(configured, [smem32, smem16] {
-        cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             smem32);
+  if (once_per_device(configured, [] {
+        cudaError_t e = cudaFuncSetAttribute(prefill_attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             pf_smem(true));
         return e != cudaSuccess ? e
-                                : cudaFuncSetAttribute(prefill_attention_kernel<16>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem16);
+                                : cudaFuncSetAttribute(prefill_attention_kernel<false>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(false));
       }) != BX_OK)
     return BX_ELAUNCH;
   PrefillParams p{};
@@ -1032,11 +1033,12 @@ int bx_prefill_attention(const int32_t* q, const int64_t* sh, const int64_t* pos
   p.den = (i64*)den;
   p.HKV = HKV;
   p.G = G;
-  const dim3 grid((unsigned)n_tiles, (unsigned)HKV);
-  if (tile_rows == 32)
-    prefill_attention_kernel<32><<<grid, PfCfg<32>::THREADS, smem32, (cudaStream_t)stream>>>(tm, p);
+  p.work = (int64_t)n_tiles * HKV;
+  const unsigned grid = (unsigned)(p.work < sms ? p.work : sms);       // persistent: one CTA per SM
+  if (exact)
+    prefill_attention_kernel<true><<<grid, PF_THREADS, pf_smem(true), (cudaStream_t)stream>>>(tm, p);
   else
-    prefill_attention_kernel<16><<<grid, PfCfg<16>::THREADS, smem16, (cudaStream_t)stream>>>(tm, p);
+    prefill_attention_kernel<false><<<grid, PF_THREADS, pf_smem(false), (cudaStream_t)stream>>>(tm, p);
   return launched(1);
 }
 

@@ -137,3 +137,60 @@ def test_tall_tiles_are_cut_and_empty_tile_lists_are_accepted():
     den = torch.ones(N, HKV, G, 1, dtype=torch.long, device="cuda")
     tri_prefill.attend(T(q), T(pos), T(planes), T(bt), ptab, torch.zeros(0, 3, dtype=torch.int32, device="cuda"), num, den)
     assert not bool(num.any())
+
+
+@pytest.mark.parametrize("table", ["given", "scaled", "jumps"])
+def test_exact_row_shifts_and_tables_outside_the_compact_form(table):
+    """Row shifts at and beyond the ends of the 32-bit form (0, 1, 31, 32, 62, a zero row), and tables that the 31-bit
+    copy cannot hold, take the general weight function; a whole tile of them equals the oracle."""
+    from bitexact_llm_b200.vllm_plugin import tri_prefill
+    rng = np.random.RandomState(len(table))
+    HKV, G, bs, nb, S = 2, 4, 16, 40, 150
+    planes = _cache(rng, nb, HKV, bs, 1 << 20)
+    bt, pos, req, tiles, live, N = _case(rng, [(0, S), (200, 9)], HKV, G, bs, nb, 224)
+    q = rng.randint(-(1 << 20), 1 << 20, (N, HKV, G, HD)).astype(np.int64)
+    shift = np.array([0, 1, 2, 9, 20, 30, 31, 32, 40, 62, 1 << 20], np.int64)
+    sh = -6 - shift[rng.randint(0, len(shift), (N, HKV, G))]
+    lut = ox.exp2_table().copy()
+    if table == "scaled":
+        lut = lut * 3 // 2
+    elif table == "jumps":
+        lut[rng.randint(0, len(lut), 50)] //= 3
+    num, den = tri_prefill.attend_exact(T(q, torch.int32), T(sh), T(pos), T(planes), T(bt), T(tiles), T(lut), ox.L2E28)
+    rows = np.flatnonzero(live)
+    wnum, wden = _oracle_rows(rows, q, sh, pos, req, planes, bt, lut, "exact", None)
+    assert np.array_equal(num.cpu().numpy()[rows], wnum)
+    assert np.array_equal(den.cpu().numpy()[rows].reshape(wden.shape), wden)
+
+
+@pytest.mark.parametrize("top", [1 << 22, (1 << 24) + 5])
+def test_int8_table_near_and_far_entries(top):
+    """Entries below the shared-memory copy (more than 8 under the maximum), its two widths, and a table too large for it."""
+    from bitexact_llm_b200.vllm_plugin import tri_paged, tri_prefill
+    rng = np.random.RandomState(top % 97)
+    HKV, G, bs, nb, S = 2, 4, 16, 40, 200
+    planes = _cache(rng, nb, HKV, bs, 1 << 15)
+    bt, pos, req, tiles, live, N = _case(rng, [(0, S), (3, 40)], HKV, G, bs, nb, 256)
+    q = rng.randint(-(1 << 13), 1 << 13, (N, HKV, G, HD)).astype(np.int64)
+    q[::2] >>= 3
+    ptab = np.sort(rng.randint(0, 1 << 16, 131073)).astype(np.int64)
+    ptab[-17408:] = np.sort(rng.randint(1 << 16, 1 << 22, 17408))
+    ptab[-1] = top
+    num = torch.zeros(N, HKV, G, HD, dtype=torch.long, device="cuda")
+    den = torch.ones(N, HKV, G, 1, dtype=torch.long, device="cuda")
+    tri_prefill.attend(T(q), T(pos), T(planes), T(bt), T(ptab, torch.int32), T(tiles), num, den)
+    # the same sums in int64 from the cache planes and the table
+    limbs = planes.reshape(nb, HKV, bs, 8, HD).astype(np.int64)
+    K = limbs[..., 0, :] + (limbs[..., 1, :] << 8) + (limbs[..., 2, :] << 16)
+    V = limbs[..., 3, :] + (limbs[..., 4, :] << 8) + (limbs[..., 5, :] << 16)
+    for n in np.flatnonzero(live):
+        keys = np.arange(pos[n] + 1)
+        b, o = bt[req[n], keys // bs], keys % bs
+        k, v = K[b, :, o], V[b, :, o]                                    # [keys, HKV, HD]
+        raw = np.einsum("hgd,shd->hgs", q[n], k)
+        z = ((raw - raw.max(-1, keepdims=True)) + (1 << 18)) >> 19
+        w = np.where(z >= -131072, ptab[np.maximum(z, -131072) + 131072], 0)
+        limb = ((w & 0xFFFFFF) + 0x808080 & 0xFFFFFF) ^ 0x808080         # three signed digits carry the weight into p.V
+        w3 = sum((((limb >> 8 * i) & 255) ^ 128) - 128 << 8 * i for i in range(3))
+        assert np.array_equal(den[n].cpu().numpy()[..., 0], w.sum(-1)), n
+        assert np.array_equal(num[n].cpu().numpy(), np.einsum("hgs,shd->hgd", w3, v)), n
