@@ -68,8 +68,7 @@ int launch_exact(const CUtensorMap& mw, const CUtensorMap& ma, const ExactEpiPar
     return BX_ELAUNCH;
   const int m_tiles = (ep.M + TA - 1) / TA;
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
-  exact_linear_kernel<TA><<<m_tiles * n_tiles, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mw, ma, ep, K, m_tiles);
-  return launched(1);
+  return launch_chained(exact_linear_kernel<TA>, dim3(m_tiles * n_tiles), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mw, ma, ep, K, m_tiles);
 }
 
 template <int TA>
@@ -84,20 +83,8 @@ int launch_exact_splitk(const CUtensorMap& mw, const CUtensorMap& ma, const Exac
     return BX_ELAUNCH;
   const int m_tiles = (ep.M + TA - 1) / TA;
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(m_tiles * n_tiles * split), 1, 1);
-  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = split;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, exact_linear_splitk_kernel<TA>, mw, ma, ep, K, m_tiles) != cudaSuccess) return BX_ELAUNCH;
-  return launched(1);
+  return launch_chained(exact_linear_splitk_kernel<TA>, dim3((unsigned)(m_tiles * n_tiles * split)), GEMM_THREADS, Cfg::SMEM_BYTES, st, split,
+                        mw, ma, ep, K, m_tiles);
 }
 
 // Split-K with the activation rows as the 128-row operand (exact_linear_rows_splitk_kernel).
@@ -113,21 +100,8 @@ int launch_exact_rows_splitk(const CUtensorMap& mact, const CUtensorMap& mwt, co
     return BX_ELAUNCH;
   const int w_tiles = (ep.N + TA - 1) / TA;
   const int row_blocks = (ep.M + WROWS - 1) / WROWS;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(w_tiles * row_blocks * split), 1, 1);
-  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = split;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, exact_linear_rows_splitk_kernel<TA>, mact, mwt, ep, K, w_tiles) != cudaSuccess)
-    return BX_ELAUNCH;
-  return launched(1);
+  return launch_chained(exact_linear_rows_splitk_kernel<TA>, dim3((unsigned)(w_tiles * row_blocks * split)), GEMM_THREADS, Cfg::SMEM_BYTES, st, split,
+                        mact, mwt, ep, K, w_tiles);
 }
 
 template <int TA>
@@ -146,8 +120,7 @@ int launch_exact_persistent(const CUtensorMap& mw, const CUtensorMap& ma, const 
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
   const int total = m_tiles * n_tiles;
   const int grid = total < sms ? total : sms;
-  exact_linear_persistent_kernel<TA><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mw, ma, ep, K, n_tiles, m_tiles);
-  return launched(1);
+  return launch_chained(exact_linear_persistent_kernel<TA>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mw, ma, ep, K, n_tiles, m_tiles);
 }
 
 // CTA pairs resident at a time for a pair kernel (clusters of 2 with its shared memory), cached per device.
@@ -230,8 +203,12 @@ int launch_exact_rows_one(const CUtensorMap& mact, const CUtensorMap& mwt, const
   const int w_tiles = (ep.N + TN - 1) / TN;
   const long total = (long)row_blocks * w_tiles;
   const int grid = (int)(total < sms ? total : sms);
-  exact_linear_rows_one_kernel<TN, NBUF><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mact, mwt, ep, K, row_blocks,
-                                                                                     w_tiles);
+  // Chained (launch_chained) while a CTA has a few tiles: 6451 against 6478 us for a decode step of 256 sequences (3.5 tiles per CTA);
+  // plain on long lists, where the early start buys nothing and measured 1 % (LM head of 700 rows, 81 tiles: 1522 against 1505 us).
+  if (total <= 8L * sms)
+    return launch_chained(exact_linear_rows_one_kernel<TN, NBUF>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mact, mwt, ep, K,
+                          row_blocks, w_tiles);
+  exact_linear_rows_one_kernel<TN, NBUF><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mact, mwt, ep, K, row_blocks, w_tiles);
   return launched(1);
 }
 
@@ -246,6 +223,9 @@ int launch_int8(const CUtensorMap& mw, const CUtensorMap& ma, const Int8EpiParam
     return BX_ELAUNCH;
   const int m_tiles = (ep.M + TA - 1) / TA;
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
+  // POST = false (raw products): its operands may be any tensors, so it does not start before the previous kernel has ended.
+  if (POST)
+    return launch_chained(int8_linear_kernel<TA, POST>, dim3(m_tiles * n_tiles), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mw, ma, ep, K, m_tiles);
   int8_linear_kernel<TA, POST><<<m_tiles * n_tiles, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mw, ma, ep, K, m_tiles);
   return launched(1);
 }
@@ -266,6 +246,9 @@ int launch_int8_persistent(const CUtensorMap& mw, const CUtensorMap& ma, const I
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
   const int total = m_tiles * n_tiles;
   const int grid = total < sms ? total : sms;
+  // POST = false (raw products): its operands may be any tensors, so it does not start before the previous kernel has ended.
+  if (POST)
+    return launch_chained(int8_linear_persistent_kernel<TA, POST>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mw, ma, ep, K, n_tiles, m_tiles);
   int8_linear_persistent_kernel<TA, POST><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mw, ma, ep, K, n_tiles, m_tiles);
   return launched(1);
 }
@@ -283,20 +266,8 @@ int launch_int8_splitk(const CUtensorMap& mw, const CUtensorMap& ma, const Int8E
     return BX_ELAUNCH;
   const int m_tiles = (ep.M + TA - 1) / TA;
   const int n_tiles = (ep.N + WROWS - 1) / WROWS;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(m_tiles * n_tiles * split), 1, 1);
-  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = split;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, int8_linear_splitk_kernel<TA>, mw, ma, ep, K, m_tiles) != cudaSuccess) return BX_ELAUNCH;
-  return launched(1);
+  return launch_chained(int8_linear_splitk_kernel<TA>, dim3((unsigned)(m_tiles * n_tiles * split)), GEMM_THREADS, Cfg::SMEM_BYTES, st, split,
+                        mw, ma, ep, K, m_tiles);
 }
 
 template <int TA>
@@ -641,15 +612,14 @@ int bx_exact_norm(int mode, const void* xin, const int64_t* yin, const int64_t* 
   cudaStream_t st = (cudaStream_t)stream;
   const i64* y = (const i64*)yin; const i64* id = (const i64*)ids;
 #define BX_NORM_LAUNCH(MODE, NT, EPT) \
-  norm_kernel<MODE, NT, EPT><<<M, NT, 0, st>>>(xin, y, id, (const i64*)gm, (const i64*)ge, (i64*)xo, q, (i64*)sh, a8, \
-                                              flag, M, D, lg, do_norm)
+  return launch_chained(norm_kernel<MODE, NT, EPT>, dim3(M), NT, 0, st, 0, xin, y, id, (const i64*)gm, (const i64*)ge, (i64*)xo, q, \
+                        (i64*)sh, a8, flag, M, D, lg, do_norm)
   if (D <= 2048) {                      // 512 threads x 4 elements
     if (mode == 0) BX_NORM_LAUNCH(0, 512, 4); else if (mode == 1) BX_NORM_LAUNCH(1, 512, 4); else BX_NORM_LAUNCH(2, 512, 4);
   } else {                              // 512 threads x 8 elements
     if (mode == 0) BX_NORM_LAUNCH(0, 512, 8); else if (mode == 1) BX_NORM_LAUNCH(1, 512, 8); else BX_NORM_LAUNCH(2, 512, 8);
   }
 #undef BX_NORM_LAUNCH
-  return launched(1);
 }
 
 int bx_exact_qkv(const int64_t* y, const int64_t* cos, const int64_t* sin, const int64_t* pos,
@@ -661,8 +631,7 @@ int bx_exact_qkv(const int64_t* y, const int64_t* cos, const int64_t* sin, const
   if (N == 0) return BX_OK;
   QkvParams p{(const i64*)y, (const i64*)cos, (const i64*)sin, (const i64*)pos, (const i64*)slot, cache, sc_nb, sc_h,
               sc_bs, bs, q, (i64*)sh, flag, H, HKV, HD};
-  qkv_kernel<<<dim3(N, HKV), HD / 2, 0, (cudaStream_t)stream>>>(p);
-  return launched(1);
+  return launch_chained(qkv_kernel, dim3(N, HKV), HD / 2, 0, (cudaStream_t)stream, 0, p);
 }
 
 int bx_kv_store(int8_t* cache, int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const int64_t* slot,
@@ -683,8 +652,7 @@ int bx_exact_attn_out(const int64_t* num, const int64_t* den, int32_t* q, int64_
       K2 / HD > AO_MAXH)
     return BX_EARG;
   if (N == 0) return BX_OK;
-  attn_out_kernel<<<N, AO_THREADS, 0, (cudaStream_t)stream>>>((const i64*)num, (const i64*)den, q, (i64*)sh, a8, N, K2, HD);
-  return launched(1);
+  return launch_chained(attn_out_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, (const i64*)num, (const i64*)den, q, (i64*)sh, a8, N, K2, HD);
 }
 
 int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_t* sh, int8_t* a8, int32_t* flag,
@@ -705,32 +673,16 @@ int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_
     // equal rounds: with 256 rows, 128 CTAs of two rows each rather than 148 CTAs of one or two
     const int rounds = (N + sms - 1) / sms;
     const int grid = (N + rounds - 1) / rounds;
-    silu_persistent_kernel<8><<<grid, SILU_P_THREADS, smem, st>>>((const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag,
+    return launch_chained(silu_persistent_kernel<8>, dim3(grid), SILU_P_THREADS, smem, st, 0, (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag,
                                                                   N, FF);
-    return launched(1);
   }
   if (FF == SILU_CL * SILU_CL_THREADS * 8 && N <= 4096) {          // decode batches of the 1B model: cluster form
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SILU_CL * N, 1, 1);
-    cfg.blockDim = dim3(SILU_CL_THREADS, 1, 1);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = SILU_CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, silu_cluster_kernel<8>, (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF) !=
-        cudaSuccess)
-      return BX_ELAUNCH;
-    return launched(1);
+    return launch_chained(silu_cluster_kernel<8>, dim3(SILU_CL * N), SILU_CL_THREADS, 0, st, SILU_CL, (const i64*)y, (const i64*)lut, q,
+                          (i64*)sh, a8, flag, N, FF);
   }
   const int ept = (FF + SILU_THREADS - 1) / SILU_THREADS;
-  if (ept <= 4) silu_kernel<4><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF);
-  else if (ept <= 16) silu_kernel<16><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF);
-  else silu_kernel<28><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF);
-  return launched(1);
+  return launch_chained(ept <= 4 ? silu_kernel<4> : ept <= 16 ? silu_kernel<16> : silu_kernel<28>, dim3(N), SILU_THREADS, 0, st, 0,
+                        (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF);
 }
 
 // Persistent streaming kernel (variants 5: 8 consumer warps, 6: 4 consumer warps). BX_ENOFIT: too few pairs or a
@@ -799,14 +751,8 @@ static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, con
     return BX_ELAUNCH;
   const int64_t grid = npairs < (int64_t)per_sm * 148 ? npairs : (int64_t)per_sm * 148;
   if (chunked && (size_t)grid * (size_t)spill_keys * 32 > spill_bytes) return forced ? BX_EARG : BX_ENOFIT;
-  if (NW == 8)
-    exact_attention_stream_kernel<8><<<(unsigned)grid, 320, smem, (cudaStream_t)stream>>>(tk, tv, p, ns, npairs,
-                                                                                          (i64*)spill, spill_keys);
-  else
-    exact_attention_stream_kernel<4><<<(unsigned)grid, 192, smem, (cudaStream_t)stream>>>(tk, tv, p, ns, npairs,
-                                                                                          (i64*)spill, spill_keys);
-  if (cudaGetLastError() != cudaSuccess) return BX_ELAUNCH;
-  return launched(1);
+  return launch_chained(NW == 8 ? exact_attention_stream_kernel<8> : exact_attention_stream_kernel<4>, dim3((unsigned)grid), 32 * NW + 64,
+                        (int)smem, (cudaStream_t)stream, 0, tk, tv, p, ns, npairs, (i64*)spill, spill_keys);
 }
 
 static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
@@ -910,9 +856,8 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return BX_ELAUNCH;
-    if ((kind == 4 ? cudaLaunchKernelEx(&cfg, exact_attention_tc_kernel<4>, tk, tv, p)
-                   : cudaLaunchKernelEx(&cfg, exact_attention_tc_kernel<8>, tk, tv, p)) != cudaSuccess)
-      return BX_ELAUNCH;
+    return launch_chained(kind == 4 ? exact_attention_tc_kernel<4> : exact_attention_tc_kernel<8>, cfg.gridDim, (int)cfg.blockDim.x,
+                          (int)smem, cfg.stream, cs, tk, tv, p);
   } else if (use_tma) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return BX_ELAUNCH;
@@ -1035,11 +980,8 @@ int bx_prefill_attention(const int32_t* q, const int64_t* sh, const int64_t* pos
   p.G = G;
   p.work = (int64_t)n_tiles * HKV;
   const unsigned grid = (unsigned)(p.work < sms ? p.work : sms);       // persistent: one CTA per SM
-  if (exact)
-    prefill_attention_kernel<true><<<grid, PF_THREADS, pf_smem(true), (cudaStream_t)stream>>>(tm, p);
-  else
-    prefill_attention_kernel<false><<<grid, PF_THREADS, pf_smem(false), (cudaStream_t)stream>>>(tm, p);
-  return launched(1);
+  return launch_chained(exact ? prefill_attention_kernel<true> : prefill_attention_kernel<false>, dim3(grid), PF_THREADS, pf_smem(exact),
+                        (cudaStream_t)stream, 0, tm, p);
 }
 
 int bx_int8_norm(int mode, const void* xin, const int64_t* yin, const int64_t* ids, const int64_t* gamma,
@@ -1050,10 +992,9 @@ int bx_int8_norm(int mode, const void* xin, const int64_t* yin, const int64_t* i
   if ((mode == 0 && !ids) || (mode == 1 && !yin) || (do_norm && (!gamma || !a8 || !mant || !e))) return BX_EARG;
   if (M == 0) return BX_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (mode == 0) i8::int8_norm_kernel<0><<<M, NORM_THREADS, 0, st>>>(xin, (const i64*)yin, (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant, (i64*)e, flag, M, D, do_norm);
-  else if (mode == 1) i8::int8_norm_kernel<1><<<M, NORM_THREADS, 0, st>>>(xin, (const i64*)yin, (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant, (i64*)e, flag, M, D, do_norm);
-  else i8::int8_norm_kernel<2><<<M, NORM_THREADS, 0, st>>>(xin, (const i64*)yin, (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant, (i64*)e, flag, M, D, do_norm);
-  return launched(1);
+  return launch_chained(mode == 0 ? i8::int8_norm_kernel<0> : mode == 1 ? i8::int8_norm_kernel<1> : i8::int8_norm_kernel<2>, dim3(M),
+                        NORM_THREADS, 0, st, 0, xin, (const i64*)yin, (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant,
+                        (i64*)e, flag, M, D, do_norm);
 }
 
 int bx_int8_qkv(const int64_t* y, const int64_t* cos, const int64_t* sin, const int64_t* pos, const int64_t* slot,
@@ -1065,8 +1006,7 @@ int bx_int8_qkv(const int64_t* y, const int64_t* cos, const int64_t* sin, const 
   if (N == 0) return BX_OK;
   i8::Qkv8Params p{(const i64*)y, (const i64*)cos, (const i64*)sin, (const i64*)pos, (const i64*)slot, cache, sc_nb,
                    sc_h, sc_bs, bs, (i64*)q64, q32, flag, H, HKV, HD};
-  i8::int8_qkv_kernel<<<dim3(N, HKV), HD / 2, 0, (cudaStream_t)stream>>>(p);
-  return launched(1);
+  return launch_chained(i8::int8_qkv_kernel, dim3(N, HKV), HD / 2, 0, (cudaStream_t)stream, 0, p);
 }
 
 int bx_int8_attn_out(const int64_t* num, const int64_t* den, int8_t* a8, int64_t* mant, int64_t* e, int N, int K2,
@@ -1076,8 +1016,7 @@ int bx_int8_attn_out(const int64_t* num, const int64_t* den, int8_t* a8, int64_t
       K2 / HD > AO_MAXH)
     return BX_EARG;
   if (N == 0) return BX_OK;
-  i8::int8_attn_out_kernel<<<N, AO_THREADS, 0, (cudaStream_t)stream>>>((const i64*)num, (const i64*)den, a8, (i64*)mant, (i64*)e, N, K2, HD);
-  return launched(1);
+  return launch_chained(i8::int8_attn_out_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, (const i64*)num, (const i64*)den, a8, (i64*)mant, (i64*)e, N, K2, HD);
 }
 
 int bx_int8_silu_quant(const int64_t* y, const int64_t* lut, int8_t* a8, int64_t* mant, int64_t* e, int64_t* scr,
@@ -1087,10 +1026,8 @@ int bx_int8_silu_quant(const int64_t* y, const int64_t* lut, int8_t* a8, int64_t
   if (N == 0) return BX_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const int ept = (FF + SILU_THREADS - 1) / SILU_THREADS;
-  if (ept <= 4) i8::int8_silu_kernel<4><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF);
-  else if (ept <= 16) i8::int8_silu_kernel<16><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF);
-  else i8::int8_silu_kernel<28><<<N, SILU_THREADS, 0, st>>>((const i64*)y, (const i64*)lut, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF);
-  return launched(1);
+  return launch_chained(ept <= 4 ? i8::int8_silu_kernel<4> : ept <= 16 ? i8::int8_silu_kernel<16> : i8::int8_silu_kernel<28>, dim3(N),
+                        SILU_THREADS, 0, st, 0, (const i64*)y, (const i64*)lut, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF);
 }
 
 int bx_int8_silu_prod(const int64_t* y, const int64_t* lut, int64_t* h, int64_t* rowmax, int64_t* scr, int N, int FFl,
@@ -1163,10 +1100,10 @@ static int run_sample(const int64_t* logits, int64_t ld, const int64_t* rows, co
   i64* pmax = (i64*)scratch;
   i64* pidx = pmax + (size_t)M * nch0;
   cudaStream_t st = (cudaStream_t)stream;
-  sample_part_kernel<<<dim3(nch, M), SAMPLE_THREADS, 0, st>>>((const i64*)logits, ld, (const i64*)rows, (const i64*)lnt,
-                                                              pmax, pidx, V, ch, nch, bits, (i64)voff);
-  sample_combine_kernel<<<(M + 127) / 128, 128, 0, st>>>(pmax, pidx, (i64*)tok, (i64*)omax, M, nch);
-  return launched(2);
+  const int rc = launch_chained(sample_part_kernel, dim3(nch, M), SAMPLE_THREADS, 0, st, 0, (const i64*)logits, ld, (const i64*)rows,
+                                (const i64*)lnt, pmax, pidx, V, ch, nch, bits, (i64)voff);
+  if (rc != BX_OK) return rc;
+  return launch_chained(sample_combine_kernel, dim3((M + 127) / 128), 128, 0, st, 0, pmax, pidx, (i64*)tok, (i64*)omax, M, nch);
 }
 
 int bx_sample(const int64_t* logits, int64_t ld, const int64_t* rows, const int64_t* lnt, void* scratch,

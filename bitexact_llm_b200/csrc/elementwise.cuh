@@ -9,6 +9,7 @@
 
 #include <cooperative_groups.h>
 
+#include "bx_ptx.cuh"
 #include "bx_rules.cuh"
 
 namespace bx {
@@ -131,6 +132,8 @@ norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64
     gmr[k] = (do_norm && c < D) ? __ldg(gm + c) : 0;
     ger[k] = (do_norm && c < D) ? __ldg(ge + c) : 0;
   }
+  launch_next();
+  wait_previous();
   i64 ax = 0;
 #pragma unroll
   for (int k = 0; k < EPT; ++k) {
@@ -214,6 +217,8 @@ __global__ void qkv_kernel(const QkvParams p) {
   const int G = p.H / p.HKV;
   const int dd = threadIdx.x;              // 0 .. HH-1
   const int64_t NT = (int64_t)(p.H + 2 * p.HKV) * p.HD;
+  launch_next();
+  wait_previous();
   const i64 pos = p.pos[row];
   const i64* yr = p.y + row * NT;
   // Everything the thread reads is requested before the first use: the row's q / k / v values and the slot are in
@@ -315,6 +320,8 @@ attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int32_
   const int64_t row = blockIdx.x;
   const int nh = K2 / HD;
   i64 o[AO_EPT];
+  launch_next();
+  wait_previous();
 #pragma unroll
   for (int k = 0; k < AO_EPT; ++k) {                  // the numerators are in flight while the reciprocals are made
     const int c = threadIdx.x + k * AO_THREADS;
@@ -380,6 +387,8 @@ silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int32_t* __r
   i64 P[EPT];
   i64 pmax = 0;
   bool anybad = false;
+  launch_next();
+  wait_previous();
 #pragma unroll
   for (int k = 0; k < EPT; ++k) {
     const int c = threadIdx.x + k * SILU_THREADS;
@@ -428,6 +437,8 @@ silu_cluster_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int3
   i64 P[EPT];
   i64 pmax = 0;
   bool anybad = false;
+  launch_next();
+  wait_previous();
 #pragma unroll
   for (int k = 0; k < EPT; ++k) {
     const int c = c0 + threadIdx.x + k * SILU_CL_THREADS;
@@ -471,6 +482,8 @@ silu_persistent_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, i
   __shared__ i64 red[33];
   for (int i = threadIdx.x; i < SILU_TABLE; i += SILU_P_THREADS) tab[i] = __ldg(lut + i);
   __syncthreads();
+  launch_next();
+  wait_previous();                                       // the table is no other kernel's work, the rows are
   const int64_t plane = (int64_t)M * FF;
   bool anybad = false;
   for (int64_t row = blockIdx.x; row < M; row += gridDim.x) {

@@ -34,6 +34,7 @@ template <int TA>
 struct ExactSplitEpi {
   using Params = ExactEpiParams;
   static constexpr int NW = 3, NA = 3, RMAX = 2, NS = (TA + 31) / 32;
+  static constexpr bool WEIGHTS_STACKED = false;                      // the weights are the 128-row operand
   struct Consts {
     int n, d, cnt, wcnt;
     bool nok;
@@ -144,6 +145,7 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
+  if (dead) wait_previous();
   bool acc_ok = false;                                                // epilogue warps: accumulators complete
   typename Epi::Consts cst = {};                                     // epilogue threads: loaded before the wait
 
@@ -152,7 +154,22 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
+      // The first stages' weights are on their way before the previous kernel has ended, their activations after it.
+      const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      for (int i = 0; i < pre; ++i) {
+        uint8_t* st = ring + i * Cfg::STAGE_BYTES;
+        mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);
+        if (Epi::WEIGHTS_STACKED) tma_load_3d(st + Cfg::W_BYTES, &tmap_a, &sh->full[i], (kb0 + i) * BKB, m0, 0);
+        else tma_load_3d(st, &tmap_w, &sh->full[i], (kb0 + i) * BKB, n0, 0);
+      }
+      wait_previous();
+      for (int i = 0; i < pre; ++i) {
+        uint8_t* st = ring + i * Cfg::STAGE_BYTES;
+        if (Epi::WEIGHTS_STACKED) tma_load_3d(st, &tmap_w, &sh->full[i], (kb0 + i) * BKB, n0, 0);
+        else tma_load_3d(st + Cfg::W_BYTES, &tmap_a, &sh->full[i], (kb0 + i) * BKB, m0, 0);
+      }
+      issued = pre;
+      for (int i = pre; i < nkb && ok; ++i) {
         const int s = i % Cfg::STAGES;
         const int round = i / Cfg::STAGES;
         if (round > 0) ok = mbar_wait(&sh->empty[s], (round - 1) & 1);
@@ -173,6 +190,7 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
   } else if (warp == 1) {
     if (lane == 0 && !dead) {
       // ---- MMA issue (as limb_gemm_tile) ----
+      wait_previous();
       constexpr uint32_t ID_ALL = umma_idesc_i8(NA * TA);
       constexpr uint32_t ID_ONE = umma_idesc_i8(TA);
       constexpr uint32_t ID_REST = umma_idesc_i8(NA > 1 ? (NA - 1) * TA : TA);
@@ -214,6 +232,7 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
   } else {
     // ---- epilogue warps: what does not depend on the accumulators (per-row constants, lists, row scales) is loaded
     //      first; at decode sizes this kernel is a latency chain ----
+    wait_previous();
     cst = Epi::load(n0, m0, warp & 3, (warp - 2) >> 2, lane, rank, S, ep);
     // ---- epilogue warps: wait for this CTA's accumulators ----
     bool ok = !dead;
@@ -289,6 +308,7 @@ template <int TA>
 struct ExactRowsSplitEpi {
   using Params = ExactEpiParams;
   static constexpr int NW = 3, NA = 3, NS = (TA + 31) / 32;
+  static constexpr bool WEIGHTS_STACKED = true;
   struct Consts {
     int m;                                                            // this lane's activation row
     bool mok;

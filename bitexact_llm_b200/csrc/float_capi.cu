@@ -42,28 +42,6 @@ bool make_map_bf16(CUtensorMap* m, const void* base, i64 K, i64 rows, i64 planes
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launch with the permission to start before the previous kernel of the stream has ended (every kernel launched this way
-// calls wait_previous before it touches dependent memory).
-template <class... P, class... A>
-int launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, int cluster, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 0 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) return BX_ELAUNCH;
-  return launched(1);
-}
-
 struct Operands {
   const void *w, *x;
   i64 ldw, gsw, ldx, gsx;

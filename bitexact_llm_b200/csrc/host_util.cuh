@@ -30,6 +30,28 @@ inline int launched(int n) {
   return BX_OK;
 }
 
+// Launch with the permission to start before the previous kernel of the stream has ended (every kernel launched this way
+// calls wait_previous before it touches dependent memory).
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) return BX_ELAUNCH;
+  return launched(1);
+}
+
 // Kernel attributes (opt-in dynamic shared memory) and device properties are per device: every cache of them is
 // indexed by the ordinal of the current device. The flags are atomics so that concurrent first calls from several
 // host threads are well defined (they would store the same value).

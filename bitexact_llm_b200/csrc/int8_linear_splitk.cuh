@@ -15,6 +15,7 @@ template <int TA>
 struct Int8SplitEpi {
   using Params = Int8EpiParams;
   static constexpr int NW = 1, NA = 2, NS = (TA + 31) / 32;
+  static constexpr bool WEIGHTS_STACKED = false;
   struct Consts {
     int n;
     bool nok;

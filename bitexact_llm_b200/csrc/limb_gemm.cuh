@@ -79,7 +79,10 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
     tma_prefetch_desc(tmap_a);
   }
   __syncthreads();
-  if (sh->abort_flag) return;
+  if (sh->abort_flag) {
+    wait_previous();
+    return;
+  }
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, Cfg::TMEM_COLS);
     tmem_relinquish();
@@ -94,7 +97,17 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
+      // The first stages' weights are on their way before the previous kernel has ended, their activations after it.
+      const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      for (int i = 0; i < pre; ++i) {
+        mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);
+        tma_load_3d(ring + i * Cfg::STAGE_BYTES, tmap_w, &sh->full[i], (kb0 + i) * BKB, n0, 0);
+      }
+      wait_previous();
+      for (int i = 0; i < pre; ++i)
+        tma_load_3d(ring + i * Cfg::STAGE_BYTES + Cfg::W_BYTES, tmap_a, &sh->full[i], (kb0 + i) * BKB, m0, 0);
+      issued = pre;
+      for (int i = pre; i < nkb && ok; ++i) {
         const int s = i % Cfg::STAGES;
         const int round = i / Cfg::STAGES;
         if (round > 0) ok = mbar_wait(&sh->empty[s], (round - 1) & 1);
@@ -115,7 +128,8 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      // ---- MMA issue ----
+      // ---- MMA issue ---- (no bounded wait begins before the previous kernel has ended)
+      wait_previous();
       constexpr uint32_t ID_ALL = umma_idesc_i8(NA * TA);
       constexpr uint32_t ID_ONE = umma_idesc_i8(TA);
       constexpr uint32_t ID_REST = umma_idesc_i8(NA > 1 ? (NA - 1) * TA : TA);
@@ -157,6 +171,7 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
     }
   } else {
     // ---- epilogue warps: row constants and L1 prefetches first, they overlap the main loop ----
+    wait_previous();
     const typename Epi::Row row = Epi::load_row(warp & 3, (warp - 2) >> 2, lane, n0, m0, ep);
     Epi::prefetch(row, (warp - 2) >> 2, lane, m0, ep);
     bool ok = true;
@@ -229,7 +244,10 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
     tma_prefetch_desc(tmap_a);
   }
   __syncthreads();
-  if (sh->abort_flag) return;
+  if (sh->abort_flag) {
+    wait_previous();
+    return;
+  }
   if (warp == 1) {
     tmem_alloc(&sh->tmem_base, TCOLS);
     tmem_relinquish();
@@ -244,9 +262,26 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
       // ---- TMA producer: one continuous stream of stages over all tiles of this CTA ----
       int it = 0;            // global stage counter
       bool ok = true;
+      // The first tile's first stages: the weights (the 128-row operand, with W_FASTEST the stacked one) are on their way
+      // before the previous kernel has ended, the activations after it.
+      const int pre = blockIdx.x >= total ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      for (int i = 0; i < pre; ++i) {
+        uint8_t* st = ring + i * Cfg::STAGE_BYTES;
+        mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);
+        if (W_FASTEST) tma_load_3d(st + Cfg::W_BYTES, tmap_a, &sh->full[i], i * BKB, a_origin(blockIdx.x), 0);
+        else tma_load_3d(st, tmap_w, &sh->full[i], i * BKB, w_origin(blockIdx.x), 0);
+      }
+      wait_previous();
+      for (int i = 0; i < pre; ++i) {
+        uint8_t* st = ring + i * Cfg::STAGE_BYTES;
+        if (W_FASTEST) tma_load_3d(st, tmap_w, &sh->full[i], i * BKB, w_origin(blockIdx.x), 0);
+        else tma_load_3d(st + Cfg::W_BYTES, tmap_a, &sh->full[i], i * BKB, a_origin(blockIdx.x), 0);
+      }
       for (int tile = blockIdx.x; tile < total && ok; tile += gridDim.x) {
         const int n0 = w_origin(tile), m0 = a_origin(tile);
-        for (int i = 0; i < nkb && ok; ++i, ++it) {
+        const int first = tile == (int)blockIdx.x ? pre : 0;
+        it += first;
+        for (int i = first; i < nkb && ok; ++i, ++it) {
           const int s = it % Cfg::STAGES, round = it / Cfg::STAGES;
           if (round > 0) ok = mbar_wait(&sh->empty[s], (round - 1) & 1);
           if (!ok) break;
@@ -265,7 +300,8 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      // ---- MMA issue ----
+      // ---- MMA issue ---- (no bounded wait begins before the previous kernel has ended)
+      wait_previous();
       constexpr uint32_t ID_ALL = umma_idesc_i8(NA * TA);
       constexpr uint32_t ID_ONE = umma_idesc_i8(TA);
       constexpr uint32_t ID_REST = umma_idesc_i8(NA > 1 ? (NA - 1) * TA : TA);
@@ -313,6 +349,7 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
     }
   } else {
     // ---- epilogue warps ----
+    wait_previous();
     int tcount = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++tcount) {

@@ -670,17 +670,6 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const int h = (int)(pz % p.HKV);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  i64 kend = 0;
-  for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[r * p.M + g] + 1);
-  kend = imin(kend, (i64)p.nblk * p.bs);
-  const i64 per = (kend + CS - 1) / CS;
-  i64 chunk = (per + KEYS - 1) / KEYS * KEYS;
-  if (chunk > p.chunk_cap) chunk = p.chunk_cap;
-  const i64 lo = imin((i64)rank * chunk, kend);
-  const i64 hi = imin(lo + chunk, kend);
-  const int nst = (int)((hi - lo + KEYS - 1) / KEYS);
-  const i64 brow = p.rmap ? p.rmap[r] : r;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < ATT3_NS; ++s) {
       mbar_init(&sm->full[s], 1);
@@ -697,6 +686,18 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     tmem_alloc(&sm->tmem_base, ATT3_TMEM_COLS);
     tmem_relinquish();
   }
+  wait_previous();
+  i64 kend = 0;
+  for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[r * p.M + g] + 1);
+  kend = imin(kend, (i64)p.nblk * p.bs);
+  const i64 per = (kend + CS - 1) / CS;
+  i64 chunk = (per + KEYS - 1) / KEYS * KEYS;
+  if (chunk > p.chunk_cap) chunk = p.chunk_cap;
+  const i64 lo = imin((i64)rank * chunk, kend);
+  const i64 hi = imin(lo + chunk, kend);
+  const int nst = (int)((hi - lo + KEYS - 1) / KEYS);
+  const i64 brow = p.rmap ? p.rmap[r] : r;
+
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1079,6 +1080,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     tma_prefetch_desc(&tmap_v);
   }
   for (int i = threadIdx.x; i < ATT6_MAXGROUPS; i += blockDim.x) sm->ptag[i] = 0;
+  wait_previous();
   if (ranked) {
     // Requests by context length, longest first, in buckets of 128 keys (ties by index): a counting sort whose
     // placement step runs in one warp over 32 requests at a time (match_any gives each lane its place among the lanes

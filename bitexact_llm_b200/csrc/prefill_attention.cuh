@@ -155,6 +155,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
 
   if (warp == PF_WARPS) {
     // ---------------- producer warp ----------------
+    wait_previous();
     const int pages = PF_KEYS / p.bs;                  // pages per block, one per lane
     int slot = 0, round = 0, issued = 0;
     uint32_t k = 0;
@@ -221,6 +222,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
     }
   } else if (warp == PF_WARPS + 1) {
     // ---------------- MMA warp: one thread ----------------
+    wait_previous();
     if (lane == 0) {
       constexpr uint32_t ID_ALL = umma_idesc_i8(3 * PF_ROWS), ID_ONE = umma_idesc_i8(PF_ROWS), ID_TWO = umma_idesc_i8(2 * PF_ROWS);
       constexpr uint32_t ID_PV = umma_idesc_i8_amn(3 * PF_ROWS);
@@ -337,6 +339,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
         fits &= check_exp2_table(table, tid, 32 * PF_WARPS) && p.w.l2e >= (1ll << 28) && p.w.l2e < (1ll << 29);
       }
       if (!fits) sm->bad_table = 1;
+      wait_previous();                                   // the table is no other kernel's work, the queries are
       if (ok && blockIdx.x < p.work) {
         ok = mbar_wait(&sm->info_full[0], 0);
         if (ok) write_q(load_q(sm->tile[0]));
