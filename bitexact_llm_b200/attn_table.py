@@ -1,0 +1,92 @@
+"""Compact weight tables of the decode attention kernels, made once per engine from the engine's own table.
+
+An attention weight is round(2^top 2^-t) with 2^-t from a 131 KB table with interpolation (exact mode) or an entry of a
+524 KB table of e^z (int8 mode). The kernels gather from neither: a CTA keeps 4097 entries of 2^-f (16 KB) in shared
+memory, from which a weight is known to within a small window, and goes to the full table only where a rounding boundary
+lies in the window. The window is a property of the full table, worked out here over all of its entries; a table that
+such a form cannot stand for gets none (None), and the kernels then read the full table for every weight.
+
+compact = (int32 tensor of the entries, window, slack, factor from a row distance to t, its left shift, 2^(top + 1)):
+window in units
+of the interpolated entry, slack (for a table that was itself rounded) in units of 2^-32 of a weight."""
+
+import ctypes
+
+import torch
+
+T_BITS, W_BITS = 26, 31                # fractional bits of t, bits of an entry
+STEP = 1 << 14                         # t steps per segment: 4096 segments
+
+
+class Native(ctypes.Structure):
+    """bx_compact_table of include/bitexact_b200.h."""
+    _fields_ = [("tab", ctypes.c_void_p)] + [(n, ctypes.c_uint32) for n in ("window", "slack", "factor", "mtop")] + [("shift", ctypes.c_int)]
+
+
+def native(compact):
+    tab, window, slack, factor, shift, mtop = compact
+    return Native(tab.data_ptr(), window, slack, factor, mtop, shift)
+
+
+def to(compact, device):
+    return None if compact is None else (compact[0].to(device), *compact[1:])
+
+
+def _walk(tab, t):
+    """The kernel's w for t (int64 tensors): the interpolated entry below the true value by at most the window."""
+    idx, rr = (t & ((1 << T_BITS) - 1)) >> 14, t & (STEP - 1)
+    a, b = tab[idx], tab[idx + 1]
+    return a - (((a - b) * rr) >> 14)
+
+
+def _fits(tab):
+    return bool((tab >= 1).all()) and bool((tab < 1 << 32).all()) and bool((tab[:-1] >= tab[1:]).all())
+
+
+def exact(lut, l2e):
+    """From the 2^-f table (int64 [16385] at 2^60, linear between the entries) and l2e = round(log2(e) 2^28)."""
+    v = lut.detach().cpu().long()
+    if v.shape != (16385,) or not (1 << 28) <= int(l2e) < (1 << 29) or int(v.min()) < 1 << 30 or int(v.max()) > 1 << 60:
+        return None
+    a = v[::4] >> (60 - W_BITS)
+    i = torch.arange(16384)
+    k, rr = i >> 2, (i & 3) << 12
+    off = v[:-1] - ((a[k] << 29) - (a[k] - a[k + 1]) * (rr << 15))       # 2^29 times the distance to the straight line
+    lo, hi = int(off.min() >> 29), int(-((-off.max()) >> 29))
+    tab = a + (lo - 2)                 # one for the floor of the kernel's product, one for the rounding of the table's rule
+    if not _fits(tab) or hi - lo > 60:
+        return None
+    return tab.to(torch.int32), hi - lo + 3, 0, int(l2e) * 8, 1, 1 << 23
+
+
+def int8(ptab):
+    """From the weight table (int32 [131073], entry 131072 - u is the weight u steps of 2^-12 below the maximum). Every
+    entry is compared with what the kernel makes of the compact form."""
+    from .exact.consts import exp2_table
+    p = ptab.detach().cpu().long()
+    if p.shape != (131073,) or int(p[0]) != 0 or not 1 <= int(p[-1]) <= 1 << 22 or int(p[-1]) & (int(p[-1]) - 1):
+        return None
+    mtop = 2 * int(p[-1])              # 2^(32 - 31) p[-1]: w mtop 2^-n is the weight at 32 fractional bits
+    factor = 3098164009                # round(log2(e) 2^31)
+    u = torch.arange(131072)
+    t = _mulhi_round(u << 15, factor)
+    n = t >> T_BITS
+    m = torch.where(n < 32, mtop >> n.clamp(max=31), torch.zeros_like(n))
+    want = p[131072 - u]
+    a = exp2_table("cpu").long()[::4] >> (60 - W_BITS)
+    slack = 1 << 21                    # the e^z table has 10 bits more than the weights: its own rounding
+    for window in (12, 16, 24, 32):
+        tab = a - window // 2 - 4
+        if not _fits(tab):
+            return None
+        r = _walk(tab, t) * m + (1 << 31) - slack
+        sure = (r & 0xFFFFFFFF) + window * m + 2 * slack < 1 << 32
+        if bool(((r >> 32) == want)[sure].all()):
+            return tab.to(torch.int32), window, slack, factor, 15, mtop
+    return None
+
+
+def _mulhi_round(x, k):
+    """(x k + 2^31) >> 32 for 0 <= x, k < 2^32 in int64."""
+    lo = x * (k & 0xFFFF) + (1 << 31)              # below 2^49
+    return (x * (k >> 16) + (lo >> 16)) >> 16

@@ -112,4 +112,39 @@ __device__ __forceinline__ uint32_t int8_weight(i64 zz, bool live, const uint8_t
 // The three signed base-256 digits of 0 <= v < 2^23 as the bytes of one word.
 __device__ __forceinline__ uint32_t limb_bytes(uint32_t v) { return (v + 0x808080u) ^ 0x808080u; }
 
+// The decode kernels' form: 4097 entries (16 KB, two to four CTAs share an SM) prepared by the caller from its table, with
+// what that form cannot say (bitexact_llm_b200/attn_table.py works both out over all entries of the full table). The
+// weight at t = factor (zz >> c) lies in [w, w + window] mtop 2^-n of the interpolated entry w, give or take `slack`, all
+// in units of 2^-32; `unsure` where a rounding boundary lies in that range.
+// Cost in cycles of a scheduler, measured: a gather from the 131 KB table 32 and an L2 round trip, the whole of this about
+// 45, of which the two 32-bit gathers from shared memory take 14.
+struct CompactTable {
+  const uint32_t* tab;          // null: none
+  uint32_t window, slack, factor, mtop;
+  int shift;
+};
+constexpr int CT_N = 4097;
+constexpr int CT_BYTES = 16400;
+
+__device__ __forceinline__ void fill_compact(uint32_t* dst, const CompactTable& ct, int tid, int n) {
+  if (ct.tab)
+    for (int i = tid; i < CT_N; i += n) dst[i] = __ldg(ct.tab + i);
+}
+// hs: a distance with hi >> hs != 0 is out of range (weight 0).
+__device__ __forceinline__ uint32_t compact_weight(const CompactTable& ct, const uint32_t* tab, i64 zz, int c, int hs, bool live,
+                                                   bool& unsure) {
+  const uint32_t lo = (uint32_t)zz, hi = (uint32_t)((u64)zz >> 32);
+  const uint32_t zf = __funnelshift_r(lo, hi, c) << ct.shift;
+  const uint32_t t = (uint32_t)(((u64)zf * ct.factor + (1ull << 31)) >> 32);
+  const uint32_t n = (t >> FT2) + (hi >> hs) * 32u;
+  const uint32_t* e = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(tab) + ((t >> 12) & 0x3ffcu));
+  const uint32_t a = e[0];
+  const uint32_t w = a - __umulhi(a - e[1], t << 18);
+  const uint32_t m = live ? shr_clamp(ct.mtop, n) : 0u;
+  const u64 r = (u64)w * m + ((1ull << 31) - ct.slack);
+  const uint32_t rl = (uint32_t)r;
+  unsure = live && rl + (m * ct.window + 2u * ct.slack) < rl;
+  return (uint32_t)(r >> 32);
+}
+
 }  // namespace bx

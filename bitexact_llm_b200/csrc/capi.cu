@@ -694,7 +694,7 @@ static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, con
                                 int64_t nb, int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt,
                                 int bt_is_int64, int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut,
                                 int64_t l2e, const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M,
-                                int min_per_sm, void* spill, size_t spill_bytes, void* stream) {
+                                CompactTable ct, int min_per_sm, void* spill, size_t spill_bytes, void* stream) {
   const bool forced = min_per_sm == 0;                          // an explicit variant: any fit will do
   const int KEYS = 8 * NW, STAGE = KEYS * 256;
   const int64_t max_keys = (int64_t)nblk * bs;
@@ -710,19 +710,27 @@ static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, con
 #endif
   const int64_t cap = chunked ? BX_ATT_CHUNK : (max_keys + KEYS - 1) / KEYS * KEYS;     // chunks: a multiple of 32 NW keys
   if (cap / 32 > ATT6_MAXGROUPS) return forced ? BX_EARG : BX_ENOFIT;
-  const int64_t fixed = 1024 + cap * 32 + (int64_t)sizeof(Attn6Small) + 1024 /* request order */;
+  int64_t fixed = 1024 + cap * 32 + (int64_t)sizeof(Attn6Small) + 1024 /* request order */;
   int per_sm = NW == 4 ? 4 : 2, ns = 0;
+  auto stages = [&](int64_t used) { return (int)((227 * 1024 / per_sm - 1024 - used) / STAGE); };
   for (; per_sm >= 1; --per_sm) {                               // most CTAs per SM that still leave a ring of 4 stages
-    const int64_t budget = 227 * 1024 / per_sm - 1024;
-    ns = (int)((budget - fixed) / STAGE);
+    ns = stages(fixed);
     if (ns >= 4 || (per_sm == 1 && ns >= 3)) break;
+  }
+  // The compact weight table where it costs neither a CTA nor the ring: 256 sequences of 512 .. 768 keys 155 -> 133 us; a
+  // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %.
+  if (ct.tab && per_sm >= 1 && stages(fixed + CT_BYTES) >= 4) {
+    fixed += CT_BYTES;
+    ns = stages(fixed);
+  } else {
+    ct = CompactTable{};
   }
   if (per_sm < 1) return forced ? BX_EARG : BX_ENOFIT;
   if (!forced && per_sm < min_per_sm) return BX_ENOFIT;
   if (ns > ATT6_MAXNS) ns = ATT6_MAXNS;
   const size_t smem = (size_t)fixed + (size_t)ns * STAGE;
   AttnParams p{q, (const i64*)sh, (const i64*)qpos, cache, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, (int)cap, ptab};
+               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, (int)cap, ptab, ct};
   static PerDevice configured;
   if (once_per_device(configured, [] {
         cudaError_t e = cudaFuncSetAttribute(exact_attention_stream_kernel<8>,
@@ -759,7 +767,8 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
                          int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
                          int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e,
                          const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M, int HD,
-                         int cluster_size, int variant, void* spill, size_t spill_bytes, void* stream) {
+                         int cluster_size, int variant, const CompactTable& ct, void* spill, size_t spill_bytes,
+                         void* stream) {
   if (!q || !qpos || !cache || !bt || !num || !den) return BX_EARG;
   if (!ptab && (!sh || !lut)) return BX_EARG;
   if (R < 0 || HKV <= 0 || M < 1 || M > 4 || HD != ATT_HD || bs <= 0 || nblk <= 0 || nb <= 0) return BX_EARG;
@@ -779,19 +788,21 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
     const int tries[3][2] = {{4, 4}, {8, 2}, {4, 2}};
     for (int t = 0; t < 3; ++t) {
       const int rc = run_attention_stream(tries[t][0], q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64,
-                                          sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, tries[t][1], nullptr, 0,
+                                          sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, tries[t][1], nullptr, 0,
                                           stream);
       if (rc != BX_ENOFIT) return rc;
     }
-    if (spill) {                                                // long contexts: chunks of 512 keys, scores in scratch
-      const int rc = run_attention_stream(4, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-                                          rmap, lut, l2e, ptab, num, den, R, HKV, M, 3, spill, spill_bytes, stream);
+    // Long contexts: chunks of 512 keys, scores in scratch. Two 8-warp CTAs per SM: against three or four of 4 warps 204 : 271 us
+    // (40 sequences of 64 .. 8192 keys), 136 : 149 us (64 of 16 .. 4096), 366 : 386 us (100 of 64 .. 8192).
+    if (spill) {
+      const int rc = run_attention_stream(8, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
+                                          rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, 2, spill, spill_bytes, stream);
       if (rc != BX_ENOFIT) return rc;
     }
   }
   if (variant == 5 || variant == 6)
     return run_attention_stream(variant == 5 ? 8 : 4, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64,
-                                sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, 0, spill, spill_bytes, stream);
+                                sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, 0, spill, spill_bytes, stream);
   // 1 direct loads, 2 TMA-staged, 3 TMA + tcgen05 p.V with 8 consumer warps, 4 the same with 4 consumer warps
   const int kind = variant != 0 ? variant : (tma_ok ? ((bs <= 32 && (int64_t)R * HKV >= 64) ? 4 : 3) : 1);
   const int nw = kind == 4 ? 4 : 8;
@@ -815,7 +826,7 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
   if (chunk_cap > cap_limit) return BX_EARG;
   const size_t smem = (size_t)fixed + (size_t)chunk_cap * 32;
   AttnParams p{q, (const i64*)sh, (const i64*)qpos, cache, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, chunk_cap, ptab};
+               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, chunk_cap, ptab, CompactTable{}};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((int64_t)cs * R * HKV), 1, 1);
   cfg.blockDim = dim3(kind == 4 ? 160 : use_tma ? ATT2_THREADS : ATT_THREADS, 1, 1);
@@ -884,7 +895,7 @@ int bx_exact_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos,
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!sh || !lut) return BX_EARG;
   return run_attention(q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
-                       nullptr, num, den, R, HKV, M, HD, cluster_size, variant, nullptr, 0, stream);
+                       nullptr, num, den, R, HKV, M, HD, cluster_size, variant, CompactTable{}, nullptr, 0, stream);
 }
 
 size_t bx_attention_scratch_bytes(int nblk, int bs) {
@@ -901,7 +912,7 @@ int bx_exact_attention_ws(const int32_t* q, const int64_t* sh, const int64_t* qp
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!sh || !lut) return BX_EARG;
   return run_attention(q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
-                       nullptr, num, den, R, HKV, M, HD, cluster_size, variant, scratch, scratch_bytes, stream);
+                       nullptr, num, den, R, HKV, M, HD, cluster_size, variant, CompactTable{}, scratch, scratch_bytes, stream);
 }
 
 int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* cache, int64_t nb, int64_t sc_nb,
@@ -911,7 +922,7 @@ int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* ca
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!ptab) return BX_EARG;
   return run_attention(q, nullptr, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, nullptr,
-                       0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, scratch, scratch_bytes, stream);
+                       0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, CompactTable{}, scratch, scratch_bytes, stream);
 }
 
 int bx_int8_attention(const int32_t* q, const int64_t* qpos, const int8_t* cache, int64_t nb, int64_t sc_nb,
@@ -921,7 +932,31 @@ int bx_int8_attention(const int32_t* q, const int64_t* qpos, const int8_t* cache
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!ptab) return BX_EARG;
   return run_attention(q, nullptr, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, nullptr,
-                       0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, nullptr, 0, stream);
+                       0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, CompactTable{}, nullptr, 0, stream);
+}
+
+int bx_exact_attention_tab(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
+                           int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
+                           int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e, int64_t* num,
+                           int64_t* den, int R, int HKV, int M, int HD, int cluster_size, int variant, void* scratch,
+                           size_t scratch_bytes, const bx_compact_table* compact, void* stream) {
+  if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
+  if (!sh || !lut || !compact) return BX_EARG;
+  const CompactTable ct{compact->tab, compact->window, compact->slack, compact->factor, compact->mtop, compact->shift};
+  return run_attention(q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
+                       nullptr, num, den, R, HKV, M, HD, cluster_size, variant, ct, scratch, scratch_bytes, stream);
+}
+
+int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* cache, int64_t nb, int64_t sc_nb,
+                          int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64, int64_t sbt, int nblk,
+                          const int64_t* rmap, const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M,
+                          int HD, int cluster_size, int variant, void* scratch, size_t scratch_bytes,
+                          const bx_compact_table* compact, void* stream) {
+  if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
+  if (!ptab || !compact) return BX_EARG;
+  const CompactTable ct{compact->tab, compact->window, compact->slack, compact->factor, compact->mtop, compact->shift};
+  return run_attention(q, nullptr, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, nullptr,
+                       0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, ct, scratch, scratch_bytes, stream);
 }
 
 int bx_prefill_attention(const int32_t* q, const int64_t* sh, const int64_t* pos, const int32_t* tiles, int n_tiles,

@@ -20,6 +20,7 @@
 
 #include <cooperative_groups.h>
 
+#include "attn_weight_tables.cuh"
 #include "bx_ptx.cuh"
 #include "bx_rules.cuh"
 
@@ -53,6 +54,7 @@ struct AttnParams {
   int M, HKV;
   int chunk_cap;        // score slots per query row in shared memory (multiple of 8)
   const int32_t* ptab;  // int8 mode: weight table rsh(e^z table, 10), 131073 entries; null = exact mode
+  CompactTable ct;      // shared-memory form of either table (the streaming kernel); tab null: none
 };
 
 struct AttnShared {
@@ -99,6 +101,62 @@ __device__ __forceinline__ i64 attn_weight_any(const AttnParams& p, i64 raw, i64
     return idx >= 0 ? (i64)__ldg(p.ptab + idx) : 0;
   }
   return attn_weight(raw, mx, rowshift, p.l2e, p.lut);
+}
+
+// The joined score of this lane from the fragments of a 16 x 8 limb product (rows 4 i + g = limb i of query g, columns =
+// keys): lane l gets query (l >> 2) & 3 and key 2 (l & 3) + (l >= 16). The lower half holds limbs 0 and 2, the upper limb 1:
+// each sends the other the sum it needs.
+__device__ __forceinline__ i64 fragment_score(const int (&acc)[3][4], int lane) {
+  i64 s0 = acc[0][0], s1 = acc[0][1], h0 = acc[0][2], h1 = acc[0][3];
+  asm("mad.wide.s32 %0, %1, 256, %0;" : "+l"(s0) : "r"(acc[1][0]));
+  asm("mad.wide.s32 %0, %1, 256, %0;" : "+l"(s1) : "r"(acc[1][1]));
+  asm("mad.wide.s32 %0, %1, 256, %0;" : "+l"(h0) : "r"(acc[1][2]));
+  asm("mad.wide.s32 %0, %1, 256, %0;" : "+l"(h1) : "r"(acc[1][3]));
+  asm("mad.wide.s32 %0, %1, 65536, %0;" : "+l"(s0) : "r"(acc[2][0]));
+  asm("mad.wide.s32 %0, %1, 65536, %0;" : "+l"(s1) : "r"(acc[2][1]));
+  asm("mad.wide.s32 %0, %1, 65536, %0;" : "+l"(h0) : "r"(acc[2][2]));
+  asm("mad.wide.s32 %0, %1, 65536, %0;" : "+l"(h1) : "r"(acc[2][3]));
+  const bool up = lane >= 16;
+  const i64 other = __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
+  const i64 top = __shfl_xor_sync(0xffffffffu, h1, 16);
+  return up ? other + shl(s1, 8) + shl(top, 16) : s0 + shl(other, 8) + shl(h0, 16);
+}
+
+// What a lane of the weight pass knows about its query row.
+struct WeightRow {
+  i64 mx, mxh, rowshift;      // maximum; with the rounding term of the row shift
+  int c, hs;
+  bool fast;                  // the compact table serves the row
+};
+__device__ __forceinline__ WeightRow weight_row(const AttnParams& p, i64 mx, i64 rowshift) {
+  WeightRow r;
+  r.mx = mx;
+  r.rowshift = rowshift;
+  r.fast = p.ct.tab != nullptr && (p.ptab || (rowshift >= 1 && rowshift <= 31));
+  r.c = p.ptab ? WT_INT8_SHIFT : r.fast ? (int)rowshift : 1;
+  r.hs = p.ptab ? 4 : r.c - 1;
+  r.mxh = mx + (p.ptab ? (1ll << (WT_INT8_SHIFT - 1)) - 1 : 1ll << (r.c - 1));
+  return r;
+}
+// The weights of 4 keys (live: visible) of one query from their scores.
+__device__ __forceinline__ void four_weights(const AttnParams& p, const WeightRow& row, const uint32_t* tab, const i64 (&sc)[4],
+                                             const bool (&live)[4], uint32_t (&pv)[4]) {
+  bool redo[4];
+  if (row.fast) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pv[j] = compact_weight(p.ct, tab, row.mxh - sc[j], row.c, row.hs, live[j], redo[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      redo[j] = live[j];
+      pv[j] = 0;
+    }
+  }
+  if (redo[0] | redo[1] | redo[2] | redo[3]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (redo[j]) pv[j] = (uint32_t)attn_weight_any(p, sc[j], row.mx, row.rowshift);
+  }
 }
 
 __global__ void __launch_bounds__(ATT_THREADS)
@@ -794,8 +852,8 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 
   bool ok = true;
   // ---- sweep 1: scores (as the TMA-staged kernel) ----
-  i64 mymax[2] = {ATT_NEG, ATT_NEG};
-  const i64 qp_s1 = (lane < 16 && (lane >> 2) < p.M) ? p.qpos[r * p.M + (lane >> 2)] : -1;
+  i64 mymax = ATT_NEG;
+  const i64 qp_s1 = ((lane >> 2) & 3) < p.M ? p.qpos[r * p.M + ((lane >> 2) & 3)] : -1;
   for (int st = 0; st < nst; ++st) {
     const int slot = st % ATT3_NS, round = st / ATT3_NS;
     if (ok) ok = mbar_wait(&sm->full[slot], round & 1);
@@ -814,23 +872,11 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
           mma_s8(acc[j], afrag[0], w.x, w.y);
           mma_s8(acc[j], afrag[1], w.z, w.w);
         }
-        i64 slo[2], shi[2];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          slo[c] = (i64)acc[0][c] + shl((i64)acc[1][c], 8) + shl((i64)acc[2][c], 16);
-          shi[c] = (i64)acc[0][2 + c] + shl((i64)acc[1][2 + c], 8) + shl((i64)acc[2][2 + c], 16);
-        }
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const i64 mid = __shfl_down_sync(0xffffffffu, slo[c], 16);
-          if (lane < 16) {
-            const i64 raw = slo[c] + shl(mid, 8) + shl(shi[c], 16);
-            const i64 kk = kb + (lane & 3) * 2 + c;
-            if (kk < hi) {
-              scores[(kk - lo) * 4 + (lane >> 2)] = raw;
-              if (kk <= qp_s1) mymax[c] = imax(mymax[c], raw);
-            }
-          }
+        const i64 raw = fragment_score(acc, lane);
+        const i64 kk = kb + (lane & 3) * 2 + (lane >> 4);
+        if (kk < hi) {
+          scores[(kk - lo) * 4 + ((lane >> 2) & 3)] = raw;
+          if (kk <= qp_s1) mymax = imax(mymax, raw);
         }
       }
     }
@@ -838,7 +884,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     if (lane == 0) mbar_arrive(&sm->empty_k[slot]);
   }
   {
-    i64 m = imax(mymax[0], mymax[1]);
+    i64 m = imax(mymax, __shfl_xor_sync(0xffffffffu, mymax, 16));
     m = imax(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = imax(m, __shfl_xor_sync(0xffffffffu, m, 2));
     if (lane < 16 && (lane & 3) == 0) sm->wmax[warp][lane >> 2] = m;
@@ -860,6 +906,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const bool gok = g2 < p.M;
   const i64 qp2 = gok ? p.qpos[r * p.M + g2] : -1;
   const i64 rowshift = (gok && p.sh) ? (i64)(FK + 3 - FZ) - p.sh[pz * p.M + g2] : 0;
+  const WeightRow wrow = weight_row(p, mx, rowshift);
   i64 den = 0;
   const int ngroups = (int)((hi - lo + 31) / 32);
   for (int grp = warp; grp < ngroups; grp += NW) {
@@ -868,18 +915,23 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     for (int j = 0; j < 4; ++j) sc[j] = scores[((i64)grp * 32 + 8 * j + (lane >> 2)) * 4 + g2];
     __syncwarp();
     uint8_t* pt = reinterpret_cast<uint8_t*>(scores) + (size_t)grp * 1024;
+    bool live[4];
+    uint32_t pv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const i64 key = lo + (i64)grp * 32 + 8 * j + (lane >> 2);
+      live[j] = key < hi && key <= qp2;
+    }
+    four_weights(p, wrow, nullptr, sc, live, pv);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int kl = 8 * j + (lane >> 2);
-      const i64 key = lo + (i64)grp * 32 + kl;
-      i64 pv = 0;
-      if (key < hi && key <= qp2) pv = attn_weight_any(p, sc[j], mx, rowshift);
-      den += pv;
-      int pr = (int)pv;
+      den += (i64)(int32_t)pv[j];
+      const uint32_t lb = limb_bytes(pv[j]);
       const int off = (kl >> 4) * 256 + (kl & 15) + g2 * 16;
-      pt[off] = (uint8_t)split8(pr);                                // row g      (limb 0)
-      pt[off + 64] = (uint8_t)split8(pr);                           // row 4 + g  (limb 1)
-      pt[off + 128] = (uint8_t)split8(pr);                          // row 8 + g  (limb 2)
+      pt[off] = (uint8_t)lb;                                          // row g      (limb 0)
+      pt[off + 64] = (uint8_t)(lb >> 8);                              // row 4 + g  (limb 1)
+      pt[off + 128] = (uint8_t)(lb >> 16);                            // row 8 + g  (limb 2)
     }
   }
   fence_proxy_async_smem();
@@ -1061,6 +1113,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
   i64* scores = reinterpret_cast<i64*>(ring + (size_t)NS * STAGE_BYTES);   // later, in place: the p-limb tiles
   Attn6Small* sm = reinterpret_cast<Attn6Small*>(reinterpret_cast<uint8_t*>(scores) + (size_t)p.chunk_cap * 32);
   uint16_t* order = reinterpret_cast<uint16_t*>(sm + 1);             // requests, longest context first (or unused)
+  uint32_t* ctab = reinterpret_cast<uint32_t*>(order + 512);         // the compact weight table, if there is one
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int C = p.chunk_cap;                                          // keys whose scores / p tiles fit in shared memory
   const int GPC = C / 32;                                             // 32-key groups per chunk (a multiple of NW)
@@ -1080,6 +1133,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     tma_prefetch_desc(&tmap_v);
   }
   for (int i = threadIdx.x; i < ATT6_MAXGROUPS; i += blockDim.x) sm->ptag[i] = 0;
+  fill_compact(ctab, p.ct, threadIdx.x, blockDim.x);
   wait_previous();
   if (ranked) {
     // Requests by context length, longest first, in buckets of 128 keys (ties by index): a counting sort whose
@@ -1310,8 +1364,8 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     }
 
     // ---- sweep 1: scores ----
-    i64 mymax[2] = {ATT_NEG, ATT_NEG};
-    const i64 qp_s1 = (lane < 16 && (lane >> 2) < p.M) ? p.qpos[r * p.M + (lane >> 2)] : -1;
+    i64 mymax = ATT_NEG;
+    const i64 qp_s1 = ((lane >> 2) & 3) < p.M ? p.qpos[r * p.M + ((lane >> 2) & 3)] : -1;
     for (int st = 0; st < nst; ++st, ++gidx) {
       const uint32_t slot = gidx % (uint32_t)NS, use = gidx / (uint32_t)NS;
       if (ok) ok = mbar_wait(&sm->full[slot], use & 1);
@@ -1330,24 +1384,13 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
             mma_s8(acc[j], afrag[0], w.x, w.y);
             mma_s8(acc[j], afrag[1], w.z, w.w);
           }
-          i64 slo[2], shi[2];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            slo[c] = (i64)acc[0][c] + shl((i64)acc[1][c], 8) + shl((i64)acc[2][c], 16);
-            shi[c] = (i64)acc[0][2 + c] + shl((i64)acc[1][2 + c], 8) + shl((i64)acc[2][2 + c], 16);
-          }
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const i64 mid = __shfl_down_sync(0xffffffffu, slo[c], 16);
-            if (lane < 16) {
-              const i64 raw = slo[c] + shl(mid, 8) + shl(shi[c], 16);
-              const i64 kk = kb + (lane & 3) * 2 + c;
-              if (kk < hi) {
-                if (spilled) my_spill[kk * 4 + (lane >> 2)] = raw;
-                else scores[kk * 4 + (lane >> 2)] = raw;
-                if (kk <= qp_s1) mymax[c] = imax(mymax[c], raw);
-              }
-            }
+          const i64 raw = fragment_score(acc, lane);
+          const i64 kk = kb + (lane & 3) * 2 + (lane >> 4);
+          if (kk < hi) {
+            const i64 at = kk * 4 + ((lane >> 2) & 3);
+            if (spilled) my_spill[at] = raw;
+            else scores[at] = raw;
+            if (kk <= qp_s1) mymax = imax(mymax, raw);
           }
         }
       }
@@ -1355,7 +1398,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
       if (lane == 0) mbar_arrive(&sm->empty[slot]);
     }
     {
-      i64 m = imax(mymax[0], mymax[1]);
+      i64 m = imax(mymax, __shfl_xor_sync(0xffffffffu, mymax, 16));
       m = imax(m, __shfl_xor_sync(0xffffffffu, m, 1));
       m = imax(m, __shfl_xor_sync(0xffffffffu, m, 2));
       if (lane < 16 && (lane & 3) == 0) sm->wmax[warp][lane >> 2] = m;
@@ -1370,6 +1413,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     const bool gok = g2 < p.M;
     const i64 qp2 = gok ? p.qpos[r * p.M + g2] : -1;
     const i64 rowshift = (gok && p.sh) ? (i64)(FK + 3 - FZ) - p.sh[pz * p.M + g2] : 0;
+    const WeightRow wrow = weight_row(p, mx, rowshift);
     i64 den = 0;
     const int ngroups = (int)((hi + 31) / 32);
     const int nchunks = (ngroups + GPC - 1) / GPC;
@@ -1391,18 +1435,23 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
         }
         __syncwarp();
         uint8_t* pt = reinterpret_cast<uint8_t*>(scores) + (size_t)place * 1024;
+        bool live[4];
+        uint32_t pv[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const i64 key = (i64)grp * 32 + 8 * j + (lane >> 2);
+          live[j] = key < hi && key <= qp2;
+        }
+        four_weights(p, wrow, ctab, sc, live, pv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int kl = 8 * j + (lane >> 2);
-          const i64 key = (i64)grp * 32 + kl;
-          i64 pv = 0;
-          if (key < hi && key <= qp2) pv = attn_weight_any(p, sc[j], mx, rowshift);
-          den += pv;
-          int pr = (int)pv;
+          den += (i64)(int32_t)pv[j];
+          const uint32_t lb = limb_bytes(pv[j]);
           const int off = (kl >> 4) * 256 + (kl & 15) + g2 * 16;
-          pt[off] = (uint8_t)split8(pr);                              // row g      (limb 0)
-          pt[off + 64] = (uint8_t)split8(pr);                         // row 4 + g  (limb 1)
-          pt[off + 128] = (uint8_t)split8(pr);                        // row 8 + g  (limb 2)
+          pt[off] = (uint8_t)lb;                                      // row g      (limb 0)
+          pt[off + 64] = (uint8_t)(lb >> 8);                          // row 4 + g  (limb 1)
+          pt[off + 128] = (uint8_t)(lb >> 16);                        // row 8 + g  (limb 2)
         }
         fence_proxy_async_smem();                                     // the tile is read by tcgen05 (async proxy)
         __syncwarp();

@@ -6,6 +6,7 @@ qkv, attention, attn_out, linear, add_norm, linear, silu_quant, linear, add_norm
 import torch
 
 from .. import _native as nv
+from .. import attn_table
 from ..engine_base import TokenRowEngine
 from ..vllm_plugin import tri_fuse, tri_paged, tri_prefill
 from .gemm_skinny import linear_post
@@ -32,6 +33,7 @@ class IntEngine(TokenRowEngine):
         self.gf, self.lm = t("gf"), lin("lm")
         self.silu_t, self.cos, self.sin, self.ln = t("silu"), t("cos"), t("sin"), t("ln")
         self.ptab = tri_paged.weight_table(t("exp"))
+        self.compact = attn_table.to(attn_table.int8(self.ptab), self.dev)                # the decode kernels' form of it
         self.fl = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self.scr = torch.zeros(self.L, 2, dtype=torch.long, device=self.dev)
         self.timer = None                                    # optional callable(M, N, K) -> context manager
@@ -64,7 +66,7 @@ class IntEngine(TokenRowEngine):
                 den = torch.ones(N, self.HKV, G, 1, dtype=torch.long, device=self.dev)    # padding rows: 0 / 1
                 tri_prefill.attend(q, pos, kvs[i], bt, self.ptab, tiles, num, den)
             else:
-                num, den = tri_paged.attend(q, qpos, kvs[i], bt, self.ptab, rmap=rmap)
+                num, den = tri_paged.attend(q, qpos, kvs[i], bt, self.ptab, rmap=rmap, compact=self.compact)
             x, *pre = fz.add_norm(self, self._lin(fz.attn_out(self, num, den), ly["wo"]), None, None, None, x, ly["gm"])
             a8, mant, e, _ = fz.silu_quant(self, self._lin(pre, ly["wgu"]), None, None, None, self.silu_t, scr=self.scr[i])
             nxt = self.layers[i + 1]["ga"] if i + 1 < self.L else None

@@ -380,7 +380,7 @@ class ColumnShardedIntEngine(TokenRowEngine):
         for i in range(b.L):
             ly = b.layers[i]
             q = fz.qkv(b, b._lin(pre, ly["wqkv"]), None, None, None, pos, slot, kvs[i], int32=True)
-            num, den = tri_paged.attend(q, qpos, kvs[i], bt, b.ptab, rmap=rmap)
+            num, den = tri_paged.attend(q, qpos, kvs[i], bt, b.ptab, rmap=rmap, compact=b.compact)
             x, a8, mant, e = fz.add_norm(b, b._lin(fz.attn_out(b, num, den), ly["wo"]), None, None, None, x, ly["gm"])
             A, Ma, Ea = gather_scaled_rows(a8.view(2, N, b.D), mant, e, self.group)
             y = self.mlps[i](A.view(2 * N * self.world, b.D), Ma, Ea, b.silu_t, b.fl, b.scr[i])

@@ -8,6 +8,7 @@ silu_quant, linear, add_norm), device tensors only, no host synchronisation insi
 import torch
 
 from .. import _native as nv
+from .. import attn_table
 from ..engine_base import TokenRowEngine
 from ..exact.model import Lin
 from . import exact_fuse, tri_exact_attn, tri_prefill
@@ -42,6 +43,7 @@ class ExactEngine(TokenRowEngine):
         self.lm = FusedLin(Lin(c, "lm", self.dev))
         self.cos, self.sin, self.exp2, self.ln = t("cos"), t("sin"), t("exp2"), t("ln")
         self.l2e = L2E28_HD[self.HD]
+        self.compact = attn_table.to(attn_table.exact(self.exp2, self.l2e), self.dev)     # the decode kernels' form of exp2
         self.fl = torch.zeros(1, dtype=torch.int32, device=self.dev)     # sticky bound flag of every kernel
 
     @property
@@ -76,7 +78,7 @@ class ExactEngine(TokenRowEngine):
                                                     kvs[i], bt, tiles, self.exp2, self.l2e)
             else:
                 num, den = tri_exact_attn.attend(qq.view(N, self.HKV, G, self.HD), shq.view(N, self.HKV, G), qpos,
-                                                 kvs[i], bt, rmap, self.exp2, self.l2e)
+                                                 kvs[i], bt, rmap, self.exp2, self.l2e, compact=self.compact)
             qo, sho = fz.attn_out(self, num, den)
             x, q, sh = fz.add_norm(self, ly["wo"](qo, sho, fl, True), x, ly["gm"], fl)
             q, sh = fz.silu_quant(self, ly["wgu"](q, sh, fl, False), self.exp2, fl)

@@ -4,9 +4,12 @@
 Cache layout, per (block, KV head, slot) row of 8 HD bytes: K limbs 0, 1, 2 at bytes [0, 3 HD), V limbs at
 [3 HD, 6 HD); the rest of the row is unused."""
 
+import ctypes
+
 import torch
 
 from .. import _native as nv
+from .. import attn_table
 
 
 def store(c, slot, k, v):
@@ -40,12 +43,12 @@ def weight_table(lut):
     return t.to(torch.int32).contiguous()
 
 
-def attend(q, qpos, cache, bt, ptab, nsplit=None, bm=None, bn=None, warps=4, rmap=None, variant=0):
+def attend(q, qpos, cache, bt, ptab, nsplit=None, bm=None, bn=None, warps=4, rmap=None, variant=0, compact=None):
     """int8-mode paged attention, M <= 4 query rows per (request, KV head): q int64 (or int32) [R, HKV, M, HD] within
     3 limbs, qpos int64 [R, M], cache int8 limb planes [nb, HKV, bs, 8 HD], bt [R, *] block-table rows, ptab =
     weight_table(exp table). Returns num int64 [R, HKV, M, HD], den int64 [R, HKV, M, 1]
     (src/bitexact/vllm_plugin/tri_paged.py:363-430, decode form). nsplit maps to the cluster size; bm, bn, warps are
-    accepted and ignored."""
+    accepted and ignored. compact: `attn_table.int8(ptab)` on the device (same weights, faster)."""
     R, HKV, M, HD = q.shape
     assert M <= 4 and HD == 64 and cache.shape[1] == HKV and cache.shape[3] == 8 * HD and cache.stride(3) == 1
     assert bt.shape[1] * cache.shape[2] < 43690 and bt.dtype in (torch.int32, torch.int64) and bt.stride(1) == 1
@@ -60,11 +63,13 @@ def attend(q, qpos, cache, bt, ptab, nsplit=None, bm=None, bn=None, warps=4, rma
             cs *= 2
     from .tri_exact_attn import _scratch
     ws, ws_bytes = _scratch(q.device, R * HKV, bt.shape[1], cache.shape[2])
-    rc = nv.lib().bx_int8_attention_ws(q32.data_ptr(), qpos.data_ptr(), cache.data_ptr(), cache.shape[0], cache.stride(0),
-                                       cache.stride(1), cache.stride(2), cache.shape[2], bt.data_ptr(),
-                                       int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
-                                       nv.ptr(rmap.long().contiguous() if rmap is not None else None), ptab.data_ptr(),
-                                       num.data_ptr(), den.data_ptr(), R, HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes,
-                                       nv.stream())
-    nv.check(rc, "bx_int8_attention_ws")
+    args = (q32.data_ptr(), qpos.data_ptr(), cache.data_ptr(), cache.shape[0], cache.stride(0), cache.stride(1), cache.stride(2),
+            cache.shape[2], bt.data_ptr(), int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
+            nv.ptr(rmap.long().contiguous() if rmap is not None else None), ptab.data_ptr(), num.data_ptr(), den.data_ptr(), R,
+            HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes)
+    if compact is None:
+        nv.check(nv.lib().bx_int8_attention_ws(*args, nv.stream()), "bx_int8_attention_ws")
+    else:
+        form = attn_table.native(compact)                       # lives until the call has read it
+        nv.check(nv.lib().bx_int8_attention_tab(*args, ctypes.addressof(form), nv.stream()), "bx_int8_attention_tab")
     return num, den

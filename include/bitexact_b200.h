@@ -220,6 +220,26 @@ int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* ca
                          const int64_t* rmap, const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M,
                          int HD, int cluster_size, int variant, void* scratch, size_t scratch_bytes, void* stream);
 
+/* The same with a compact form of the weight table (4097 entries, 16 KB of shared memory per CTA) beside the table itself:
+ * a weight is read off it where that decides the weight, and off the full table elsewhere, so the results are the same
+ * for any table the form was made from (bitexact_llm_b200/attn_table.py: `exact`, `int8`). shift is the left shift of a
+ * row distance before the product with factor; window, slack and mtop as described there. */
+typedef struct {
+  const uint32_t* tab;
+  uint32_t window, slack, factor, mtop;
+  int shift;
+} bx_compact_table;
+int bx_exact_attention_tab(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
+                           int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
+                           int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e, int64_t* num,
+                           int64_t* den, int R, int HKV, int M, int HD, int cluster_size, int variant, void* scratch,
+                           size_t scratch_bytes, const bx_compact_table* compact, void* stream);
+int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* cache, int64_t nb, int64_t sc_nb,
+                          int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64, int64_t sbt, int nblk,
+                          const int64_t* rmap, const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M,
+                          int HD, int cluster_size, int variant, void* scratch, size_t scratch_bytes,
+                          const bx_compact_table* compact, void* stream);
+
 /* ---- prefill attention (both weight rules) -------------------------------------------------------------------------
  * Attention of whole TILES of prompt tokens: a tile is up to tile_rows / G consecutive tokens of one request; one CTA
  * per (tile, KV head) stages every K / V row once for the tile's query rows (token x G query heads), runs both integer
