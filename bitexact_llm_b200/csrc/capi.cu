@@ -464,13 +464,20 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     }
     if (ta <= 48 && n_tiles * ((M + ta - 1) / ta) > 2 * 148) persistent = true;
     if (ta == 64 && K <= 4096 && n_tiles * ((M + 47) / 48) > 2 * 148) { ta = 48; persistent = true; }
-    // Long tile lists of batches that fill blocks of 128 rows about as well as tiles of 48: the activation rows go
-    // to the MMA M side, 64 weight rows per tile (no ragged sixth tile at 256 rows, warp-uniform residual lists,
-    // wider MMAs). Measured, gate / up and LM head: 80 -> 67 us and 519 -> 429 us at M = 256, 46 -> 42 us and
-    // 277 -> 238 us at M = 128, gate / up 878 -> 809 us at M = 4096.
-    if (persistent && ta == 48 && M >= WROWS) {
-      const long ra = ((M + WROWS - 1) / WROWS) * (long)WROWS, rw = ((M + 47) / 48) * 48L;
-      if (10 * ra <= 11 * rw) ta = 664;
+    // Lists of more than one wave from 128 rows on: the activation rows on the MMA M side with 64 weight rows per tile
+    // (wider MMAs, residual lists warp-uniform, epilogue not overlapped) or 48 (two accumulator buffers), or tiles of 48
+    // activation rows where those leave less padding. A tile costs about its K blocks plus, for 64, six of them for the
+    // epilogue; what decides is the waves. Measured, us, before -> now: N 2048 K 8192, 3750 rows 475 -> 392, 1900 240 -> 212, 748
+    // 103 -> 92; N 3072 K 2048, 512 rows 41 -> 32; N 2048 K 2048, 748 rows 39 -> 32; N 8192 K 1024, 2000 rows 184 -> 155; N 16384
+    // K 2048 (the 64-row form as before) 130 / 256 / 3750 rows 48 / 68 / 789.
+    const long blocks = (M + WROWS - 1) / WROWS, t64 = blocks * ((N + 63) / 64);
+    if (M >= WROWS && t64 > 148 && n_tiles * ((M + 63) / 64) > 148) {       // (64 activation rows in one wave: 560 rows, 60 : 90 us)
+      const long nkb = (K + BKB - 1) / BKB;
+      auto waves = [](long tiles) { return (tiles + 147) / 148; };
+      const long c64 = waves(t64) * (40 * nkb + 240), c48 = waves(blocks * ((N + 47) / 48)) * (42 * nkb + 40);
+      const long cw = waves(n_tiles * ((M + 47) / 48)) * (43 * nkb + 48);
+      persistent = true;
+      ta = c64 <= c48 && c64 <= cw ? 664 : c48 <= cw ? 648 : 48;
     }
   }
   int want_split = 0;                 // 10000 S + 200 + rows: split-K over clusters of exactly S CTAs

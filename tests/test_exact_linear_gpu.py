@@ -265,3 +265,19 @@ def test_unfused_linear_api_and_bmm():
         assert np.array_equal(bmm(a2, bkn).cpu().numpy(), want), (Z, M, K, N, "contiguous b")
     assert bmm(torch.zeros(2, 3, 0, dtype=torch.long, device="cuda"), torch.zeros(2, 0, 4, dtype=torch.long, device="cuda")) \
         .abs().sum().item() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 9600, 256), (130, 9601, 272), (300, 3265, 256), (561, 2432, 1040), (748, 2048, 256),
+                                   (749, 3072, 272), (2000, 600, 128)])
+def test_automatic_tiles_of_long_lists(M, N, K):
+    """Around the borders between 64 and 48 weight rows, 48 activation rows and single-wave lists: the tiles chosen by size
+    give the integers of 32 activation rows per tile."""
+    rng = np.random.RandomState(M + N)
+    dec = {"limbs": rng.randint(-128, 128, (3, N, K)).astype(np.int8), "g": rng.randint(-34, -24, N).astype(np.int64),
+           "d": rng.randint(0, 31, N).astype(np.int64), "rr": np.sort(rng.randint(0, N, N // 16)).astype(np.int64),
+           "rc": rng.randint(0, K, N // 16).astype(np.int64), "rv": rng.randint(-(1 << 20), 1 << 20, N // 16).astype(np.int64)}
+    q, sh = rng.randint(-(1 << 22), 1 << 22, (M, K)).astype(np.int64), rng.randint(-45, -8, M).astype(np.int64)
+    fl = _lin(dec)
+    y, flag = _run(fl, q, sh, True, None)
+    want, wflag = _run(fl, q, sh, True, 32)
+    assert np.array_equal(y, want) and flag == wflag
