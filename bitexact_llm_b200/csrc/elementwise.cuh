@@ -88,6 +88,38 @@ __device__ __forceinline__ i64 block_reduce(i64 v, i64* buf) {
   return buf[32];
 }
 
+// Bits of a row maximum. The row exponents and the power-of-two bounds need only the bit length of max |v|, and the OR of the
+// magnitudes has the same: two logic operations per value and two warp reductions of 32 bits, where a 64-bit maximum
+// costs eight issue slots per value and a shuffle tree (measured; 64-bit compares are the dearest common operation).
+// (-2^63, whose magnitude does not exist, counts as 0, as it does for a maximum.)
+__device__ __forceinline__ i64 mag_or(i64 acc, i64 v) { return acc | (iabs(v) & 0x7fffffffffffffffll); }
+__device__ __forceinline__ i64 warp_or(i64 v) {
+  const uint32_t lo = __reduce_or_sync(0xffffffffu, (uint32_t)v), hi = __reduce_or_sync(0xffffffffu, (uint32_t)((u64)v >> 32));
+  return (i64)(((u64)hi << 32) | lo);
+}
+// Sum of 0 <= v < 2^57 over the warp, 26 bits at a time.
+__device__ __forceinline__ i64 warp_sum_pos(i64 v) {
+  const u64 a = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0x3ffffffu), b = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 26) & 0x3ffffffu);
+  const u64 c = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 52));
+  return (i64)(a + (b << 26) + (c << 52));
+}
+// Over the CTA, for all threads, with one barrier: every warp folds the warps' results itself. `buf` holds 32 i64 in shared
+// memory that no other reduction of the kernel uses (between two calls with the same buffer stands another barrier).
+__device__ __forceinline__ i64 block_or(i64 v, i64* buf) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_or(v);
+  if (lane == 0) buf[warp] = v;
+  __syncthreads();
+  return warp_or(lane < nw ? buf[lane] : 0);
+}
+__device__ __forceinline__ i64 block_sum_pos(i64 v, i64* buf) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum_pos(v);
+  if (lane == 0) buf[warp] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? buf[lane] : 0);
+}
+
 // 2^-t at out_bits for t >= 0 at 26 fractional bits: table 2^-f at 2^60 (step 2^-14) + linear interpolation
 // (exact/ops.py:108-116).
 template <bool SMEM_TABLE = false>
@@ -122,7 +154,7 @@ __global__ void __launch_bounds__(NT)
 norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64* __restrict__ ids,
             const i64* __restrict__ gm, const i64* __restrict__ ge, i64* __restrict__ xo, int32_t* __restrict__ q,
             i64* __restrict__ sh_out, int8_t* __restrict__ a8, int32_t* flag, int M, int D, int lg, int do_norm) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[3][32];
   const int64_t row = blockIdx.x;
   i64 x[EPT];
   i64 gmr[EPT], ger[EPT];          // gamma, loaded up front: their latency overlaps the row's loads and reductions
@@ -144,10 +176,10 @@ norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64
       else if (MODE == 1) x[k] = reinterpret_cast<const i64*>(xin)[row * D + c] + yin[row * D + c];
       else x[k] = reinterpret_cast<const i64*>(xin)[row * D + c];
       if (xo) xo[row * D + c] = x[k];
-      ax = imax(ax, iabs(x[k]));
+      ax = mag_or(ax, x[k]);
     }
   }
-  ax = block_reduce<true>(ax, red);
+  ax = block_or(ax, red[0]);                 // the bits of the maximum: what follows reads no more of it
   if (threadIdx.x == 0 && ax >= (1ll << 40)) *flag = 1;
   if (!do_norm) return;
   // rms (exact/ops.py:92-105)
@@ -159,7 +191,7 @@ norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64
     const i64 xs = rshc(x[k], shx);
     S += xs * xs;
   }
-  S = block_reduce<false>(S, red);
+  S = block_sum_pos(S, red[1]);              // at most EPT squares of 2^25 per thread
   const i64 T = S + rshc(EPS60 * D, 60 - 2 * (FR - shx));
   const i64 m = (62 + lg - (i64)bitlen(T)) >> 1;
   const i64 s = 2 * m - lg;
@@ -174,10 +206,10 @@ norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64
     const int c = threadIdx.x + k * NT;
     if (c < D) {
       x[k] = div_round_recip<3>(x[k] * gmr[k], ger[k] - FR - er + FN, (u64)r, inv);
-      pmax = imax(pmax, iabs(x[k]));
+      pmax = mag_or(pmax, x[k]);
     }
   }
-  pmax = block_reduce<true>(pmax, red);
+  pmax = block_or(pmax, red[2]);
   const i64 sh = quant_sh(pmax, -FN);
   if (threadIdx.x == 0) sh_out[row] = sh;
   const int64_t plane = (int64_t)M * D;
@@ -210,7 +242,8 @@ struct QkvParams {
 };
 
 __global__ void qkv_kernel(const QkvParams p) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[2][32];
+  int turn = 0;
   const int64_t row = blockIdx.x;
   const int h = blockIdx.y;
   const int HH = p.HD / 2;
@@ -246,10 +279,10 @@ __global__ void qkv_kernel(const QkvParams p) {
   i64 shmax = NEG_BIG;
   auto head = [&](int g, i64 x1, i64 x2) {
     const int64_t qc = (int64_t)(h * G + g) * p.HD + dd;
-    big = imax(big, imax(iabs(x1), iabs(x2)));
+    big = mag_or(mag_or(big, x1), x2);
     const i64 p1 = x1 * cs - x2 * sn;
     const i64 p2 = x2 * cs + x1 * sn;
-    const i64 amax = block_reduce<true>(imax(iabs(p1), iabs(p2)), red);
+    const i64 amax = block_or(mag_or(mag_or(0, p1), p2), red[turn ^= 1]);
     const i64 sh = quant_sh(amax, -(FR + FT));
     shmax = imax(shmax, sh);
     int32_t* qo = p.q + row * ((int64_t)p.H * p.HD) + qc;
@@ -264,15 +297,14 @@ __global__ void qkv_kernel(const QkvParams p) {
     const int64_t qc = (int64_t)(h * G + g) * p.HD + dd;
     head(g, yr[qc], yr[qc + HH]);
   }
-  big = imax(big, imax(imax(iabs(k1), iabs(k2)), imax(iabs(v1r), iabs(v2r))));
+  big = mag_or(mag_or(mag_or(mag_or(big, k1), k2), v1r), v2r);
   const i64 k1o = rshs<FR + FT - FK>(k1 * cs - k2 * sn);
   const i64 k2o = rshs<FR + FT - FK>(k2 * cs + k1 * sn);
   const i64 v1 = rshs<FR - FV>(v1r);
   const i64 v2 = rshs<FR - FV>(v2r);
   const i64 kvbig = imax(imax(iabs(k1o), iabs(k2o)), imax(iabs(v1), iabs(v2)));
-  big = block_reduce<true>(big, red);
-  const i64 kvmax = block_reduce<true>(kvbig, red);
-  if (threadIdx.x == 0 && (big >= (1ll << 31) || kvmax > LIM3 || shmax > FK + 3 - FZ)) *p.flag = 1;
+  const int over = __syncthreads_or(big >= (1ll << 31) || kvbig > LIM3);
+  if (threadIdx.x == 0 && (over || shmax > FK + 3 - FZ)) *p.flag = 1;
   if (p.cache) {
     if (slot >= 0) {
       int8_t* base = p.cache + (slot / p.bs) * p.sc_nb + (int64_t)h * p.sc_h + (slot % p.bs) * p.sc_bs;
@@ -315,7 +347,7 @@ constexpr int AO_MAXH = 64;
 __global__ void __launch_bounds__(AO_THREADS)
 attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int32_t* __restrict__ q,
                 i64* __restrict__ sh_out, int8_t* __restrict__ a8, int M, int K2, int HD) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[32];
   __shared__ u64 dens[AO_MAXH], invs[AO_MAXH];
   const int64_t row = blockIdx.x;
   const int nh = K2 / HD;
@@ -340,10 +372,10 @@ attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int32_
     if (c < K2) {
       const int hd = c / HD;
       o[k] = dens[hd] ? div_round_recip<1>(o[k], FR - FV, dens[hd], invs[hd]) : 0;
-      omax = imax(omax, iabs(o[k]));
+      omax = mag_or(omax, o[k]);
     }
   }
-  omax = block_reduce<true>(omax, red);
+  omax = block_or(omax, red);
   const i64 sh = quant_sh(omax, -FR);
   if (threadIdx.x == 0) sh_out[row] = sh;
   const int64_t plane = (int64_t)M * K2;
@@ -397,11 +429,11 @@ silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int32_t* __r
       bool bad;
       P[k] = silu_p(yr[c], yr[FF + c], lut, bad);
       anybad |= bad;
-      pmax = imax(pmax, iabs(P[k]));
+      pmax = mag_or(pmax, P[k]);
     }
   }
   if (anybad) *flag = 1;
-  pmax = block_reduce<true>(pmax, red);
+  pmax = block_or(pmax, red);
   const i64 sh = quant_sh(pmax, -2 * FR);
   if (threadIdx.x == 0) sh_out[row] = sh;
   const int64_t plane = (int64_t)M * FF;
@@ -445,15 +477,15 @@ silu_cluster_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int3
     bool bad;
     P[k] = silu_p(yr[c], yr[FF + c], lut, bad);
     anybad |= bad;
-    pmax = imax(pmax, iabs(P[k]));
+    pmax = mag_or(pmax, P[k]);
   }
   if (anybad) *flag = 1;
-  pmax = block_reduce<true>(pmax, red);
+  pmax = block_or(pmax, red);
   if (threadIdx.x == 0) cta_max = pmax;
   cluster.sync();
   i64 rmax = 0;
 #pragma unroll
-  for (int r = 0; r < SILU_CL; ++r) rmax = imax(rmax, *cluster.map_shared_rank(&cta_max, r));
+  for (int r = 0; r < SILU_CL; ++r) rmax |= *cluster.map_shared_rank(&cta_max, r);
   const i64 sh = quant_sh(rmax, -2 * FR);
   if (part == 0 && threadIdx.x == 0) sh_out[row] = sh;
   const int64_t plane = (int64_t)M * FF;
@@ -479,7 +511,8 @@ silu_persistent_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, i
                        i64* __restrict__ sh_out, int8_t* __restrict__ a8, int32_t* flag, int M, int FF) {
   extern __shared__ __align__(16) uint8_t silu_smem[];
   i64* tab = reinterpret_cast<i64*>(silu_smem);
-  __shared__ i64 red[33];
+  __shared__ i64 red[2][32];
+  int turn = 0;
   for (int i = threadIdx.x; i < SILU_TABLE; i += SILU_P_THREADS) tab[i] = __ldg(lut + i);
   __syncthreads();
   launch_next();
@@ -498,10 +531,11 @@ silu_persistent_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, i
         bool bad;
         P[k] = silu_p<true>(yr[c], yr[FF + c], tab, bad);
         anybad |= bad;
-        pmax = imax(pmax, iabs(P[k]));
+        pmax = mag_or(pmax, P[k]);
       }
     }
-    pmax = block_reduce<true>(pmax, red);
+    pmax = block_or(pmax, red[turn ^= 1]);               // a warp is at most one row ahead of another
+
     const i64 sh = quant_sh(pmax, -2 * FR);
     if (threadIdx.x == 0) sh_out[row] = sh;
 #pragma unroll

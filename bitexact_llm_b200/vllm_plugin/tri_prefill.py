@@ -1,7 +1,7 @@
 """Prefill attention on the token-major layout: drop-in for `bitexact.vllm_plugin.tri_prefill`
 (src/bitexact/vllm_plugin/tri_prefill.py:86-108) on the tile kernel of libbitexact_b200 (`bx_prefill_attention`).
 
-One CTA handles a tile of consecutive query tokens of one request and one KV head: every K / V row is staged once
+A tile is a run of consecutive query tokens of one request and one KV head: every K / V row is staged once
 per tile, both sweeps run inside the CTA, the limb products run on tcgen05. Key s is visible to a query iff
 s <= its position and every sum is an exact integer reduction, so the grouping of tokens into tiles cannot change a
 bit. The same kernel serves exact mode (`attend_exact`: per-row exponents and the 2^-f table), which has no
@@ -13,8 +13,7 @@ from .. import _native as nv
 
 BM = 32     # query rows per tile (BM // G tokens): the reference's default
 BN = 64
-ROWS = 32   # tile height the kernel runs by default: 32 query rows per CTA (16: two smaller CTAs per SM; measured
-#             equal on 512-token prompts, 5 % slower on 2048-token ones)
+ROWS = 32   # query rows of a tile (16: tiles of half the height, which fill half of the kernel's rows)
 
 
 def tile_table(pre, G, bm=BM):

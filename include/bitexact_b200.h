@@ -243,8 +243,8 @@ int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* c
 /* ---- prefill attention (both weight rules) -------------------------------------------------------------------------
  * Attention of whole TILES of prompt tokens: a tile is up to tile_rows / G consecutive tokens of one request; one CTA
  * per (tile, KV head) stages every K / V row once for the tile's query rows (token x G query heads), runs both integer
- * sweeps and has the limb products (scores and p.V) on tcgen05 with TMEM accumulators. tile_rows: 32 (one CTA of
- * 512 threads per SM; 0 selects it) or 16 (two CTAs of 256 threads per SM). No effect on results.
+ * sweeps and has the limb products (scores and p.V) on tcgen05 with TMEM accumulators. tile_rows: 32 (0 selects it) or
+ * 16 (tiles of half the height; the kernel's other rows stay empty). No effect on results.
  *   q      int32 [N, HKV, G, 64] token-major (|q| <= 2^22 exact mode; within three limbs int8 mode), 16-byte aligned
  *   sh     int64 [N, HKV, G] row exponents (exact mode; NULL with ptab)
  *   pos    int64 [N] position of each token: key s is visible iff s <= pos
