@@ -61,10 +61,11 @@ __device__ __forceinline__ i64 fdiv_pos_est(i64 num, i64 den) {
 }
 
 // ---- block reductions (exact, order free) ----
+// High words first, then the low words of the lanes that hold the largest (two 32-bit warp reductions).
 __device__ __forceinline__ i64 warp_max(i64 v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = imax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+  const int hi = __reduce_max_sync(0xffffffffu, (int)(v >> 32));
+  const uint32_t lo = __reduce_max_sync(0xffffffffu, (int)(v >> 32) == hi ? (uint32_t)v : 0u);
+  return (i64)(((u64)(uint32_t)hi << 32) | lo);
 }
 __device__ __forceinline__ i64 warp_sum(i64 v) {
 #pragma unroll
@@ -111,6 +112,13 @@ __device__ __forceinline__ i64 block_or(i64 v, i64* buf) {
   if (lane == 0) buf[warp] = v;
   __syncthreads();
   return warp_or(lane < nw ? buf[lane] : 0);
+}
+__device__ __forceinline__ i64 block_max(i64 v, i64* buf) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  v = warp_max(v);
+  if (lane == 0) buf[warp] = v;
+  __syncthreads();
+  return warp_max(lane < nw ? buf[lane] : (i64)0x8000000000000000ull);
 }
 __device__ __forceinline__ i64 block_sum_pos(i64 v, i64* buf) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 int8_norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, const i64* __restrict__ ids,
                  const i64* __restrict__ gamma, i64* __restrict__ xo, int8_t* __restrict__ a8, i64* __restrict__ mant,
                  i64* __restrict__ eo, int32_t* flag, int M, int D, int do_norm) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[3][32];
   const int64_t row = blockIdx.x;
   i64 x[NORM_EPT];
   i64 ax = 0;
@@ -69,10 +69,10 @@ int8_norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, cons
       else if (MODE == 1) x[k] = reinterpret_cast<const i64*>(xin)[row * D + c] + yin[row * D + c];
       else x[k] = reinterpret_cast<const i64*>(xin)[row * D + c];
       if (xo) xo[row * D + c] = x[k];
-      ax = imax(ax, iabs(x[k]));
+      ax = mag_or(ax, x[k]);
     }
   }
-  ax = block_reduce<true>(ax, red);
+  ax = block_or(ax, red[0]);                                          // its bit length and a power-of-two bound are what is read
   if (!do_norm) {
     if (threadIdx.x == 0 && ax >= (1ll << 42)) *flag = 1;
     return;
@@ -89,8 +89,8 @@ int8_norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, cons
       zmax = imax(zmax, iabs(x[k]));
     }
   }
-  S = block_reduce<false>(S, red);
-  zmax = block_reduce<true>(zmax, red);
+  S = block_sum_pos(S, red[1]);
+  zmax = block_max(zmax, red[2]);
   const i64 r = isqrt(S / D + rsh_t(EPS40, 40 - 2 * (FR - shx)));
   i64 sh, as_;
   quant_scale(zmax, sh, as_);
@@ -174,7 +174,7 @@ __global__ void int8_qkv_kernel(const Qkv8Params p) {
 __global__ void __launch_bounds__(AO_THREADS)
 int8_attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int8_t* __restrict__ a8,
                      i64* __restrict__ mant, i64* __restrict__ eo, int M, int K2, int HD) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[32];
   __shared__ u64 dens[AO_MAXH], invs[AO_MAXH];
   const int64_t row = blockIdx.x;
   const int nh = K2 / HD;
@@ -198,7 +198,7 @@ int8_attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, i
       omax = imax(omax, iabs(o[k]));
     }
   }
-  omax = block_reduce<true>(omax, red);
+  omax = block_max(omax, red);
   i64 sh, as_;
   quant_scale(omax, sh, as_);
   const u64 inv = ~0ull / (u64)(2 * as_);
@@ -227,7 +227,7 @@ template <int EPT>
 __global__ void __launch_bounds__(SILU_THREADS)
 int8_silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int8_t* __restrict__ a8,
                  i64* __restrict__ mant, i64* __restrict__ eo, i64* __restrict__ scr, int M, int FF) {
-  __shared__ i64 red[33];
+  __shared__ i64 red[3][32];
   const int64_t row = blockIdx.x;
   const i64* yr = y + row * (2 * (int64_t)FF);
   i64 hv[EPT];
@@ -246,9 +246,9 @@ int8_silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int8_t*
       umax = imax(umax, iabs(u));
     }
   }
-  hmax = block_reduce<true>(hmax, red);
-  smax = block_reduce<true>(smax, red);
-  umax = block_reduce<true>(umax, red);
+  hmax = block_max(hmax, red[0]);
+  smax = block_max(smax, red[1]);
+  umax = block_max(umax, red[2]);
   if (threadIdx.x == 0 && scr) {
     atomicMax(reinterpret_cast<long long*>(scr), (long long)smax);
     atomicMax(reinterpret_cast<long long*>(scr + 1), (long long)umax);
