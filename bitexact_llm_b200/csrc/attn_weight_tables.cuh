@@ -16,6 +16,7 @@
 // same integers for any table.
 #pragma once
 
+#include "bx_ptx.cuh"
 #include "bx_rules.cuh"
 
 namespace bx {
@@ -126,6 +127,10 @@ struct CompactTable {
 constexpr int CT_N = 4097;
 constexpr int CT_BYTES = 16400;
 
+__device__ __forceinline__ void prefetch_compact(const CompactTable& ct, int tid, int n) {     // into L2, the grid's CTAs a part each
+  if (ct.tab)
+    for (int i = 8 * (blockIdx.x * n + tid); i < CT_N; i += 8 * gridDim.x * n) prefetch_l2(ct.tab + i);
+}
 __device__ __forceinline__ void fill_compact(uint32_t* dst, const CompactTable& ct, int tid, int n) {
   if (ct.tab)
     for (int i = tid; i < CT_N; i += n) dst[i] = __ldg(ct.tab + i);

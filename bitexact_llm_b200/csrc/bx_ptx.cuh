@@ -33,12 +33,21 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // Hint: bring the line that holds *p into L1 (no register, no wait).
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
+// The same into L2 only, the point of coherence: a line asked for before its writer has ended is never read stale.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Programmatic dependent launch: the kernels of a step are launched so that the next one may start (barriers, TMEM, the
 // first weight tiles) while the last CTAs of the one before it are still running. `launch_next` permits that, as soon as
-// every CTA has come this far; `wait_previous` returns when the previous kernel has completed and its writes are visible,
-// and stands before the first access to anything another kernel of the step reads or writes. Weights are exempt. A
+// every CTA has come this far; `wait_previous` returns when the previous kernel has completed and its writes are visible. A
 // kernel that allocates TMEM calls `launch_next` after the allocation: a CTA of the next kernel on the same SM could
 // otherwise take the columns first and wait, holding them, for the CTA that needs them.
+//
+// In the integer library `wait_previous` stands before the first access to global memory, tables and scales included:
+// whoever wrote them may be the kernel in front, and its writes are visible only then (also where it permits nothing and
+// this kernel starts at its very end). The weights of a linear may be read ahead of it where the caller says that the
+// kernel in front is the stage that made the activations (`early`); for that to hold for all that ran before the stage,
+// a stage calls `launch_next` only after its own `wait_previous`. (The float library reads weights ahead in every product
+// and permits first: include/bitexact_float.h.)
 //
 // In the integer library the row-local stages permit it: the linear or attention kernel behind them does its set-up, its
 // first weight tiles or its weight table meanwhile. The linear and attention kernels do not: the stages behind them have

@@ -438,7 +438,7 @@ int bx_split_limbs(const int32_t* q, int64_t ldq, int8_t* a8, int M, int K, void
 static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs, const int64_t* d,
                              const int64_t* g, const int32_t* cnt, const int32_t* ec, const int64_t* ev, int R,
                              const int8_t* planes, int64_t* y, int32_t* flag, int M, int N, int K, int checked,
-                             int tile_rows, void* stream) {
+                             int tile_rows, int early, void* stream) {
   int8_t* scratch = const_cast<int8_t*>(planes);
   cudaStream_t st = (cudaStream_t)stream;
   int ta = tile_rows;
@@ -504,7 +504,7 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
       CUtensorMap mact, mwt;
       if (!make_map(&mact, scratch, (uint64_t)K, (uint64_t)M, 3, WROWS)) return BX_ELAUNCH;
       if (!make_map(&mwt, limbs, (uint64_t)K, (uint64_t)N, 3, 64)) return BX_ELAUNCH;
-      ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked};
+      ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked, early};
       return launch_exact_rows_splitk<64>(mact, mwt, ep, K, split, st);
     }
     ta = 664;                          // K too short to split: the same tile shape on the one-CTA kernel
@@ -516,7 +516,7 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     CUtensorMap mw, mb;
     if (!make_map(&mw, limbs, (uint64_t)K, (uint64_t)N, 3, WROWS)) return BX_ELAUNCH;
     if (!make_map_chunks(&mb, scratch, (uint64_t)K, (uint64_t)M, 3, (uint32_t)(ta / 2))) return BX_ELAUNCH;
-    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked};
+    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked, early};
     switch (ta) {
       case 16: return launch_exact_pair<16>(mw, mb, ep, K, st);
       case 32: return launch_exact_pair<32>(mw, mb, ep, K, st);
@@ -529,7 +529,7 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     CUtensorMap ma, mw;
     if (!make_map(&ma, scratch, (uint64_t)K, (uint64_t)M, 3, WROWS)) return BX_ELAUNCH;
     if (!make_map_chunks(&mw, limbs, (uint64_t)K, (uint64_t)N, 3, (uint32_t)(ta / 2))) return BX_ELAUNCH;
-    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked};
+    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked, early};
     switch (ta) {
       case 16: return launch_exact_rows<16, true>(ma, mw, ep, K, st);
       case 32: return launch_exact_rows<32, true>(ma, mw, ep, K, st);
@@ -544,7 +544,7 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     CUtensorMap mact, mwt;
     if (!make_map(&mact, scratch, (uint64_t)K, (uint64_t)M, 3, WROWS)) return BX_ELAUNCH;
     if (!make_map(&mwt, limbs, (uint64_t)K, (uint64_t)N, 3, (uint32_t)ta)) return BX_ELAUNCH;
-    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked};
+    ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked, early};
     switch (ta) {
       case 16: return launch_exact_rows_one<16, 2>(mact, mwt, ep, K, st);
       case 32: return launch_exact_rows_one<32, 2>(mact, mwt, ep, K, st);
@@ -581,7 +581,7 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
   CUtensorMap mw, ma;
   if (!make_map(&mw, limbs, (uint64_t)K, (uint64_t)N, 3, WROWS)) return BX_ELAUNCH;
   if (!make_map(&ma, scratch, (uint64_t)K, (uint64_t)M, 3, (uint32_t)ta)) return BX_ELAUNCH;
-  ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked};
+  ExactEpiParams ep{q, ldq, sh, d, g, cnt, ec, ev, R, y, flag, M, N, checked, early};
   if (split >= 2) {
     switch (ta) {
       case 16: return launch_exact_splitk<16>(mw, ma, ep, K, split, st);
@@ -1468,17 +1468,29 @@ int bx_exact_epilogue(const int64_t* T, const int64_t* B, const int32_t* q, int6
 int bx_int8_mm(const int8_t* a, const int8_t* w, int32_t* c, int M, int N, int K, int tile_rows, void* stream) {
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!c) return BX_EARG;
-  Int8EpiParams ep{c, nullptr, 0, nullptr, nullptr, nullptr, nullptr, M, N, 0};
+  Int8EpiParams ep{c, nullptr, 0, nullptr, nullptr, nullptr, nullptr, M, N, 0, 0};
   return run_int8<false>(a, w, ep, K, tile_rows, (cudaStream_t)stream);
+}
+
+static int int8_linear_post(const int8_t* a, const int8_t* w, const int64_t* mul, int64_t fmsh, const int64_t* mant,
+                            const int64_t* e, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
+                            int early, void* stream) {
+  if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
+  if (!mul || !mant || !e || !y || !flag) return BX_EARG;
+  Int8EpiParams ep{nullptr, mul, fmsh, mant, e, y, flag, M, N, checked, early};
+  return run_int8<true>(a, w, ep, K, tile_rows, (cudaStream_t)stream);
 }
 
 int bx_int8_linear_post(const int8_t* a, const int8_t* w, const int64_t* mul, int64_t fmsh, const int64_t* mant,
                         const int64_t* e, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
                         void* stream) {
-  if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
-  if (!mul || !mant || !e || !y || !flag) return BX_EARG;
-  Int8EpiParams ep{nullptr, mul, fmsh, mant, e, y, flag, M, N, checked};
-  return run_int8<true>(a, w, ep, K, tile_rows, (cudaStream_t)stream);
+  return int8_linear_post(a, w, mul, fmsh, mant, e, y, flag, M, N, K, checked, tile_rows, 0, stream);
+}
+
+int bx_int8_linear_post_early(const int8_t* a, const int8_t* w, const int64_t* mul, int64_t fmsh, const int64_t* mant,
+                              const int64_t* e, int64_t* y, int32_t* flag, int M, int N, int K, int checked,
+                              int tile_rows, void* stream) {
+  return int8_linear_post(a, w, mul, fmsh, mant, e, y, flag, M, N, K, checked, tile_rows, 1, stream);
 }
 
 int bx_exact_linear(const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs, const int64_t* d,
@@ -1492,19 +1504,33 @@ int bx_exact_linear(const int32_t* q, int64_t ldq, const int64_t* sh, const int8
   if (M == 0) return BX_OK;
   int rc = bx_split_limbs(q, ldq, scratch, M, K, stream);
   if (rc != BX_OK) return rc;
-  return exact_linear_core(q, ldq, sh, limbs, d, g, cnt, ec, ev, R, scratch, y, flag, M, N, K, checked, tile_rows, stream);
+  return exact_linear_core(q, ldq, sh, limbs, d, g, cnt, ec, ev, R, scratch, y, flag, M, N, K, checked, tile_rows, 1, stream);
 }
 
-int bx_exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs,
+static int exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs,
                            const int64_t* d, const int64_t* g, const int32_t* cnt, const int32_t* ec, const int64_t* ev,
-                           int R, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
+                           int R, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows, int early,
                            void* stream) {
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!planes || !sh || !limbs || !d || !g || !y || !flag) return BX_EARG;
   if (M < 0 || N <= 0 || K <= 0 || K % 16 || K >= 43690 || !aligned16(limbs) || !aligned16(planes)) return BX_EARG;
   if (cnt && (!ec || !ev || R <= 0 || !q)) return BX_EARG;
   if (M == 0) return BX_OK;
-  return exact_linear_core(q, ldq, sh, limbs, d, g, cnt, ec, ev, R, planes, y, flag, M, N, K, checked, tile_rows, stream);
+  return exact_linear_core(q, ldq, sh, limbs, d, g, cnt, ec, ev, R, planes, y, flag, M, N, K, checked, tile_rows, early, stream);
+}
+
+int bx_exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs,
+                           const int64_t* d, const int64_t* g, const int32_t* cnt, const int32_t* ec, const int64_t* ev,
+                           int R, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
+                           void* stream) {
+  return exact_linear_planes(planes, q, ldq, sh, limbs, d, g, cnt, ec, ev, R, y, flag, M, N, K, checked, tile_rows, 0, stream);
+}
+
+int bx_exact_linear_planes_early(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh,
+                                 const int8_t* limbs, const int64_t* d, const int64_t* g, const int32_t* cnt,
+                                 const int32_t* ec, const int64_t* ev, int R, int64_t* y, int32_t* flag, int M, int N,
+                                 int K, int checked, int tile_rows, void* stream) {
+  return exact_linear_planes(planes, q, ldq, sh, limbs, d, g, cnt, ec, ev, R, y, flag, M, N, K, checked, tile_rows, 1, stream);
 }
 
 // ---- allocation-free variant of the exact linear ----

@@ -26,6 +26,7 @@ struct ExactEpiParams {
   int32_t* flag;         // sticky lost-bit / range flag (only ever set to 1)
   int M, N;
   int checked;
+  int early;             // the weights may be read before the previous kernel has ended
 };
 
 template <int TA>
@@ -188,7 +189,8 @@ exact_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     const ExactEpiParams ep, int K, int m_tiles) {
   const int mt = blockIdx.x % m_tiles;
   const int nt = blockIdx.x / m_tiles;
-  limb_gemm_tile<3, 3, TA, ExactEpilogue<TA>>(&tmap_w, &tmap_a, nt * WROWS, mt * TA, 0, (K + BKB - 1) / BKB, ep);
+  limb_gemm_tile<3, 3, TA, ExactEpilogue<TA>>(&tmap_w, &tmap_a, nt * WROWS, mt * TA, 0, (K + BKB - 1) / BKB, ep,
+                                               ep.early != 0);
 }
 
 // Persistent form (one CTA per SM, double-buffered accumulators): used when the tile list is longer than one wave.
@@ -196,7 +198,8 @@ template <int TA>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 exact_linear_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                                const ExactEpiParams ep, int K, int n_tiles, int m_tiles) {
-  limb_gemm_persistent<3, 3, TA, ExactEpilogue<TA>>(&tmap_w, &tmap_a, n_tiles, m_tiles, (K + BKB - 1) / BKB, ep);
+  limb_gemm_persistent<3, 3, TA, ExactEpilogue<TA>>(&tmap_w, &tmap_a, n_tiles, m_tiles, (K + BKB - 1) / BKB, ep,
+                                                     ep.early != 0);
 }
 
 // CTA-pair form (tcgen05 .cta_group::2, see limb_gemm_pair.cuh): a cluster of two CTAs per 256 weight rows, one pair

@@ -154,7 +154,8 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      // The first stages' weights are on their way before the previous kernel has ended, their activations after it.
+      // The first stages' weights first; with `early` they are on their way before the previous kernel has ended.
+      if (!ep.early) wait_previous();
       const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         uint8_t* st = ring + i * Cfg::STAGE_BYTES;

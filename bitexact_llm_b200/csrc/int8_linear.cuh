@@ -54,6 +54,7 @@ struct Int8EpiParams {
   int32_t* flag;         // post: sticky |t| >= 2^38 flag
   int M, N;
   int checked;
+  int early;             // the weights may be read before the previous kernel has ended
 };
 
 template <int TA, bool POST>
@@ -129,7 +130,8 @@ int8_linear_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                    const Int8EpiParams ep, int K, int m_tiles) {
   const int mt = blockIdx.x % m_tiles;
   const int nt = blockIdx.x / m_tiles;
-  limb_gemm_tile<1, 2, TA, Int8Epilogue<TA, POST>>(&tmap_w, &tmap_a, nt * WROWS, mt * TA, 0, (K + BKB - 1) / BKB, ep);
+  limb_gemm_tile<1, 2, TA, Int8Epilogue<TA, POST>>(&tmap_w, &tmap_a, nt * WROWS, mt * TA, 0, (K + BKB - 1) / BKB, ep,
+                                                   ep.early != 0);
 }
 
 // Persistent form (one CTA per SM walks the tile list, two accumulator buffers: the post epilogue of tile i overlaps
@@ -138,7 +140,8 @@ template <int TA, bool POST>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 int8_linear_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                               const Int8EpiParams ep, int K, int n_tiles, int m_tiles) {
-  limb_gemm_persistent<1, 2, TA, Int8Epilogue<TA, POST>>(&tmap_w, &tmap_a, n_tiles, m_tiles, (K + BKB - 1) / BKB, ep);
+  limb_gemm_persistent<1, 2, TA, Int8Epilogue<TA, POST>>(&tmap_w, &tmap_a, n_tiles, m_tiles, (K + BKB - 1) / BKB, ep,
+                                                         ep.early != 0);
 }
 
 }  // namespace bx

@@ -58,8 +58,8 @@ int8_norm_kernel(const void* __restrict__ xin, const i64* __restrict__ yin, cons
   const int64_t row = blockIdx.x;
   i64 x[NORM_EPT];
   i64 ax = 0;
-  launch_next();
   wait_previous();
+  launch_next();
 #pragma unroll
   for (int k = 0; k < NORM_EPT; ++k) {
     const int c = threadIdx.x + k * NORM_THREADS;
@@ -131,8 +131,8 @@ __global__ void int8_qkv_kernel(const Qkv8Params p) {
   const int HH = p.HD / 2, G = p.H / p.HKV, dd = threadIdx.x;
   const int64_t NT = (int64_t)(p.H + 2 * p.HKV) * p.HD;
   constexpr int SHR = FT + FR - FQ;
-  launch_next();
   wait_previous();
+  launch_next();
   const i64 pos = p.pos[row];
   const i64 cs = p.cos[pos * HH + dd], sn = p.sin[pos * HH + dd];
   const i64* yr = p.y + row * NT;
@@ -178,8 +178,8 @@ int8_attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, i
   __shared__ u64 dens[AO_MAXH], invs[AO_MAXH];
   const int64_t row = blockIdx.x;
   const int nh = K2 / HD;
-  launch_next();
   wait_previous();
+  launch_next();
   if (threadIdx.x < nh) {
     const u64 dv = 2 * (u64)den[row * nh + threadIdx.x];
     dens[threadIdx.x] = dv;
@@ -232,8 +232,8 @@ int8_silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int8_t*
   const i64* yr = y + row * (2 * (int64_t)FF);
   i64 hv[EPT];
   i64 hmax = 0, smax = 0, umax = 0;
-  launch_next();
   wait_previous();
+  launch_next();
 #pragma unroll
   for (int k = 0; k < EPT; ++k) {
     const int c = threadIdx.x + k * SILU_THREADS;

@@ -52,11 +52,12 @@ struct GemmShared {
 };
 
 // Runs the main loop for the output tile (weight rows n0.., activation rows m0..) over k blocks [kb0, kb1).
+// early: the weights may be read before the previous kernel of the stream has ended.
 // On return, for warps 2..5, the accumulators are complete in TMEM (returns false after a timeout).
 // Epi::run(tmem_base, lane_quarter, group, lane, ...) is called by the epilogue warps.
 template <int NW, int NA, int TA, class Epi>
 __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const CUtensorMap* tmap_a, int n0, int m0,
-                                               int kb0, int kb1, const typename Epi::Params& ep) {
+                                               int kb0, int kb1, const typename Epi::Params& ep, bool early = false) {
   using Cfg = GemmCfg<NW, NA, TA>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -97,7 +98,8 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      // The first stages' weights are on their way before the previous kernel has ended, their activations after it.
+      // The first stages' weights first; with `early` they are on their way before the previous kernel has ended.
+      if (!early) wait_previous();
       const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);
@@ -210,10 +212,10 @@ struct GemmSharedP {
 
 // NBUF accumulator buffers in TMEM (2: the epilogue of a tile runs behind the MMAs of the next one; 1: tiles too wide
 // for two buffers, the MMAs of the next tile wait until the epilogue has read the accumulators out, while the TMA
-// warp already fills the ring for it). W_FASTEST: consecutive tiles walk the 128-row operand first.
+// warp already fills the ring for it). W_FASTEST: consecutive tiles walk the 128-row operand first. early: as above.
 template <int NW, int NA, int TA, class Epi, int NBUF = 2, bool W_FASTEST = false>
 __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, const CUtensorMap* tmap_a, int n_tiles,
-                                                     int m_tiles, int nkb, const typename Epi::Params& ep) {
+                                                     int m_tiles, int nkb, const typename Epi::Params& ep, bool early) {
   using Cfg = GemmCfg<NW, NA, TA>;
   static_assert(NBUF == 1 || NBUF == 2, "one or two accumulator buffers");
   static_assert(NBUF * Cfg::COLS <= 512, "the accumulator buffers must fit in TMEM");
@@ -262,8 +264,9 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
       // ---- TMA producer: one continuous stream of stages over all tiles of this CTA ----
       int it = 0;            // global stage counter
       bool ok = true;
-      // The first tile's first stages: the weights (the 128-row operand, with W_FASTEST the stacked one) are on their way
-      // before the previous kernel has ended, the activations after it.
+      // The first tile's first stages: the weights first (the 128-row operand, with W_FASTEST the stacked one); with `early`
+      // they are on their way before the previous kernel has ended.
+      if (!early) wait_previous();
       const int pre = blockIdx.x >= total ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         uint8_t* st = ring + i * Cfg::STAGE_BYTES;

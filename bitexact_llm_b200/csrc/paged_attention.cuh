@@ -1133,8 +1133,9 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     tma_prefetch_desc(&tmap_v);
   }
   for (int i = threadIdx.x; i < ATT6_MAXGROUPS; i += blockDim.x) sm->ptag[i] = 0;
-  fill_compact(ctab, p.ct, threadIdx.x, blockDim.x);
+  prefetch_compact(p.ct, threadIdx.x, blockDim.x);
   wait_previous();
+  fill_compact(ctab, p.ct, threadIdx.x, blockDim.x);
   if (ranked) {
     // Requests by context length, longest first, in buckets of 128 keys (ties by index): a counting sort whose
     // placement step runs in one warp over 32 requests at a time (match_any gives each lane its place among the lanes

@@ -333,6 +333,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
     auto sync_weights = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(32 * PF_WARPS) : "memory"); };
     const bool start = ok;
     // ---- the weight table, and the first tile's queries ----
+    wait_previous();
     {
       bool fits = EXACT ? fill_exp2_table(table, p.w.lut, tid, 32 * PF_WARPS) : fill_int8_table(table, p.w.ptab, tid, 32 * PF_WARPS);
       if (EXACT) {
@@ -340,7 +341,6 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
         fits &= check_exp2_table(table, tid, 32 * PF_WARPS) && p.w.l2e >= (1ll << 28) && p.w.l2e < (1ll << 29);
       }
       if (!fits) sm->bad_table = 1;
-      wait_previous();                                   // the table is no other kernel's work, the queries are
       if (ok && blockIdx.x < p.work) {
         ok = mbar_wait(&sm->info_full[0], 0);
         if (ok) write_q(load_q(sm->tile[0]));

@@ -211,8 +211,8 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
   __shared__ i64 gtab[41];
   const int64_t row = blockIdx.y;
   const int chunk = blockIdx.x;
-  launch_next();
   wait_previous();
+  launch_next();
   const i64 tn = rows[4 * row + 2], td = rows[4 * row + 3];
   const int64_t c0 = (int64_t)chunk * ch;
   const int64_t c1 = c0 + ch < V ? c0 + ch : V;
@@ -306,8 +306,8 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
 __global__ void sample_combine_kernel(const i64* __restrict__ pmax, const i64* __restrict__ pidx,
                                       i64* __restrict__ tok, i64* __restrict__ omax, int M, int nch) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  launch_next();
   wait_previous();
+  launch_next();
   if (row >= M) return;
   i64 best = pmax[(int64_t)row * nch], bidx = pidx[(int64_t)row * nch];
   for (int c = 1; c < nch; ++c) {

@@ -45,10 +45,11 @@ class IntEngine(TokenRowEngine):
             raise OverflowError("integer bound violated (int8 mode)")
 
     def _lin(self, pre, lin):
+        """The linear directly behind the stage that made `pre`."""
         if self.timer is not None:
             with self.timer(pre[1].shape[0], lin[0].shape[0], lin[0].shape[1]):
                 return linear_post(pre[0], lin[0], lin[1], lin[2], pre[1], pre[2], self.fl, True)
-        return linear_post(pre[0], lin[0], lin[1], lin[2], pre[1], pre[2], self.fl, True)
+        return linear_post(pre[0], lin[0], lin[1], lin[2], pre[1], pre[2], self.fl, True, early=True)
 
     def forward(self, kvs, ids, pos, slot, bt, rmap, tiles=None):
         """Same contract as ExactEngine.forward; returns the residual stream int64 [N, D] at 16 bits."""

@@ -21,16 +21,17 @@ def int_mm(a, w, M=None):
     return c
 
 
-def linear_post(a, w, m, fmsh, mant, e, flag, check=True, M=None):
+def linear_post(a, w, m, fmsh, mant, e, flag, check=True, M=None, early=False):
     """post(join_limbs(int_mm(a, w)), m, fmsh, mant, e) in one kernel: int64 [M, N] at 16 fractional bits.
-    m int64 [N], fmsh int, mant / e int64 [M]; flag int32 [1] is set when check and some |t| >= 2^38."""
+    m int64 [N], fmsh int, mant / e int64 [M]; flag int32 [1] is set when check and some |t| >= 2^38.
+    early: as `vllm_plugin.exact_gemm.FusedLin.__call__`."""
     R, K = a.shape
     N = w.shape[0]
     M = mant.shape[0] if M is None else M
     assert a.dtype == torch.int8 and w.dtype == torch.int8 and a.is_contiguous() and w.is_contiguous() and R >= 2 * M
     y = torch.empty(M, N, dtype=torch.long, device=a.device)
-    rc = nv.lib().bx_int8_linear_post(a.data_ptr(), w.data_ptr(), m.data_ptr(), int(fmsh), mant.contiguous().data_ptr(),
-                                      e.contiguous().data_ptr(), y.data_ptr(), flag.data_ptr(), M, N, K,
-                                      int(bool(check)), 0, nv.stream())
+    call = nv.lib().bx_int8_linear_post_early if early else nv.lib().bx_int8_linear_post
+    rc = call(a.data_ptr(), w.data_ptr(), m.data_ptr(), int(fmsh), mant.contiguous().data_ptr(), e.contiguous().data_ptr(),
+              y.data_ptr(), flag.data_ptr(), M, N, K, int(bool(check)), 0, nv.stream())
     nv.check(rc, "bx_int8_linear_post")
     return y

@@ -32,7 +32,9 @@ class FusedLin:
         self.cfg = cfg                                           # tile rows (16..80) or None = automatic
         self.timer = None                                        # optional callable(M, N, K) -> context manager
 
-    def __call__(self, q, sh, flag, checked=True):
+    def __call__(self, q, sh, flag, checked=True, early=False):
+        """early: the call stands directly behind the stage that made q, on the same stream, so that the weights may be read
+        while that stage still runs (nothing else wrote them since the stage was launched)."""
         M, K = q.shape
         assert q.dtype == torch.int32 and q.stride(1) == 1 and K == self.K and sh.dtype == torch.int64
         sh = sh.contiguous()
@@ -41,18 +43,17 @@ class FusedLin:
             return y
         if self.timer is not None:
             with self.timer(M, self.N, K):
-                return self._run(q, sh, flag, checked, y, M, K)
-        return self._run(q, sh, flag, checked, y, M, K)
+                return self._run(q, sh, flag, checked, y, M, K)     # the timer may launch work of its own: not early
+        return self._run(q, sh, flag, checked, y, M, K, early)
 
-    def _run(self, q, sh, flag, checked, y, M, K):
+    def _run(self, q, sh, flag, checked, y, M, K, early=False):
         from .exact_fuse import planes_of
         planes = planes_of(q, M, K)                      # limb planes written by the stage kernel that produced q
         if planes is not None:
-            rc = nv.lib().bx_exact_linear_planes(planes.data_ptr(), q.data_ptr(), q.stride(0), sh.data_ptr(),
-                                                 self.limbs.data_ptr(), self.d.data_ptr(), self.g.data_ptr(),
-                                                 nv.ptr(self.cnt), nv.ptr(self.ec), nv.ptr(self.ev), self.R,
-                                                 y.data_ptr(), flag.data_ptr(), M, self.N, K, int(bool(checked)),
-                                                 self.cfg or 0, nv.stream())
+            call = nv.lib().bx_exact_linear_planes_early if early else nv.lib().bx_exact_linear_planes
+            rc = call(planes.data_ptr(), q.data_ptr(), q.stride(0), sh.data_ptr(), self.limbs.data_ptr(), self.d.data_ptr(),
+                      self.g.data_ptr(), nv.ptr(self.cnt), nv.ptr(self.ec), nv.ptr(self.ev), self.R, y.data_ptr(),
+                      flag.data_ptr(), M, self.N, K, int(bool(checked)), self.cfg or 0, nv.stream())
             nv.check(rc, "bx_exact_linear_planes")
             return y
         scratch = torch.empty(3 * M * K, dtype=torch.int8, device=q.device)

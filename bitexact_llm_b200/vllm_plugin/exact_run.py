@@ -72,7 +72,7 @@ class ExactEngine(TokenRowEngine):
         x, q, sh = fz.embed_norm(self, ids.long(), self.layers[0]["ga"], fl)
         for i in range(self.L):
             ly = self.layers[i]
-            qq, shq = fz.qkv(self, ly["wqkv"](q, sh, fl, False), pos, slot, kvs[i], fl)
+            qq, shq = fz.qkv(self, ly["wqkv"](q, sh, fl, False, early=True), pos, slot, kvs[i], fl)
             if tiles is not None:
                 num, den = tri_prefill.attend_exact(qq.view(N, self.HKV, G, self.HD), shq.view(N, self.HKV, G), pos,
                                                     kvs[i], bt, tiles, self.exp2, self.l2e)
@@ -80,13 +80,13 @@ class ExactEngine(TokenRowEngine):
                 num, den = tri_exact_attn.attend(qq.view(N, self.HKV, G, self.HD), shq.view(N, self.HKV, G), qpos,
                                                  kvs[i], bt, rmap, self.exp2, self.l2e, compact=self.compact)
             qo, sho = fz.attn_out(self, num, den)
-            x, q, sh = fz.add_norm(self, ly["wo"](qo, sho, fl, True), x, ly["gm"], fl)
-            q, sh = fz.silu_quant(self, ly["wgu"](q, sh, fl, False), self.exp2, fl)
+            x, q, sh = fz.add_norm(self, ly["wo"](qo, sho, fl, True, early=True), x, ly["gm"], fl)
+            q, sh = fz.silu_quant(self, ly["wgu"](q, sh, fl, False, early=True), self.exp2, fl)
             nxt = self.layers[i + 1]["ga"] if i + 1 < self.L else None
-            x, q, sh = fz.add_norm(self, ly["wd"](q, sh, fl, True), x, nxt, fl)
+            x, q, sh = fz.add_norm(self, ly["wd"](q, sh, fl, True, early=True), x, nxt, fl)
         return x
 
     def logits(self, h):
         """Final residual rows [M, D] -> int64 logits [M, V] at 24 bits."""
         q, sh = exact_fuse.pre_norm(self, h, self.gf, self.fl)
-        return self.lm(q, sh, self.fl, True)
+        return self.lm(q, sh, self.fl, True, early=True)

@@ -4,6 +4,11 @@
  * bound violations never raise: kernels set the caller's sticky `flag` word to 1 (it is never cleared).
  * `stream` is a cudaStream_t passed as void* (NULL = default stream). Calls are asynchronous.
  *
+ * Stream order: many kernels are launched so that they may start (barriers, tensor memory, descriptors) while the kernel
+ * in front of them is still running. They read and write nothing before that kernel has ended, so a call sees all that
+ * was put on the stream before it, weights and tables too. The only reads that come earlier are those of the weights in
+ * bx_exact_linear (its own splitting pass is the kernel in front) and in the two entry points named *_early.
+ *
  * Each declaration cites the reference interface it replaces (paths inside mynotwo/bitexact-llm).
  */
 #ifndef BITEXACT_B200_H
@@ -86,6 +91,14 @@ int bx_exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t ldq, 
                            int R, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
                            void* stream);
 
+/* bx_exact_linear_planes directly behind the stage kernel of this library that wrote `planes`, on the same stream: the
+ * weights (limbs) may be read while that kernel is still running. It must not be the one that writes them; any kernel
+ * in front of it may be. Same results as bx_exact_linear_planes, which waits for the kernel in front whatever it is. */
+int bx_exact_linear_planes_early(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh,
+                                 const int8_t* limbs, const int64_t* d, const int64_t* g, const int32_t* cnt,
+                                 const int32_t* ec, const int64_t* ev, int R, int64_t* y, int32_t* flag, int M, int N,
+                                 int K, int checked, int tile_rows, void* stream);
+
 /* bx_exact_linear for callers that must not allocate device memory. It has no counterpart in the reference.
  *
  * Some hosts of this library cannot provide the scratch buffer bx_exact_linear asks for: a plugin that is
@@ -122,11 +135,16 @@ int bx_exact_linear_static(const int32_t* q, int64_t ldq, const int64_t* sh, con
  * CTA per SM, two accumulator buffers), the automatic choice when there are more tiles than SMs; for
  * bx_int8_linear_post also 216, 232, 264 (10000 S + 2xx: clusters of exactly S = 2, 4 or 8): that many rows per tile
  * with the K dimension split over a cluster of CTAs, the automatic choice when the tile list covers less than half
- * of the SMs. No effect on results. */
+ * of the SMs. No effect on results.
+ *
+ * bx_int8_linear_post_early: directly behind the stage kernel that wrote `a`, as bx_exact_linear_planes_early. */
 int bx_int8_mm(const int8_t* a, const int8_t* w, int32_t* c, int M, int N, int K, int tile_rows, void* stream);
 int bx_int8_linear_post(const int8_t* a, const int8_t* w, const int64_t* mul, int64_t fmsh, const int64_t* mant,
                         const int64_t* e, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,
                         void* stream);
+int bx_int8_linear_post_early(const int8_t* a, const int8_t* w, const int64_t* mul, int64_t fmsh, const int64_t* mant,
+                              const int64_t* e, int64_t* y, int32_t* flag, int M, int N, int K, int checked,
+                              int tile_rows, void* stream);
 
 /* Activation limb planes only: q int32 [M, K] -> a8 int8 [3, M, K] (signed base-256 digits,
  * src/bitexact/intops.py:62-70). */

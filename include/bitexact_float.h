@@ -3,6 +3,11 @@
  * otherwise, BX_* status codes, `stream` is a cudaStream_t, calls are asynchronous and allocate nothing.
  *
  * Element type T of a call: dtype BXF_BF16 (bfloat16) or BXF_F32 (float, no reduced-precision product anywhere).
+ * Stream order: the kernels of this library may start while those in front of them are still running, and read WEIGHTS
+ * (products, convolutions, decays, stream mixes) ahead of their end; everything else only after it. A caller that
+ * rewrites weights on the stream puts something that is not of this library behind the write (any kernel or copy), or
+ * synchronises, before the next call.
+ *
  * "row" = one token of the step. Rows of one sequence are consecutive and in position order.
  * Leading dimensions (ld*) and group strides (gs*) count elements. In bf16, operands of the products start on 16-byte
  * boundaries and have leading dimensions and group strides that are multiples of 8; the extents themselves are free.
