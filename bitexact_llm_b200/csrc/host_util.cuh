@@ -48,7 +48,10 @@ int launch_chained(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaS
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = cluster > 0 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) return BX_ELAUNCH;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...) != cudaSuccess) {
+    cudaGetLastError();                 // told by the return value: the next call's own check must not find it
+    return BX_ELAUNCH;
+  }
   return launched(1);
 }
 

@@ -92,3 +92,20 @@ def test_device_status_word_stops_the_kernels_and_surfaces_on_the_host(engines):
     assert torch.equal(lin(q, sh, eng.fl, True), want)
     eng.check()
     eng8.check()
+
+
+def test_a_refused_launch_leaves_the_next_call_alone():
+    """65536 KV heads are more than a grid holds in its second dimension: the launch is refused with BX_ELAUNCH, and the next
+    call, which is in order, is not blamed for it."""
+    from bitexact_llm_b200 import _native as nv
+    lib = nv.lib()
+    for launch in ("bx_exact_qkv", "bx_int8_qkv"):
+        def call(heads):
+            z = lambda n, dt=torch.long: torch.zeros(n, dtype=dt, device="cuda")
+            y, cos, pos, q, sh, flag = z(3 * heads * 64), z(32), z(1), z(heads * 64, torch.int32), z(heads), z(1, torch.int32)
+            head = (y.data_ptr(), cos.data_ptr(), cos.data_ptr(), pos.data_ptr(), pos.data_ptr(), None, 0, 0, 0, 1)
+            out = (q.data_ptr(), sh.data_ptr()) if launch == "bx_exact_qkv" else (None, q.data_ptr())
+            return getattr(lib, launch)(*head, *out, flag.data_ptr(), 1, heads, heads, 64, nv.stream())
+        assert call(65536) == nv.BX_ELAUNCH
+        assert call(4) == nv.BX_OK
+    torch.cuda.synchronize()
