@@ -203,13 +203,10 @@ int launch_exact_rows_one(const CUtensorMap& mact, const CUtensorMap& mwt, const
   const int w_tiles = (ep.N + TN - 1) / TN;
   const long total = (long)row_blocks * w_tiles;
   const int grid = (int)(total < sms ? total : sms);
-  // Chained (launch_chained) while a CTA has a few tiles: 6451 against 6478 us for a decode step of 256 sequences (3.5 tiles per CTA);
-  // plain on long lists, where the early start buys nothing and measured 1 % (LM head of 700 rows, 81 tiles: 1522 against 1505 us).
-  if (total <= 8L * sms)
-    return launch_chained(exact_linear_rows_one_kernel<TN, NBUF>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mact, mwt, ep, K,
-                          row_blocks, w_tiles);
-  exact_linear_rows_one_kernel<TN, NBUF><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mact, mwt, ep, K, row_blocks, w_tiles);
-  return launched(1);
+  // Chained whatever the length of the list: plainly, a decode step of 256 sequences took 6041 us in place of 6011; on long lists (LM
+  // head of 700 rows, 81 tiles per CTA) the two differ by less than two runs of one.
+  return launch_chained(exact_linear_rows_one_kernel<TN, NBUF>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mact, mwt, ep, K,
+                        row_blocks, w_tiles);
 }
 
 template <int TA, bool POST>

@@ -154,9 +154,9 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      // The first stages' weights first; with `early` they are on their way before the previous kernel has ended.
-      if (!ep.early) wait_previous();
-      const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      // early: the first stages' weights are on their way before the previous kernel has ended. (Otherwise a stage's two operands
+      // are requested together: all weights in front of the first activations cost a short list 1 .. 2 us.)
+      const int pre = !ep.early ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         uint8_t* st = ring + i * Cfg::STAGE_BYTES;
         mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);

@@ -98,9 +98,8 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
       // ---- TMA producer ----
       int issued = 0;
       bool ok = true;
-      // The first stages' weights first; with `early` they are on their way before the previous kernel has ended.
-      if (!early) wait_previous();
-      const int pre = nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      // early: the first stages' weights are on their way before the previous kernel has ended.
+      const int pre = !early ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);
         tma_load_3d(ring + i * Cfg::STAGE_BYTES, tmap_w, &sh->full[i], (kb0 + i) * BKB, n0, 0);
@@ -264,10 +263,9 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
       // ---- TMA producer: one continuous stream of stages over all tiles of this CTA ----
       int it = 0;            // global stage counter
       bool ok = true;
-      // The first tile's first stages: the weights first (the 128-row operand, with W_FASTEST the stacked one); with `early`
-      // they are on their way before the previous kernel has ended.
-      if (!early) wait_previous();
-      const int pre = blockIdx.x >= total ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
+      // early: the weights of the first tile's first stages (the 128-row operand, with W_FASTEST the stacked one) are on
+      // their way before the previous kernel has ended.
+      const int pre = !early || blockIdx.x >= total ? 0 : nkb < Cfg::STAGES ? nkb : Cfg::STAGES;
       for (int i = 0; i < pre; ++i) {
         uint8_t* st = ring + i * Cfg::STAGE_BYTES;
         mbar_arrive_expect_tx(&sh->full[i], Cfg::STAGE_BYTES);

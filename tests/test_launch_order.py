@@ -32,10 +32,13 @@ def test_no_kernel_reads_memory_before_its_wait():
 
 
 def test_weight_tiles_are_requested_behind_the_wait_unless_asked_for_early():
+    seen = 0
     for name, src in _integer_sources().items():
-        for m in re.finditer(r"---- TMA producer.*?\n(.*?)tma_load_3d\(", src, re.S):
-            if "wait_previous" in src:
-                assert re.search(r"if \(!(ep\.)?early\) wait_previous\(\);", m.group(1)), name
+        for m in re.finditer(r"---- TMA producer.*?\n(.*?)wait_previous\(\);", src, re.S):
+            seen += 1
+            assert re.search(r"const int pre = !(ep\.)?early", m.group(1)) and "for (int i = 0; i < pre;" in m.group(1), name
+            assert m.group(1).count("for (") == 1, name      # nothing but those first tiles is asked for in front of the wait
+    assert seen == 3
 
 
 def test_only_the_engines_ask_for_weights_early(monkeypatch):
