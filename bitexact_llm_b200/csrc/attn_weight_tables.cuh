@@ -127,13 +127,13 @@ struct CompactTable {
 constexpr int CT_N = 4097;
 constexpr int CT_BYTES = 16400;
 
-__device__ __forceinline__ void prefetch_compact(const CompactTable& ct, int tid, int n) {     // into L2, the grid's CTAs a part each
-  if (ct.tab)
-    for (int i = 8 * (blockIdx.x * n + tid); i < CT_N; i += 8 * gridDim.x * n) prefetch_l2(ct.tab + i);
-}
-__device__ __forceinline__ void fill_compact(uint32_t* dst, const CompactTable& ct, int tid, int n) {
-  if (ct.tab)
-    for (int i = tid; i < CT_N; i += n) dst[i] = __ldg(ct.tab + i);
+// One thread asks for the table; it is complete when the phase of `bar` is (16-byte aligned ct.tab and dst). The copy runs
+// behind the scores of the first pair. Copied by all threads in front of them instead, it held up batches of short
+// contexts: 64 sequences of up to 64 keys 18 : 22.5 us.
+__device__ __forceinline__ void fetch_compact(uint32_t* dst, const CompactTable& ct, uint64_t* bar) {
+  mbar_arrive_expect_tx(bar, (CT_N - 1) * 4);
+  bulk_load(dst, ct.tab, bar, (CT_N - 1) * 4);
+  dst[CT_N - 1] = __ldg(ct.tab + CT_N - 1);
 }
 // hs: a distance with hi >> hs != 0 is out of range (weight 0).
 __device__ __forceinline__ uint32_t compact_weight(const CompactTable& ct, const uint32_t* tab, i64 zz, int c, int hs, bool live,

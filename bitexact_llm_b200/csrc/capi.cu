@@ -723,7 +723,7 @@ static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, con
   }
   // The compact weight table where it costs neither a CTA nor the ring: 256 sequences of 512 .. 768 keys 155 -> 133 us; a
   // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %.
-  if (ct.tab && per_sm >= 1 && stages(fixed + CT_BYTES) >= 4) {
+  if (ct.tab && aligned16(ct.tab) && per_sm >= 1 && stages(fixed + CT_BYTES) >= 4) {
     fixed += CT_BYTES;
     ns = stages(fixed);
   } else {

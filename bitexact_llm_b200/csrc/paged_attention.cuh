@@ -1069,13 +1069,14 @@ namespace bx {
 constexpr int ATT6_MAXNS = 8;
 constexpr int ATT6_MAXGROUPS = 160;        // 32-key groups per pair (5120 keys)
 
-struct Attn6Small {
+struct alignas(16) Attn6Small {
   i64 cnum[4][ATT_HD];
   i64 pden[ATT_WARPS][4];
   i64 wmax[ATT_WARPS][4];
   uint64_t full[ATT6_MAXNS];
   uint64_t empty[ATT6_MAXNS];
   uint64_t acc_done;
+  uint64_t table_full;
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t ptag[ATT6_MAXGROUPS];           // ordinal + 1 of the pair whose weights the group's p tile holds
@@ -1127,15 +1128,20 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
       mbar_init(&sm->empty[s], NW);
     }
     mbar_init(&sm->acc_done, 1);
+    mbar_init(&sm->table_full, 1);
     sm->abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
   }
   for (int i = threadIdx.x; i < ATT6_MAXGROUPS; i += blockDim.x) sm->ptag[i] = 0;
-  prefetch_compact(p.ct, threadIdx.x, blockDim.x);
   wait_previous();
-  fill_compact(ctab, p.ct, threadIdx.x, blockDim.x);
+  auto context = [&](int64_t t) -> i64 {                              // keys of request t
+    i64 kend = 0;
+    for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[t * p.M + g] + 1);
+    return imin(imax(kend, 0), (i64)p.nblk * p.bs);
+  };
+  if (p.ct.tab && threadIdx.x == 0) fetch_compact(ctab, p.ct, &sm->table_full);
   if (ranked) {
     // Requests by context length, longest first, in buckets of 128 keys (ties by index): a counting sort whose
     // placement step runs in one warp over 32 requests at a time (match_any gives each lane its place among the lanes
@@ -1145,10 +1151,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     for (int t = threadIdx.x; t < 512; t += blockDim.x) base[t] = 0;
     __syncthreads();
     for (int t = threadIdx.x; t < nreq; t += blockDim.x) {
-      i64 kend = 0;
-      for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[(int64_t)t * p.M + g] + 1);
-      kend = imin(imax(kend, 0), (i64)p.nblk * p.bs);
-      lens[t] = 511 - (int)imin(kend >> 7, 511);                       // bucket 0 = the longest contexts
+      lens[t] = 511 - (int)imin(context(t) >> 7, 511);                       // bucket 0 = the longest contexts
     }
     __syncthreads();
     bool same = true;
@@ -1207,10 +1210,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
   };
   auto keys_of = [&](int64_t pz) -> i64 {
     const int64_t r = pz / p.HKV;
-    i64 kend = 0;
-    for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[r * p.M + g] + 1);
-    kend = imin(kend, (i64)p.nblk * p.bs);
-    return imin(kend, my_spill ? (i64)spill_keys : (i64)C);
+    return imin(context(r), my_spill ? (i64)spill_keys : (i64)C);
   };
 
   if (warp == NW) {
@@ -1326,6 +1326,13 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
 
   // ---------------- consumer warps ----------------
   bool ok = true;
+  bool table = p.ct.tab == nullptr;                                  // the compact table is there, or there is none
+  auto wait_table = [&]() {
+    table = true;
+    if (__all_sync(0xffffffffu, mbar_wait(&sm->table_full, 0))) return;
+    ok = false;
+    if (lane == 0) { atomicAdd(&g_wait_timeouts, 1); sm->abort_flag = 1; }
+  };
   uint32_t gidx = 0;
   uint32_t wave = 0;                                                 // chunks handed over so far (acc_done phases)
   for (int64_t w = blockIdx.x; w < npairs; w += gridDim.x) {
@@ -1418,6 +1425,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     i64 den = 0;
     const int ngroups = (int)((hi + 31) / 32);
     const int nchunks = (ngroups + GPC - 1) / GPC;
+    if (!table && ngroups > 0) wait_table();
     for (int ck = 0; ck < nchunks; ++ck) {
       if (ck > 0) {
         // the p tiles of the previous chunk are still being read by its MMAs until they are committed
@@ -1514,6 +1522,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     wave += (uint32_t)nchunks;
     asm volatile("bar.sync 1, %0;" ::"r"(CTHREADS) : "memory");     // cnum / pden / wmax are free for the next pair
   }
+  if (!table) wait_table();                                          // no pair had a key: the copy lands before the CTA ends
   __syncthreads();
   if (warp == 0) {
     __syncwarp();
