@@ -365,6 +365,82 @@ int run_int8(const int8_t* a, const int8_t* w, const Int8EpiParams& ep, int K, i
   }
 }
 
+// What a tile list takes, in units of 10 ns: launch + waves of 148 tiles x (K blocks x block + tile). Fitted to 1026 pairs of a
+// batch (128 .. 4096 rows) and a shape of weights (83 shapes, N 512 .. 128256, K 256 .. 14336; flushed L2), the lists with residual
+// entries and those without on their own. Single times are off by up to 10 %; what counts is which form is ahead.
+struct ListCost {
+  int launch, block, tile;
+  long of(long tiles, long nkb, long more = 0) const { return launch + (tiles + 147) / 148 * (block * nkb + tile + more); }
+};
+struct ListCosts {
+  ListCost act64, act48, act32, act48p, act32p, w64, w48;     // activation rows per tile (p: persistent), weight rows per tile
+};
+constexpr ListCosts LIST_PLAIN = {{182, 71, 572}, {678, 62, 496}, {330, 60, 638}, {1008, 63, 131}, {877, 58, 90},
+                                  {1274, 65, 335}, {1451, 60, 154}};
+constexpr ListCosts LIST_RESIDUAL = {{0, 94, 888}, {467, 72, 742}, {360, 70, 786}, {1417, 68, 108}, {210, 63, 436},
+                                     {1496, 68, 319}, {1445, 63, 138}};
+// More for a tile of 64 / 48 weight rows where the rows of y start off 32-byte boundaries: they are written row by row.
+constexpr int ODD_W64 = 580, ODD_W48 = 410;
+
+// The tile form (a tile_rows value) of an exact linear.
+int exact_linear_auto(int M, int N, int K, bool residual) {
+  // Activation rows per CTA: the size that needs the fewest wave-rows (below); a tile list of more than two waves
+  // goes to the persistent kernel (48 rows, overlapped epilogue).
+  const long n_tiles = (N + WROWS - 1) / WROWS, nkb = (K + BKB - 1) / BKB;
+  auto act_tiles = [&](int rows) { return n_tiles * ((M + rows - 1) / rows); };
+  int ta = M <= 16 ? 16 : M <= 32 ? 32 : 48;
+  if (M > 48) {
+    // waves of 148 CTAs x (rows of a tile + a fixed cost of about 16 rows' worth of prologue and epilogue)
+    long best = -1;
+    const int cand[3] = {64, 48, 32};
+    for (int i = 0; i < 3; ++i) {
+      const long cost = ((act_tiles(cand[i]) + 147) / 148) * (cand[i] + 16);
+      if (best < 0 || cost < best) { best = cost; ta = cand[i]; }
+    }
+  }
+  bool persistent = ta <= 48 && act_tiles(ta) > 2 * 148;
+  if (ta == 64 && K <= 4096 && act_tiles(48) > 2 * 148) { ta = 48; persistent = true; }
+  const long blocks = (M + WROWS - 1) / WROWS, w64_tiles = blocks * ((N + 63) / 64);
+  const bool full_blocks = 10 * blocks * WROWS <= 11 * (((M + 47) / 48) * 48L);     // 128-row blocks pad about as little as 48
+  // Few tiles: K split over clusters, so that the tile list covers the SMs.
+  if (!persistent && M >= WROWS && K >= 8192) {
+    // a batch that fills blocks of 128 rows (the down projection at 256 rows): activation rows on the MMA M side, 64 weight
+    // rows per tile, as many K slices as keep the CTA count within the SMs
+    if (full_blocks && w64_tiles * 2 <= 148) return w64_tiles * 4 <= 148 ? 40764 : 20764;
+    // 64-row tiles with K split over CTA pairs read less shared memory per product than one wave of 32-row tiles
+    // (measured 47 -> 39 us)
+    if (M > 128 && act_tiles(64) * 2 <= 148) return 20264;
+  }
+  if (!persistent && M <= 128 && ta != 48 && act_tiles(ta) * 2 <= 148) {
+    int split = (int)(148 / act_tiles(ta));
+    const int lim = ta == 16 ? splitk_limit<16>() : ta == 32 ? splitk_limit<32>() : splitk_limit<64>();
+    if (split > lim) split = lim;
+    if (split > nkb / 2) split = (int)(nkb / 2);
+    while (split & (split - 1)) --split;
+    // at most 4: clusters of 8 measured 1.3 - 1.5 x slower on these shapes (fewer of them are resident at a time)
+    if (split > 4) split = 4;
+    return split >= 2 ? 10000 * split + 200 + ta : ta;
+  }
+  if (M < WROWS) return persistent ? -ta : ta;
+  // From 128 rows on: the activation rows on the MMA M side with 64 weight rows per tile (wider MMAs, residual lists
+  // warp-uniform, epilogue not overlapped) or 48 (two accumulator buffers), or 48 activation rows on the persistent kernel,
+  // where one of them is predicted to be faster than what the rules so far give. Over the fitted sizes that is 0.95 of the time
+  // of those rules (8 of 1026 more than 2 % slower, with residual entries 7), and 0.96 / 0.98 of that of a choice by waves with
+  // three fixed costs, which took up to 1.6 x as long (N 9601, K 272, 160 rows 22.5 -> 31.7 us; N 4096, K 14336, 560 rows
+  // 223 -> 259 us).
+  const int form = persistent ? (ta == 48 && full_blocks ? 664 : -ta) : ta;
+  const ListCosts& c = residual ? LIST_RESIDUAL : LIST_PLAIN;
+  const long t48 = act_tiles(48);
+  const long cost[3] = {c.w64.of(w64_tiles, nkb, N % 4 ? ODD_W64 : 0), c.w48.of(blocks * ((N + 47) / 48), nkb, N % 4 ? ODD_W48 : 0),
+                        c.act48p.of(t48, nkb)};
+  const long given = form == 664 ? cost[0] : form == -48 ? cost[2] : form == -32 ? c.act32p.of(act_tiles(32), nkb)
+                   : form == 64 ? c.act64.of(act_tiles(64), nkb) : form == 48 ? c.act48.of(t48, nkb)
+                   : c.act32.of(act_tiles(32), nkb);
+  const int forms[3] = {664, 648, -48};
+  const int best = cost[0] <= cost[1] && cost[0] <= cost[2] ? 0 : cost[1] <= cost[2] ? 1 : 2;
+  return 100 * cost[best] < 99 * given ? forms[best] : form;
+}
+
 }  // namespace
 
 extern "C" {
@@ -438,59 +514,17 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
                              int tile_rows, int early, void* stream) {
   int8_t* scratch = const_cast<int8_t*>(planes);
   cudaStream_t st = (cudaStream_t)stream;
-  int ta = tile_rows;
-  bool persistent = false;
-  if (ta < 0) {                       // negative: that tile size on the persistent kernel (16, 32, 48)
+  int ta = tile_rows == 0 ? exact_linear_auto(M, N, K, cnt != nullptr) : tile_rows;
+  const bool persistent = ta < 0;     // negative: that tile size on the persistent kernel (16, 32, 48)
+  if (persistent) {
     ta = -ta;
-    persistent = true;
     if (ta != 16 && ta != 32 && ta != 48) return BX_EARG;
-  } else if (ta == 0) {
-    // Activation rows per CTA: the size that needs the fewest wave-rows (below); a tile list of more than two waves
-    // goes to the persistent kernel (48 rows, overlapped epilogue).
-    const long n_tiles = (N + WROWS - 1) / WROWS;
-    ta = M <= 16 ? 16 : M <= 32 ? 32 : 48;
-    if (M > 48) {
-      // waves of 148 CTAs x (rows of a tile + a fixed cost of about 16 rows' worth of prologue and epilogue)
-      long best = -1;
-      const int cand[3] = {64, 48, 32};
-      for (int i = 0; i < 3; ++i) {
-        const long tiles = n_tiles * ((M + cand[i] - 1) / cand[i]);
-        const long cost = ((tiles + 147) / 148) * (cand[i] + 16);
-        if (best < 0 || cost < best) { best = cost; ta = cand[i]; }
-      }
-    }
-    if (ta <= 48 && n_tiles * ((M + ta - 1) / ta) > 2 * 148) persistent = true;
-    if (ta == 64 && K <= 4096 && n_tiles * ((M + 47) / 48) > 2 * 148) { ta = 48; persistent = true; }
-    // Lists of more than one wave from 128 rows on: the activation rows on the MMA M side with 64 weight rows per tile
-    // (wider MMAs, residual lists warp-uniform, epilogue not overlapped) or 48 (two accumulator buffers), or tiles of 48
-    // activation rows where those leave less padding. A tile costs about its K blocks plus, for 64, six of them for the
-    // epilogue; what decides is the waves. Measured, us, before -> now: N 2048 K 8192, 3750 rows 475 -> 392, 1900 240 -> 212, 748
-    // 103 -> 92; N 3072 K 2048, 512 rows 41 -> 32; N 2048 K 2048, 748 rows 39 -> 32; N 8192 K 1024, 2000 rows 184 -> 155; N 16384
-    // K 2048 (the 64-row form as before) 130 / 256 / 3750 rows 48 / 68 / 789.
-    const long blocks = (M + WROWS - 1) / WROWS, t64 = blocks * ((N + 63) / 64);
-    if (M >= WROWS && t64 > 148 && n_tiles * ((M + 63) / 64) > 148) {       // (64 activation rows in one wave: 560 rows, 60 : 90 us)
-      const long nkb = (K + BKB - 1) / BKB;
-      auto waves = [](long tiles) { return (tiles + 147) / 148; };
-      const long c64 = waves(t64) * (40 * nkb + 240), c48 = waves(blocks * ((N + 47) / 48)) * (42 * nkb + 40);
-      const long cw = waves(n_tiles * ((M + 47) / 48)) * (43 * nkb + 48);
-      persistent = true;
-      ta = c64 <= c48 && c64 <= cw ? 664 : c48 <= cw ? 648 : 48;
-    }
   }
   int want_split = 0;                 // 10000 S + 200 + rows: split-K over clusters of exactly S CTAs
   if (ta >= 10000) {
     want_split = ta / 10000;
     ta %= 10000;
     if (!((ta >= 200 && ta < 300) || ta == 764) || (want_split != 2 && want_split != 4 && want_split != 8)) return BX_EARG;
-  }
-  // Long K, few tiles, a batch that fills blocks of 128 rows (the down projection at 256 rows): K split over CTA
-  // pairs with the activation rows on the MMA M side, 64 weight rows per tile (764; 10000 S + 764: clusters of S).
-  if (tile_rows == 0 && !persistent && M >= WROWS && K >= 8192 &&
-      10 * (((M + WROWS - 1) / WROWS) * (long)WROWS) <= 11 * (((M + 47) / 48) * 48L) &&
-      ((M + WROWS - 1) / WROWS) * (long)((N + 63) / 64) * 2 <= 148) {
-    const long tiles = ((M + WROWS - 1) / WROWS) * (long)((N + 63) / 64);
-    ta = 764;
-    want_split = tiles * 4 <= 148 ? 4 : 2;           // as many K slices as keep the CTA count within the SMs
   }
   if (ta == 764) {
     int split = want_split ? want_split : 2;
@@ -506,8 +540,6 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     }
     ta = 664;                          // K too short to split: the same tile shape on the one-CTA kernel
   }
-  // Split-K over a cluster of CTAs (200 + activation rows per tile asks for it; automatic for small batches whose
-  // tile list covers less than half of the SMs): as many K slices as keep the CTA count within the 148 SMs.
   if (ta == 416 || ta == 432 || ta == 448) {          // 400 + rows: that tile size on the CTA-pair kernel
     ta -= 400;
     CUtensorMap mw, mb;
@@ -550,20 +582,12 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
       default: return launch_exact_rows_one<80, 1>(mact, mwt, ep, K, st);
     }
   }
+  // Split-K over a cluster of CTAs: 200 + activation rows per tile.
   int split = 0;
   if (ta >= 200) {
     ta -= 200;
     split = want_split ? want_split : SPLITK_MAX;
     if (ta != 16 && ta != 32 && ta != 64) return BX_EARG;
-  } else if (tile_rows == 0 && !persistent && M <= 128 && (ta == 16 || ta == 32 || ta == 64)) {
-    const long tiles = ((N + WROWS - 1) / WROWS) * ((M + ta - 1) / ta);
-    if (tiles * 2 <= 148) split = (int)(148 / tiles);
-  } else if (tile_rows == 0 && !persistent && M > 128 && K >= 8192 &&
-             ((N + WROWS - 1) / WROWS) * (long)((M + 63) / 64) * 2 <= 148) {
-    // Long K, few tiles (the down projection at a batch of 256): 64-row tiles with K split over CTA pairs read less
-    // shared memory per product than one wave of 32-row tiles (measured 47 -> 39 us).
-    ta = 64;
-    split = 2;
   }
   if (split > 0) {
     const int nkb = (K + BKB - 1) / BKB;
@@ -571,9 +595,6 @@ static int exact_linear_core(const int32_t* q, int64_t ldq, const int64_t* sh, c
     if (split > lim) split = lim;
     if (split > nkb / 2) split = nkb / 2;                      // at least two K blocks per slice
     while (split & (split - 1)) --split;   // clusters of 2, 4 or 8: a cluster of 6 ran 1.6 x slower than one of 4
-    // automatic choice: at most 4 (clusters of 8 measured 1.3 - 1.5 x slower on these shapes: fewer of them are
-    // resident at a time); an explicit request (tile_rows 2xx) may still take 8
-    if (tile_rows == 0 && split > 4) split = 4;
   }
   CUtensorMap mw, ma;
   if (!make_map(&mw, limbs, (uint64_t)K, (uint64_t)N, 3, WROWS)) return BX_ELAUNCH;
@@ -1514,6 +1535,11 @@ static int exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t l
   if (cnt && (!ec || !ev || R <= 0 || !q)) return BX_EARG;
   if (M == 0) return BX_OK;
   return exact_linear_core(q, ldq, sh, limbs, d, g, cnt, ec, ev, R, planes, y, flag, M, N, K, checked, tile_rows, early, stream);
+}
+
+int bx_exact_linear_tile(int M, int N, int K, int residual) {
+  if (M < 0 || N <= 0 || K <= 0 || K % 16 || K >= 43690) return BX_EARG;
+  return exact_linear_auto(M, N, K, residual != 0);
 }
 
 int bx_exact_linear_planes(const int8_t* planes, const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs,

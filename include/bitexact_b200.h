@@ -67,16 +67,17 @@ int bx_i8_tensor_peak(int iters, int repeats, double* tops, void* stream);
  *   tile_rows  activation rows per CTA tile: 0 = automatic, else one of 16, 32, 48, 64, 80; -16, -32, -48 select
  *              that tile size on the persistent kernel (one CTA per SM, overlapped epilogue); 216, 232, 264 select
  *              16, 32, 64 rows with the K dimension split over a cluster of up to 8 CTAs (partial sums through
- *              distributed shared memory), the automatic choice for M <= 128 when the tile list covers less than
- *              half of the SMs (10000 S + 2xx: clusters of exactly S = 2, 4 or 8 CTAs); 416, 432, 448: that many
- *              activation rows on CTA pairs (tcgen05 cta_group::2, 256 weight rows per pair); 516 .. 580 and
- *              616 .. 680 (steps of 16): the ACTIVATION rows on the MMA M side and that many weight rows per tile,
- *              on CTA pairs / on one CTA (the automatic choice for long tile lists of batches of 128 rows and
- *              more: 664); 764 (10000 S + 764): 64 weight rows per tile with the activation rows on the M side and
- *              K split over clusters of S = 2 or 4 CTAs (the automatic choice for short tile lists with K >= 8192
- *              at 128 rows and more). No effect on results.
+ *              distributed shared memory; 10000 S + 2xx: clusters of exactly S = 2, 4 or 8 CTAs); 416, 432, 448:
+ *              that many activation rows on CTA pairs (tcgen05 cta_group::2, 256 weight rows per pair); 516 .. 580
+ *              and 616 .. 680 (steps of 16): the ACTIVATION rows on the MMA M side and that many weight rows per
+ *              tile, on CTA pairs / on one CTA; 764 (10000 S + 764): 64 weight rows per tile with the activation
+ *              rows on the M side and K split over clusters of S = 2 or 4 CTAs. No effect on results.
+ *   bx_exact_linear_tile: the automatic choice for these sizes (residual: cnt is given), as a tile_rows value: the split
+ *              forms where the tile list covers less than half of the SMs (M <= 128, or K >= 8192), from 128 rows on
+ *              664, 648 or -48 for long lists by their predicted time.
  */
 size_t bx_exact_linear_scratch_bytes(int M, int K);
+int bx_exact_linear_tile(int M, int N, int K, int residual);
 int bx_exact_linear(const int32_t* q, int64_t ldq, const int64_t* sh, const int8_t* limbs, const int64_t* d,
                     const int64_t* g, const int32_t* cnt, const int32_t* ec, const int64_t* ev, int R,
                     int8_t* scratch, int64_t* y, int32_t* flag, int M, int N, int K, int checked, int tile_rows,

@@ -36,6 +36,21 @@ def test_argument_contracts_fail_before_touching_a_device():
     assert lib.bx_exact_linear_scratch_bytes(3, 64) == 3 * 3 * 64
 
 
+def test_tile_choice_of_the_exact_linear():
+    """Forms by size, told without a device: short lists, small batches, both sides of borders between long-list forms, rows of
+    y that start off 32-byte boundaries."""
+    from bitexact_llm_b200 import _native as nv
+    tile = nv.lib().bx_exact_linear_tile
+    assert [tile(M, 3072, 2048, 1) for M in (1, 16, 17, 40, 100, 128, 193, 289, 385, 513, 577)] == \
+        [40216, 40216, 40232, 48, 32, 32, 48, 64, 648, -48, 664]
+    assert [tile(M, 2048, 8192, 1) for M in (1, 64, 128, 192, 193, 257, 865)] == [40216, 40232, 40764, 20264, 20764, 32, 664]
+    assert [tile(M, 16384, 2048, 0) for M in (1, 40, 128, 240, 241)] == [16, 48, 664, -48, 664]
+    assert tile(560, 4096, 14336, 1) == 64 and tile(576, 4096, 14336, 0) == 64
+    for M in (128, 200, 560, 1024, 4096):                    # off 32-byte boundaries with short K: never by weight rows
+        assert tile(M, 9601, 272, 0) in (-48, -32) and tile(M, 9601, 272, 1) in (-48, -32)
+    assert tile(4, 64, 100, 0) == nv.BX_EARG and tile(-1, 64, 128, 0) == nv.BX_EARG
+
+
 def test_no_product_module_imports_the_oracle():
     pkg = os.path.join(ROOT, "bitexact_llm_b200")
     for dp, _, files in os.walk(pkg):

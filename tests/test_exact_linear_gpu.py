@@ -270,8 +270,8 @@ def test_unfused_linear_api_and_bmm():
 @pytest.mark.parametrize("M,N,K", [(128, 9600, 256), (130, 9601, 272), (300, 3265, 256), (561, 2432, 1040), (748, 2048, 256),
                                    (749, 3072, 272), (2000, 600, 128)])
 def test_automatic_tiles_of_long_lists(M, N, K):
-    """Around the borders between 64 and 48 weight rows, 48 activation rows and single-wave lists: the tiles chosen by size
-    give the integers of 32 activation rows per tile."""
+    """Lists of one wave and more with short K, ragged in rows, columns and K: the tiles chosen by size give the integers of 32
+    activation rows per tile."""
     rng = np.random.RandomState(M + N)
     dec = {"limbs": rng.randint(-128, 128, (3, N, K)).astype(np.int8), "g": rng.randint(-34, -24, N).astype(np.int64),
            "d": rng.randint(0, 31, N).astype(np.int64), "rr": np.sort(rng.randint(0, N, N // 16)).astype(np.int64),
@@ -281,3 +281,27 @@ def test_automatic_tiles_of_long_lists(M, N, K):
     y, flag = _run(fl, q, sh, True, None)
     want, wflag = _run(fl, q, sh, True, 32)
     assert np.array_equal(y, want) and flag == wflag
+
+
+@pytest.mark.parametrize("M,N,K,entries,form", [
+    (384, 3072, 2048, 1, 64), (385, 3072, 2048, 1, 648), (385, 3072, 2048, 0, -48), (576, 3072, 2048, 1, -48),
+    (577, 3072, 2048, 1, 664), (240, 16384, 2048, 0, -48), (241, 16384, 2048, 0, 664), (289, 16384, 2048, 1, 648),
+    (256, 2048, 8192, 1, 20764), (257, 2048, 8192, 1, 32), (1152, 2048, 8192, 1, 664), (1153, 2048, 8192, 1, 648),
+    (160, 9601, 272, 1, -32), (161, 9601, 272, 1, -48), (624, 4096, 512, 1, -48), (625, 4096, 512, 1, 648),
+    (912, 2432, 1040, 1, -48), (913, 2432, 1040, 1, 648)])
+def test_automatic_tiles_on_both_sides_of_a_border(M, N, K, entries, form):
+    """The form told by bx_exact_linear_tile on either side of a border of the choice, with residual entries or without, gives
+    the integers of 32 activation rows per tile."""
+    from bitexact_llm_b200 import _native as nv
+    assert nv.lib().bx_exact_linear_tile(M, N, K, entries) == form
+    rng = np.random.RandomState(M + N + K)
+    n = N // 16 if entries else 0
+    dec = {"limbs": rng.randint(-128, 128, (3, N, K), dtype=np.int8), "g": rng.randint(-34, -24, N).astype(np.int64),
+           "d": rng.randint(0, 31, N).astype(np.int64), "rr": np.sort(rng.randint(0, N, n)).astype(np.int64),
+           "rc": rng.randint(0, K, n).astype(np.int64), "rv": rng.randint(-(1 << 20), 1 << 20, n).astype(np.int64)}
+    q, sh = rng.randint(-(1 << 22), 1 << 22, (M, K)).astype(np.int64), rng.randint(-45, -8, M).astype(np.int64)
+    fl = _lin(dec)
+    y, flag = _run(fl, q, sh, True, None)
+    for tile in (form, 32):
+        want, wflag = _run(fl, q, sh, True, tile)
+        assert np.array_equal(y, want) and flag == wflag, tile
