@@ -113,7 +113,7 @@ __device__ __forceinline__ uint32_t int8_weight(i64 zz, bool live, const uint8_t
 // The three signed base-256 digits of 0 <= v < 2^23 as the bytes of one word.
 __device__ __forceinline__ uint32_t limb_bytes(uint32_t v) { return (v + 0x808080u) ^ 0x808080u; }
 
-// The decode kernels' form: 4097 entries (16 KB, two to four CTAs share an SM) prepared by the caller from its table, with
+// The decode kernels' form: 4097 entries (16 KB; two CTAs share an SM, four with block tables of up to 64 keys) prepared by the caller from its table, with
 // what that form cannot say (bitexact_llm_b200/attn_table.py works both out over all entries of the full table). The
 // weight at t = factor (zz >> c) lies in [w, w + window] mtop 2^-n of the interpolated entry w, give or take `slack`, all
 // in units of 2^-32; `unsure` where a rounding boundary lies in that range.

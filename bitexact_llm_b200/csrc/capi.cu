@@ -710,52 +710,82 @@ int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_
                         (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF);
 }
 
-// Persistent streaming kernel (variants 5: 8 consumer warps, 6: 4 consumer warps). BX_ENOFIT: too few pairs or a
-// context whose scores do not fit beside the ring (the caller falls back to the cluster kernels unless the variant
-// was asked for explicitly).
 constexpr int BX_ENOFIT = -100;
-
-static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache,
-                                int64_t nb, int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt,
-                                int bt_is_int64, int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut,
-                                int64_t l2e, const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M,
-                                CompactTable ct, int min_per_sm, void* spill, size_t spill_bytes, void* stream) {
-  const bool forced = min_per_sm == 0;                          // an explicit variant: any fit will do
-  const int KEYS = 8 * NW, STAGE = KEYS * 256;
-  const int64_t max_keys = (int64_t)nblk * bs;
-  const int64_t npairs = (int64_t)R * HKV;
-  if (bs > KEYS || KEYS % bs != 0 || 32 % bs != 0) return forced ? BX_EARG : BX_ENOFIT;
-  if (!forced && npairs < 2 * 148) return BX_ENOFIT;
-  // Scores in shared memory for the whole context, or (scratch given) chunks of 512 keys with the scores of longer
-  // pairs in the caller's scratch buffer, one slice per CTA.
-  const int64_t spill_keys = (max_keys + 63) / 64 * 64;
-  const bool chunked = spill != nullptr;
 #ifndef BX_ATT_CHUNK
 #define BX_ATT_CHUNK 512
 #endif
-  const int64_t cap = chunked ? BX_ATT_CHUNK : (max_keys + KEYS - 1) / KEYS * KEYS;     // chunks: a multiple of 32 NW keys
-  if (cap / 32 > ATT6_MAXGROUPS) return forced ? BX_EARG : BX_ENOFIT;
-  int64_t fixed = 1024 + cap * 32 + (int64_t)sizeof(Attn6Small) + 1024 /* request order */;
-  int per_sm = NW == 4 ? 4 : 2, ns = 0;
-  auto stages = [&](int64_t used) { return (int)((227 * 1024 / per_sm - 1024 - used) / STAGE); };
-  for (; per_sm >= 1; --per_sm) {                               // most CTAs per SM that still leave a ring of 4 stages
-    ns = stages(fixed);
-    if (ns >= 4 || (per_sm == 1 && ns >= 3)) break;
+
+// How the persistent streaming kernel (variants 5: 8 consumer warps, 6: 4) would run.
+struct StreamPlan {
+  int warps, per_sm, stages;      // per_sm 0: it does not fit
+  bool chunked, table;            // scores of long contexts in scratch; with the compact weight table
+  int64_t cap;                    // keys whose scores stay in shared memory
+  size_t smem;
+};
+
+// chunked: scores of contexts beyond `cap` in the caller's scratch; else in shared memory for the widest context.
+static StreamPlan stream_plan(int NW, int64_t max_keys, bool chunked, bool table) {
+  const int KEYS = 8 * NW, STAGE = KEYS * 256;
+  StreamPlan p{NW, 0, 0, chunked, false, chunked ? BX_ATT_CHUNK : (max_keys + KEYS - 1) / KEYS * KEYS, 0};  // chunks: a multiple of 32 NW keys
+  if (p.cap / 32 > ATT6_MAXGROUPS) return p;
+  int64_t fixed = 1024 + p.cap * 32 + (int64_t)sizeof(Attn6Small) + 1024 /* request order */;
+  auto stages = [&](int64_t used) { return (int)((227 * 1024 / p.per_sm - 1024 - used) / STAGE); };
+  for (p.per_sm = NW == 4 ? 4 : 2; p.per_sm >= 1; --p.per_sm) {  // most CTAs per SM that still leave a ring of 4 stages
+    p.stages = stages(fixed);
+    if (p.stages >= 4 || (p.per_sm == 1 && p.stages >= 3)) break;
   }
+  if (p.per_sm < 1) return p;
   // The compact weight table where it costs neither a CTA nor the ring: 256 sequences of 512 .. 768 keys 155 -> 133 us; a
-  // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %.
-  if (ct.tab && aligned16(ct.tab) && per_sm >= 1 && stages(fixed + CT_BYTES) >= 4) {
+  // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %. With
+  // pages of 16 keys that is: tables of up to 64 keys, 592 .. 832, 1360 .. 1888, and all that are chunked.
+  p.table = table && stages(fixed + CT_BYTES) >= 4;
+  if (p.table) {
     fixed += CT_BYTES;
-    ns = stages(fixed);
-  } else {
-    ct = CompactTable{};
+    p.stages = stages(fixed);
   }
-  if (per_sm < 1) return forced ? BX_EARG : BX_ENOFIT;
-  if (!forced && per_sm < min_per_sm) return BX_ENOFIT;
-  if (ns > ATT6_MAXNS) ns = ATT6_MAXNS;
-  const size_t smem = (size_t)fixed + (size_t)ns * STAGE;
+  if (p.stages > ATT6_MAXNS) p.stages = ATT6_MAXNS;
+  p.smem = (size_t)fixed + (size_t)p.stages * STAGE;
+  return p;
+}
+
+constexpr int64_t STREAM_PAIRS = 2 * 148;         // fewer (request, KV head) pairs than this leave SMs idle: cluster kernels
+
+static bool stream_page_ok(int NW, int bs) { return bs <= 8 * NW && 8 * NW % bs == 0 && 32 % bs == 0; }
+
+// The automatic choice, by CTAs that fit on an SM beside the score buffer: four 4-warp CTAs, else two 8-warp CTAs, else two or
+// three 4-warp CTAs, else, with scratch, chunks; per_sm 0: the cluster kernels (they stream better than one CTA per SM).
+static StreamPlan stream_auto(int64_t pairs, int64_t max_keys, int bs, bool scratch, bool table) {
+  const StreamPlan none{};
+  if (pairs < STREAM_PAIRS) return none;
+  const int tries[3][2] = {{4, 4}, {8, 2}, {4, 2}};
+  for (int t = 0; t < 3; ++t) {
+    const StreamPlan p = stream_plan(tries[t][0], max_keys, false, table);
+    if (stream_page_ok(tries[t][0], bs) && p.per_sm >= tries[t][1]) return p;
+  }
+  if (!scratch) return none;
+  // Chunks. Without the compact table four 4-warp CTAs per SM serve many pairs best (us, 4 : 8 warps; 64 sequences of 64 .. 8192
+  // keys 311 : 307, 128 of 32 .. 256 / 64 .. 2048 / 64 .. 8192 39 : 45, 146 : 152, 512 : 499, 256 of the same 61 : 73, 246 : 260,
+  // 917 : 945), few pairs two of 8 warps (48 sequences of 64 .. 8192 keys 300 : 244). With it 8 warps at any number of pairs (256
+  // sequences of 64 .. 2048 / 64 .. 8192 keys 215 : 246, 731 : 917), which batches of contexts much shorter than their block
+  // table pay for (256 of 8 .. 64 / 32 .. 256 / 200 .. 600 keys 50 : 41, 68 : 61, 108 : 109); the host does not know the contexts, and
+  // a second launch that leaves at once where it is not wanted took 8 us.
+  const int NW = !table && pairs >= 1024 ? 4 : 8;
+  const StreamPlan p = stream_plan(NW, max_keys, true, table);
+  return stream_page_ok(NW, bs) && p.per_sm >= 2 ? p : none;
+}
+
+static int run_attention_stream(const StreamPlan& plan, const int32_t* q, const int64_t* sh, const int64_t* qpos,
+                                const int8_t* cache, int64_t nb, int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs,
+                                const void* bt, int bt_is_int64, int64_t sbt, int nblk, const int64_t* rmap,
+                                const int64_t* lut, int64_t l2e, const int32_t* ptab, int64_t* num, int64_t* den, int R,
+                                int HKV, int M, const CompactTable& given, void* spill, size_t spill_bytes, void* stream) {
+  const int64_t npairs = (int64_t)R * HKV;
+  const int64_t spill_keys = ((int64_t)nblk * bs + 63) / 64 * 64;
+  const int64_t grid = npairs < (int64_t)plan.per_sm * 148 ? npairs : (int64_t)plan.per_sm * 148;
+  if (spill && (size_t)grid * (size_t)spill_keys * 32 > spill_bytes) return BX_ENOFIT;      // one slice per CTA
+  const CompactTable ct = plan.table ? given : CompactTable{};
   AttnParams p{q, (const i64*)sh, (const i64*)qpos, cache, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, (int)cap, ptab, ct};
+               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, (int)plan.cap, ptab, ct};
   static PerDevice configured;
   if (once_per_device(configured, [] {
         cudaError_t e = cudaFuncSetAttribute(exact_attention_stream_kernel<8>,
@@ -782,18 +812,18 @@ static int run_attention_stream(int NW, const int32_t* q, const int64_t* sh, con
          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_64B,
          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return BX_ELAUNCH;
-  const int64_t grid = npairs < (int64_t)per_sm * 148 ? npairs : (int64_t)per_sm * 148;
-  if (chunked && (size_t)grid * (size_t)spill_keys * 32 > spill_bytes) return forced ? BX_EARG : BX_ENOFIT;
-  return launch_chained(NW == 8 ? exact_attention_stream_kernel<8> : exact_attention_stream_kernel<4>, dim3((unsigned)grid), 32 * NW + 64,
-                        (int)smem, (cudaStream_t)stream, 0, tk, tv, p, ns, npairs, (i64*)spill, spill_keys);
+  return launch_chained(plan.warps == 8 ? exact_attention_stream_kernel<8> : exact_attention_stream_kernel<4>, dim3((unsigned)grid),
+                        32 * plan.warps + 64, (int)plan.smem, (cudaStream_t)stream, 0, tk, tv, p, plan.stages, npairs, (i64*)spill,
+                        spill_keys);
 }
 
 static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
                          int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
                          int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e,
                          const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M, int HD,
-                         int cluster_size, int variant, const CompactTable& ct, void* spill, size_t spill_bytes,
+                         int cluster_size, int variant, const CompactTable& given, void* spill, size_t spill_bytes,
                          void* stream) {
+  const CompactTable ct = aligned16(given.tab) ? given : CompactTable{};
   if (!q || !qpos || !cache || !bt || !num || !den) return BX_EARG;
   if (!ptab && (!sh || !lut)) return BX_EARG;
   if (R < 0 || HKV <= 0 || M < 1 || M > 4 || HD != ATT_HD || bs <= 0 || nblk <= 0 || nb <= 0) return BX_EARG;
@@ -806,28 +836,19 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
                       sc_nb % 16 == 0 && sc_bs >= 384 && aligned16(cache);
   if (variant >= 2 && !tma_ok) return BX_EARG;
   if (variant < 0 || variant > 6 || (variant == 4 && bs > 32)) return BX_EARG;
-  // 5 / 6: persistent streaming kernel (8 / 4 consumer warps). Automatic choice, by CTAs that fit on an SM beside the
-  // score buffer: four 4-warp CTAs, else two 8-warp CTAs, else two or three 4-warp CTAs; with a single CTA per SM
-  // the cluster kernels below stream better.
-  if (variant == 0 && tma_ok) {
-    const int tries[3][2] = {{4, 4}, {8, 2}, {4, 2}};
-    for (int t = 0; t < 3; ++t) {
-      const int rc = run_attention_stream(tries[t][0], q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64,
-                                          sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, tries[t][1], nullptr, 0,
-                                          stream);
-      if (rc != BX_ENOFIT) return rc;
-    }
-    // Long contexts: chunks of 512 keys, scores in scratch. Two 8-warp CTAs per SM: against three or four of 4 warps 204 : 271 us
-    // (40 sequences of 64 .. 8192 keys), 136 : 149 us (64 of 16 .. 4096), 366 : 386 us (100 of 64 .. 8192).
-    if (spill) {
-      const int rc = run_attention_stream(8, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-                                          rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, 2, spill, spill_bytes, stream);
-      if (rc != BX_ENOFIT) return rc;
-    }
+  if (variant == 5 || variant == 6 || (variant == 0 && tma_ok)) {
+    const int NW = variant == 5 ? 8 : 4;
+    if (variant != 0 && !stream_page_ok(NW, bs)) return BX_EARG;
+    const StreamPlan plan = variant == 0 ? stream_auto((int64_t)R * HKV, max_keys, bs, spill != nullptr, ct.tab != nullptr)
+                                         : stream_plan(NW, max_keys, spill != nullptr, ct.tab != nullptr);
+    int rc = BX_ENOFIT;
+    if (plan.per_sm > 0)
+      rc = run_attention_stream(plan, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
+                                ptab, num, den, R, HKV, M, ct, plan.chunked ? spill : nullptr,
+                                spill_bytes, stream);
+    if (variant != 0) return rc == BX_ENOFIT ? BX_EARG : rc;
+    if (rc != BX_ENOFIT) return rc;
   }
-  if (variant == 5 || variant == 6)
-    return run_attention_stream(variant == 5 ? 8 : 4, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64,
-                                sbt, nblk, rmap, lut, l2e, ptab, num, den, R, HKV, M, ct, 0, spill, spill_bytes, stream);
   // 1 direct loads, 2 TMA-staged, 3 TMA + tcgen05 p.V with 8 consumer warps, 4 the same with 4 consumer warps
   const int kind = variant != 0 ? variant : (tma_ok ? ((bs <= 32 && (int64_t)R * HKV >= 64) ? 4 : 3) : 1);
   const int nw = kind == 4 ? 4 : 8;
@@ -922,6 +943,14 @@ int bx_exact_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos,
   return run_attention(q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
                        nullptr, num, den, R, HKV, M, HD, cluster_size, variant, CompactTable{}, nullptr, 0, stream);
 }
+
+int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table) {
+  if (R < 0 || HKV <= 0 || nblk <= 0 || bs <= 0) return BX_EARG;
+  const StreamPlan p = stream_auto((int64_t)R * HKV, (int64_t)nblk * bs, bs, scratch != 0, table != 0);
+  return p.per_sm == 0 ? 0 : 1000 * p.chunked + 100 * p.warps + 10 * p.per_sm + p.table;
+}
+
+int bx_attention_stream_pairs(void) { return (int)STREAM_PAIRS; }
 
 size_t bx_attention_scratch_bytes(int nblk, int bs) {
   if (nblk <= 0 || bs <= 0) return 0;

@@ -1,7 +1,7 @@
 // Row-local integer stages between the linears of exact mode: RMSNorm + quantisation, RoPE + per-head
 // quantisation + KV limb store, attention output division, SiLU * up + quantisation.
-// One CTA per row (or per token and KV head); row maxima and sums are exact integer reductions (warp shuffles,
-// then shared memory), so the thread count cannot change a bit. Bound violations set the sticky flag word.
+// One CTA per row (or per token and KV head); row maxima and sums are exact integer reductions (the warp's
+// reduce instructions, then shared memory), so the thread count cannot change a bit. Bound violations set the sticky flag word.
 //
 // Same integers as src/bitexact/exact/segs.py:49-128 and the fused kernels of
 // src/bitexact/vllm_plugin/exact_fuse.py:136-334.

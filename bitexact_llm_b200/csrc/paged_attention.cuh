@@ -1059,7 +1059,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 // key, mostly L2 traffic), and sweep 2 runs in chunks of C keys: the weights of a chunk are written as p-limb tiles
 // into the shared-memory buffer, the MMA warp consumes the chunk's V stages, and the buffer is reused for the next
 // chunk once the chunk's MMAs have completed (acc_done is committed per chunk). One CTA therefore owns a pair of
-// any length, with no cluster and no cross-CTA exchange, and the CTAs stay small enough for three or four per SM.
+// any length, with no cluster and no cross-CTA exchange, and the CTAs stay small enough for two of 8 warps or four of 4 per SM.
 //
 // V tiles: [V limb 0 | V limb 1] (cache bytes 192..319) and [V limb 1 | V limb 2] (bytes 256..383), both 128-byte
 // swizzled rows, so no byte outside the limbs is fetched; TMEM lanes 0..63 of the second accumulator repeat limb 1

@@ -12,7 +12,7 @@ from .. import attn_table
 def _scratch(device, pairs, nblk, bs):
     """Scratch for the scores of contexts beyond the shared-memory buffer of the streaming kernel: only when the
     block table is wide enough to need it and there are enough (request, KV head) pairs for that kernel."""
-    if nblk * bs <= 896 or pairs < 296:
+    if nblk * bs <= 896 or pairs < nv.lib().bx_attention_stream_pairs():
         return None, 0
     n = nv.lib().bx_attention_scratch_bytes(nblk, bs)
     return torch.empty(n, dtype=torch.uint8, device=device), n
@@ -43,7 +43,7 @@ def attend(q, sh, qpos, cache, bt, rmap, lut, l2e, nsplit=None, bn=64, warps=4, 
             cache.stride(2), cache.shape[2], bt.data_ptr(), int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
             nv.ptr(rmap.long().contiguous() if rmap is not None else None), lut.data_ptr(), int(l2e), num.data_ptr(),
             den.data_ptr(), R, HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes)
-    if compact is None or (R * HKV < 296 and variant == 0):           # below, the cluster kernels run: they use none
+    if compact is None or (variant == 0 and R * HKV < nv.lib().bx_attention_stream_pairs()):   # the cluster kernels use none
         nv.check(nv.lib().bx_exact_attention_ws(*args, nv.stream()), "bx_exact_attention_ws")
     else:
         form = attn_table.native(compact)                       # lives until the call has read it

@@ -13,7 +13,7 @@ from .. import _native as nv
 
 BM = 32     # query rows per tile (BM // G tokens): the reference's default
 BN = 64
-ROWS = 32   # query rows of a tile (16: tiles of half the height, which fill half of the kernel's rows)
+ROWS = 32   # query rows of a tile (16: tiles of half the height fill half of the kernel's rows and take twice as long per token)
 
 
 def tile_table(pre, G, bm=BM):

@@ -259,11 +259,19 @@ int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* c
                           int HD, int cluster_size, int variant, void* scratch, size_t scratch_bytes,
                           const bx_compact_table* compact, void* stream);
 
+/* What variant 0 of the attention calls runs for R x HKV (request, KV head) pairs and block tables of nblk pages of bs keys, with
+ * `scratch` and the compact `table` or without, on a cache that tensor maps can describe: 0 the
+ * cluster kernels, else the streaming kernel as 1000 (contexts in chunks, scores in scratch) + 100 x warps + 10 x CTAs per SM
+ * + 1 (it uses the table). bx_attention_stream_pairs: pairs below which it is always 0. */
+int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table);
+int bx_attention_stream_pairs(void);
+
 /* ---- prefill attention (both weight rules) -------------------------------------------------------------------------
- * Attention of whole TILES of prompt tokens: a tile is up to tile_rows / G consecutive tokens of one request; one CTA
- * per (tile, KV head) stages every K / V row once for the tile's query rows (token x G query heads), runs both integer
- * sweeps and has the limb products (scores and p.V) on tcgen05 with TMEM accumulators. tile_rows: 32 (0 selects it) or
- * 16 (tiles of half the height; the kernel's other rows stay empty). No effect on results.
+ * Attention of whole TILES of prompt tokens: a tile is up to tile_rows / G consecutive tokens of one request. One
+ * persistent CTA per SM walks the (tile, KV head) list, stages every K / V row once for the tile's query rows (token x G
+ * query heads), runs both integer sweeps and has the limb products (scores and p.V) on tcgen05 with TMEM accumulators.
+ * tile_rows: 32 (0 selects it) or 16, kept for callers with tables of shorter tiles: half of the kernel's rows stay empty,
+ * so it takes about twice as long per token. No effect on results.
  *   q      int32 [N, HKV, G, 64] token-major (|q| <= 2^22 exact mode; within three limbs int8 mode), 16-byte aligned
  *   sh     int64 [N, HKV, G] row exponents (exact mode; NULL with ptab)
  *   pos    int64 [N] position of each token: key s is visible iff s <= pos

@@ -69,3 +69,81 @@ def test_decode_attention_with_the_compact_table(mode, variant, R, HKV, M, nblk)
     want, wden = run(None)
     assert torch.equal(num, want) and torch.equal(den, wden)
     assert np.unique(den.cpu().numpy()).size > 1
+
+
+def test_where_the_automatic_choice_uses_the_table():
+    """Per block-table width in pages of 16 keys: warps, CTAs per SM, chunks and table of the streaming kernel."""
+    from bitexact_llm_b200 import _native as nv
+    plan = lambda R, keys, table: nv.lib().bx_attention_plan(R, 8, keys // 16, 16, int(keys > 896), table)
+    assert [plan(37, keys, 1) for keys in (64, 80, 576, 592, 832, 848, 1344, 1360, 1888, 1904, 2400, 2416, 8192)] == \
+        [441, 440, 440, 821, 821, 820, 820, 421, 421, 420, 420, 1821, 1821]
+    assert [plan(37, keys, 0) for keys in (64, 592, 1360, 2416, 8192)] == [440, 820, 420, 1820, 1820]
+    assert plan(127, 8192, 0) == 1820 and plan(128, 8192, 0) == 1440 and plan(256, 8192, 1) == 1821
+    assert plan(36, 784, 1) == 0 and nv.lib().bx_attention_stream_pairs() == 296
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,nblk", [(37, 1), (75, 4), (37, 37), (40, 52), (37, 85), (41, 118), (37, 151), (38, 300)])
+@pytest.mark.parametrize("mode", ["exact", "int8"])
+def test_streaming_kernel_with_the_table_equals_the_oracle(mode, R, nblk):
+    """Every form of the streaming kernel that uses the table by itself (both ends of each band of widths), and the forced
+    ones: the full table's integers for all pairs, the CPU oracle's for some; contexts of 1 key up to the whole table."""
+    from bitexact_llm_b200 import _native as nv
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
+    from oracle import exact as ox
+    from oracle import int8 as o8
+    HKV, M, bs, nb = 8, 3, 16, 401
+    assert nv.lib().bx_attention_plan(R, HKV, nblk, bs, int(nblk * bs > 896), 1) % 10 == 1
+    g = torch.Generator().manual_seed(R * nblk)
+    rng = lambda lo, hi, *n: torch.randint(lo, hi, n, generator=g)
+    bits = 18 if mode == "exact" else 13
+    k, v = (rng(-(1 << bits), 1 << bits, nb, HKV, bs, 64) >> rng(0, 4, nb, 1, 1, 1) for _ in range(2))
+    cache = tri_paged.to_limbs(torch.cat([k, v], -1).int())
+    bt = rng(1, nb, R, nblk).int()
+    pos = rng(0, nblk * bs, R, 1)
+    pos[:4, 0] = torch.tensor([nblk * bs - 1, 0, min(31, nblk * bs - 1), nblk * bs // 2])
+    qpos = (pos - rng(0, 3, R, M)).clamp(min=0)
+    q = (rng(-(1 << 20), 1 << 20, R, HKV, M, 64) >> rng(0, 6, R, HKV, M, 1)).int()
+    pick = np.array([0, 1, 2, 3, R - 1])
+    rows = [t.numpy() for t in (q[pick].long(), qpos[pick], cache, bt)]
+    if mode == "exact":
+        shift = torch.tensor([0, 1, 5, 11, 14, 16, 18, 24, 31, 32, 62])
+        sh = -6 - shift[rng(0, 11, R, HKV, M)]
+        lut = exp2_table("cuda").long()
+        run = lambda c, var=0: tri_exact_attn.attend(q.cuda(), sh.cuda(), qpos.cuda(), cache.cuda(), bt.cuda(), None, lut, L2E,
+                                                     variant=var, compact=c)
+        compact = attn_table.exact(lut, L2E)
+        want = ox.paged_attention(rows[0], sh[pick].numpy(), *rows[1:], pick, ox.exp2_table())
+    else:
+        q >>= 7
+        ptab = consts8.weight_table(consts8.exp_table()).cuda()
+        run = lambda c, var=0: tri_paged.attend(q.cuda(), qpos.cuda(), cache.cuda(), bt.cuda(), ptab, variant=var, compact=c)
+        compact = attn_table.int8(ptab)
+        want = o8.paged_attention(q[pick].long().numpy(), *rows[1:], pick, o8.exp_table())
+    compact = attn_table.to(compact, "cuda")
+    num, den = run(compact)
+    for other in (run(None), run(compact, 5), run(compact, 6), run(None, 3)):
+        assert torch.equal(num, other[0]) and torch.equal(den, other[1])
+    assert np.array_equal(num.cpu().numpy()[pick], want[0])
+    assert np.array_equal(den.cpu().numpy()[pick].reshape(want[1].shape), want[1])
+
+
+@pytest.mark.gpu
+def test_many_pairs_in_chunks_without_a_table():
+    """From 1024 pairs on 4-warp CTAs serve wide block tables for callers without a compact table."""
+    from bitexact_llm_b200 import _native as nv
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
+    R, HKV, M, bs, nblk, nb = 129, 8, 4, 16, 160, 200
+    assert nv.lib().bx_attention_plan(R, HKV, nblk, bs, 1, 0) == 1440
+    g = torch.Generator().manual_seed(5)
+    rng = lambda lo, hi, *n: torch.randint(lo, hi, n, generator=g)
+    cache = tri_paged.to_limbs((rng(-(1 << 18), 1 << 18, nb, HKV, bs, 128)).int()).cuda()
+    bt, pos = rng(1, nb, R, nblk).int().cuda(), rng(0, nblk * bs, R, 1)
+    pos[:20] = rng(0, 40, 20, 1)
+    qpos = pos.expand(-1, M).contiguous().cuda()
+    q, sh = rng(-(1 << 20), 1 << 20, R, HKV, M, 64).int().cuda(), (-6 - rng(12, 20, R, HKV, M)).cuda()
+    run = lambda var: tri_exact_attn.attend(q, sh, qpos, cache, bt, None, exp2_table("cuda").long(), L2E, variant=var)
+    num, den = run(0)
+    for var in (3, 5):
+        other = run(var)
+        assert torch.equal(num, other[0]) and torch.equal(den, other[1])
