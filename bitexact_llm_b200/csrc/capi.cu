@@ -203,10 +203,14 @@ int launch_exact_rows_one(const CUtensorMap& mact, const CUtensorMap& mwt, const
   const int w_tiles = (ep.N + TN - 1) / TN;
   const long total = (long)row_blocks * w_tiles;
   const int grid = (int)(total < sms ? total : sms);
-  // Chained whatever the length of the list: plainly, a decode step of 256 sequences took 6041 us in place of 6011; on long lists (LM
-  // head of 700 rows, 81 tiles per CTA) the two differ by less than two runs of one.
-  return launch_chained(exact_linear_rows_one_kernel<TN, NBUF>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mact, mwt, ep, K,
-                        row_blocks, w_tiles);
+  // Chained (launch_chained) while a CTA has a few tiles: a decode step of 256 sequences (3.5 tiles per CTA) took 6011 us so, 6041
+  // plainly. Plain on long lists: scoring 700 rows (LM head, 81 tiles per CTA) 1732 us plainly, 1760 chained; on other days
+  // 1505 : 1522 and 1705 : 1712.
+  if (total <= 8L * sms)
+    return launch_chained(exact_linear_rows_one_kernel<TN, NBUF>, dim3(grid), GEMM_THREADS, Cfg::SMEM_BYTES, st, 0, mact, mwt, ep, K,
+                          row_blocks, w_tiles);
+  exact_linear_rows_one_kernel<TN, NBUF><<<grid, GEMM_THREADS, Cfg::SMEM_BYTES, st>>>(mact, mwt, ep, K, row_blocks, w_tiles);
+  return launched(1);
 }
 
 template <int TA, bool POST>
