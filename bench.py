@@ -568,8 +568,8 @@ def run_b200(args, rank, world):
                      "traffic": 1.02 * alg_bytes_per_launch,
                      "traffic_note": "1.02 x the algorithmic bytes per launch computed in this run (weight limbs once + "
                                      "activation planes + int64 outputs, mean over the step's GEMM launches); the factor "
-                                     "is the ncu dram read+write / algorithmic ratio of profiles/"
-                                     "exact_linear_limb_gemm_ncu.md (102.6 MB measured vs 100.7 MB for gate/up)",
+                                     "is the dram read+write / algorithmic ratio of a profiled "
+                                     "gate/up launch (102.6 MB measured vs 100.7 MB)",
                      "algorithmic_bytes_per_launch": alg_bytes_per_launch},
         "extra": {"limb_gemm_int8_tops": achieved, "limb_gemm_ms_per_step_eager": lin_ms / K},
     }

@@ -242,7 +242,8 @@ int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* ca
 /* The same with a compact form of the weight table (4097 entries, 16 KB of shared memory per CTA) beside the table itself:
  * a weight is read off it where that decides the weight, and off the full table elsewhere, so the results are the same
  * for any table the form was made from (bitexact_llm_b200/attn_table.py: `exact`, `int8`). shift is the left shift of a
- * row distance before the product with factor; window, slack and mtop as described there. */
+ * row distance before the product with factor; window, slack and mtop as described there. A tab that does not start on a
+ * 16-byte boundary is not used. */
 typedef struct {
   const uint32_t* tab;
   uint32_t window, slack, factor, mtop;
@@ -260,9 +261,8 @@ int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* c
                           const bx_compact_table* compact, void* stream);
 
 /* What variant 0 of the attention calls runs for R x HKV (request, KV head) pairs and block tables of nblk pages of bs keys, with
- * `scratch` and the compact `table` or without, on a cache that tensor maps can describe: 0 the
- * cluster kernels, else the streaming kernel as 1000 (contexts in chunks, scores in scratch) + 100 x warps + 10 x CTAs per SM
- * + 1 (it uses the table). bx_attention_stream_pairs: pairs below which it is always 0. */
+ * `scratch` and the compact `table` or without, on a cache that tensor maps can describe: 0 the cluster kernels, else the
+ * streaming kernel as 1000 (contexts in chunks, scores in scratch) + 100 x warps + 10 x CTAs per SM + 1 (it uses the table). bx_attention_stream_pairs: pairs below which it is always 0. */
 int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table);
 int bx_attention_stream_pairs(void);
 
