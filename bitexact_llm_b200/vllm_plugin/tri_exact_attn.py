@@ -2,6 +2,7 @@
 (src/bitexact/vllm_plugin/tri_exact_attn.py:138-165)."""
 
 import ctypes
+import functools
 
 import torch
 
@@ -9,10 +10,16 @@ from .. import _native as nv
 from .. import attn_table
 
 
+@functools.lru_cache(maxsize=None)
+def stream_pairs():
+    """(request, KV head) pairs from which the streaming kernel runs: with fewer the cluster kernels do."""
+    return nv.lib().bx_attention_stream_pairs()
+
+
 def _scratch(device, pairs, nblk, bs):
     """Scratch for the scores of contexts beyond the shared-memory buffer of the streaming kernel: only when the
     block table is wide enough to need it and there are enough (request, KV head) pairs for that kernel."""
-    if nblk * bs <= 896 or pairs < nv.lib().bx_attention_stream_pairs():
+    if nblk * bs <= 896 or pairs < stream_pairs():
         return None, 0
     n = nv.lib().bx_attention_scratch_bytes(nblk, bs)
     return torch.empty(n, dtype=torch.uint8, device=device), n
@@ -43,7 +50,7 @@ def attend(q, sh, qpos, cache, bt, rmap, lut, l2e, nsplit=None, bn=64, warps=4, 
             cache.stride(2), cache.shape[2], bt.data_ptr(), int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
             nv.ptr(rmap.long().contiguous() if rmap is not None else None), lut.data_ptr(), int(l2e), num.data_ptr(),
             den.data_ptr(), R, HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes)
-    if compact is None or (variant == 0 and R * HKV < nv.lib().bx_attention_stream_pairs()):   # the cluster kernels use none
+    if compact is None or (variant == 0 and R * HKV < stream_pairs()):   # the cluster kernels use none
         nv.check(nv.lib().bx_exact_attention_ws(*args, nv.stream()), "bx_exact_attention_ws")
     else:
         form = attn_table.native(compact)                       # lives until the call has read it
