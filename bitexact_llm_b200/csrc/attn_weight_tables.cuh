@@ -66,13 +66,6 @@ __device__ __forceinline__ bool fill_int8_table(uint8_t* tab, const int32_t* __r
   return ok;
 }
 
-// A shift right that gives 0 from 32 on.
-__device__ __forceinline__ uint32_t shr_clamp(uint32_t x, uint32_t s) {
-  uint32_t r;
-  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(s));
-  return r;
-}
-
 // The exact rule's weight of a key at zz = (row maximum - score) + 2^(c - 1), for a row shift of c = 1 .. 31 bits and
 // 2^28 <= l2e < 2^29: zf = zz >> c; from zf = 2^31 on the weight is 0 (t >= 32 at 26 bits), below it t fits 32 bits.
 // With a 31-bit table w = a + ((b - a) rr >> 12) the full value lies in [w, w + 2] 2^29, and rounding is monotone:
@@ -109,9 +102,6 @@ __device__ __forceinline__ uint32_t int8_weight(i64 zz, bool live, const uint8_t
   }
   return v;
 }
-
-// The three signed base-256 digits of 0 <= v < 2^23 as the bytes of one word.
-__device__ __forceinline__ uint32_t limb_bytes(uint32_t v) { return (v + 0x808080u) ^ 0x808080u; }
 
 // The decode kernels' form: 4097 entries (16 KB; two CTAs share an SM, four with block tables of up to 64 keys) prepared by the caller from its table, with
 // what that form cannot say (bitexact_llm_b200/attn_table.py works both out over all entries of the full table). The

@@ -101,6 +101,16 @@ __device__ __forceinline__ int split8(int& r) {
   return lo;
 }
 
+// The three signed base-256 digits of v as the bytes of one word (the digits split8 gives, for every v).
+__device__ __forceinline__ uint32_t limb_bytes(uint32_t v) { return (v + 0x808080u) ^ 0x808080u; }
+
+// A shift right that gives 0 from 32 on.
+__device__ __forceinline__ uint32_t shr_clamp(uint32_t x, uint32_t s) {
+  uint32_t r;
+  asm("shr.u32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(s));
+  return r;
+}
+
 // Per-tile scalars held across the lanes of a warp: slot s of lane l holds the value of tile row (or column)
 // 32 s + l. A warp loads them once per tile, before it waits for the accumulators, and hands a value round by
 // shuffle when an output needs it: no global load remains between the accumulator read-out and the stores.

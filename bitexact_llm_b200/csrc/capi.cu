@@ -640,14 +640,21 @@ int bx_exact_norm(int mode, const void* xin, const int64_t* yin, const int64_t* 
   while ((1 << lg) < D) ++lg;
   cudaStream_t st = (cudaStream_t)stream;
   const i64* y = (const i64*)yin; const i64* id = (const i64*)ids;
-#define BX_NORM_LAUNCH(MODE, NT, EPT) \
-  return launch_chained(norm_kernel<MODE, NT, EPT>, dim3(M), NT, 0, st, 0, xin, y, id, (const i64*)gm, (const i64*)ge, (i64*)xo, q, \
-                        (i64*)sh, a8, flag, M, D, lg, do_norm)
-  if (D <= 2048) {                      // 512 threads x 4 elements
-    if (mode == 0) BX_NORM_LAUNCH(0, 512, 4); else if (mode == 1) BX_NORM_LAUNCH(1, 512, 4); else BX_NORM_LAUNCH(2, 512, 4);
-  } else {                              // 512 threads x 8 elements
-    if (mode == 0) BX_NORM_LAUNCH(0, 512, 8); else if (mode == 1) BX_NORM_LAUNCH(1, 512, 8); else BX_NORM_LAUNCH(2, 512, 8);
-  }
+  const int sms = device_sms();
+  if (sms <= 0) return BX_ELAUNCH;
+  // rows of D int64, D a multiple of 32: every access is as wide as the base pointers are aligned
+  const bool wide = aligned_to(xin, 32) && aligned_to(yin, 32) && aligned_to(gm, 32) && aligned_to(ge, 32) && aligned_to(xo, 32) &&
+                    aligned_to(q, 16) && aligned_to(a8, 4);
+#define BX_NORM_LAUNCH(MODE, NT, Q) \
+  return launch_chained(norm_kernel<MODE, NT, Q>, dim3(even_grid(M, sms * (1024 / NT))), NT, 0, st, 0, xin, y, id, (const i64*)gm, \
+                        (const i64*)ge, (i64*)xo, q, (i64*)sh, a8, flag, M, D, lg, do_norm, wide)
+#define BX_NORM_MODES(NT, Q) \
+  if (mode == 0) BX_NORM_LAUNCH(0, NT, Q); else if (mode == 1) BX_NORM_LAUNCH(1, NT, Q); else BX_NORM_LAUNCH(2, NT, Q)
+  if (D <= 512) { BX_NORM_MODES(128, 1); }
+  else if (D == 1024) { BX_NORM_MODES(256, 1); }
+  else if (D == 2048) { BX_NORM_MODES(512, 1); }
+  else { BX_NORM_MODES(512, 2); }
+#undef BX_NORM_MODES
 #undef BX_NORM_LAUNCH
 }
 
@@ -681,7 +688,12 @@ int bx_exact_attn_out(const int64_t* num, const int64_t* den, int32_t* q, int64_
       K2 / HD > AO_MAXH)
     return BX_EARG;
   if (N == 0) return BX_OK;
-  return launch_chained(attn_out_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, (const i64*)num, (const i64*)den, q, (i64*)sh, a8, N, K2, HD);
+  const i64 *nm = (const i64*)num, *dn = (const i64*)den;
+  if (HD % 4)
+    return launch_chained(attn_out_any_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, nm, dn, q, (i64*)sh, a8, N, K2, HD);
+  const bool wide = aligned_to(num, 32) && aligned_to(q, 16) && aligned_to(a8, 4);
+  return launch_chained(K2 <= 1024 ? attn_out_kernel<256, 1> : K2 <= 2048 ? attn_out_kernel<512, 1> : attn_out_kernel<512, 2>, dim3(N),
+                        K2 <= 1024 ? 256 : 512, 0, (cudaStream_t)stream, 0, nm, dn, q, (i64*)sh, a8, N, K2, HD, wide);
 }
 
 int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_t* sh, int8_t* a8, int32_t* flag,
@@ -690,24 +702,34 @@ int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_
   if (!y || !lut || !q || !sh || !flag || N < 0 || FF <= 0 || FF > SILU_THREADS * 28) return BX_EARG;
   if (N == 0) return BX_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  if (FF <= 8 * SILU_P_THREADS && N >= 64) {        // one persistent CTA per SM, 2^-f table in shared memory
+  const bool wide = aligned_to(y, 32) && aligned_to(q, 16) && aligned_to(a8, 4);
+  // Many rows: one persistent CTA per SM, 2^-f table in shared memory (copied in about 4 us); up to 128 rows a row over a
+  // cluster, with gathers from L2 (us, cluster : persistent, FF 8192: 64 rows 8.0 : 10.4, 100 rows 10.7 : 10.8, 200 rows 18.8 : 17.5;
+  // FF 4096: 64 rows 5.4 : 9.4, 256 rows 13.8 : 11.8; FF 14336: 64 rows 13.8 : 15.4).
+  if (FF % 4 == 0 && N > 128) {
     static PerDevice configured;
     const int smem = SILU_TABLE * 8;
     if (once_per_device(configured, [smem] {
-          return cudaFuncSetAttribute(silu_persistent_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+          cudaError_t e = cudaSuccess;
+          for (auto* k : {silu_persistent_kernel<256, 4>, silu_persistent_kernel<512, 2>, silu_persistent_kernel<512, 4>,
+                          silu_persistent_kernel<1024, 2>, silu_persistent_kernel<1024, 4>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+          return e;
         }) != BX_OK)
       return BX_ELAUNCH;
     const int sms = device_sms();
     if (sms <= 0) return BX_ELAUNCH;
-    // equal rounds: with 256 rows, 128 CTAs of two rows each rather than 148 CTAs of one or two
-    const int rounds = (N + sms - 1) / sms;
-    const int grid = (N + rounds - 1) / rounds;
-    return launch_chained(silu_persistent_kernel<8>, dim3(grid), SILU_P_THREADS, smem, st, 0, (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag,
-                                                                  N, FF);
+    // rows at a time in a CTA: as many as its threads can hold, but no more than the rows there are for an SM
+    const int room = FF <= 4096 ? 4 : FF <= 8192 ? 2 : 1, groups = N > 2 * sms ? room : N > sms && room > 2 ? 2 : N > sms ? room : 1;
+    auto* kernel = FF > 8192 ? silu_persistent_kernel<1024, 4> : FF > 4096 ? (groups == 2 ? silu_persistent_kernel<512, 4> : silu_persistent_kernel<1024, 2>)
+                   : groups == 4 ? silu_persistent_kernel<256, 4> : groups == 2 ? silu_persistent_kernel<512, 2> : silu_persistent_kernel<1024, 2>;
+    return launch_chained(kernel, dim3(even_grid((N + groups - 1) / groups, sms)), SILU_P_THREADS, smem, st, 0, (const i64*)y, (const i64*)lut, q,
+                          (i64*)sh, a8, flag, N, FF, wide);
   }
-  if (FF == SILU_CL * SILU_CL_THREADS * 8 && N <= 4096) {          // decode batches of the 1B model: cluster form
-    return launch_chained(silu_cluster_kernel<8>, dim3(SILU_CL * N), SILU_CL_THREADS, 0, st, SILU_CL, (const i64*)y, (const i64*)lut, q,
-                          (i64*)sh, a8, flag, N, FF);
+  if (FF % 4 == 0 && FF >= 1024) {     // decode batches: a row over a cluster
+    const int cl = N * 8 <= 148 ? 8 : 4, per = (FF / 4 + cl - 1) / cl;
+    return launch_chained(per <= SILU_CL_THREADS ? silu_cluster_kernel<1> : per <= 2 * SILU_CL_THREADS ? silu_cluster_kernel<2> : silu_cluster_kernel<4>,
+                          dim3(cl * N), SILU_CL_THREADS, 0, st, cl, (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF, wide);
   }
   const int ept = (FF + SILU_THREADS - 1) / SILU_THREADS;
   return launch_chained(ept <= 4 ? silu_kernel<4> : ept <= 16 ? silu_kernel<16> : silu_kernel<28>, dim3(N), SILU_THREADS, 0, st, 0,

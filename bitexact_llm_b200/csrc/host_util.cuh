@@ -111,7 +111,15 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+inline bool aligned_to(const void* p, int n) { return (reinterpret_cast<uintptr_t>(p) & (uintptr_t)(n - 1)) == 0; }
+inline bool aligned16(const void* p) { return aligned_to(p, 16); }
+
+// CTAs for `work` equal pieces where `most` fit at a time: equal rounds (with 256 rows on 148 SMs, 128 CTAs of two rows
+// each rather than 148 of one or two).
+inline int even_grid(int work, int most) {
+  const int rounds = (work + most - 1) / most;
+  return (work + rounds - 1) / rounds;
+}
 
 // The device status word of this library: read (synchronises), clear, write.
 inline int status_read() {
