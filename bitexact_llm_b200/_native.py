@@ -58,6 +58,7 @@ _SIGNATURES = {
     "bx_int8_qkv": (I, [P, P, P, P, P, P, L, L, L, I, P, P, P, I, I, I, I, P]),
     "bx_int8_attn_out": (I, [P, P, P, P, P, I, I, I, P]),
     "bx_int8_silu_quant": (I, [P, P, P, P, P, P, I, I, P]),
+    "bx_int8_silu_quant_tab": (I, [P, P, P, P, P, P, P, I, I, P]),
     "bx_int8_flag_end": (I, [P, P, I, P]),
     "bx_int8_silu_prod": (I, [P, P, P, P, P, I, I, P]),
     "bx_int8_quant_rows": (I, [P, P, P, P, P, I, I, P]),

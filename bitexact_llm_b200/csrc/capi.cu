@@ -696,6 +696,13 @@ int bx_exact_attn_out(const int64_t* num, const int64_t* den, int32_t* q, int64_
                         K2 <= 1024 ? 256 : 512, 0, (cudaStream_t)stream, 0, nm, dn, q, (i64*)sh, a8, N, K2, HD, wide);
 }
 
+// Rows at a time in a CTA of the persistent SiLU kernels: as many as its threads can hold, but no more than the rows there
+// are for an SM.
+static int silu_groups(int N, int FF, int sms) {
+  const int room = FF <= 4096 ? 4 : FF <= 8192 ? 2 : 1, rows = N > 2 * sms ? 4 : N > sms ? 2 : 1;
+  return room < rows ? room : rows;
+}
+
 int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_t* sh, int8_t* a8, int32_t* flag,
                         int N, int FF, void* stream) {
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
@@ -703,6 +710,8 @@ int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_
   if (N == 0) return BX_OK;
   cudaStream_t st = (cudaStream_t)stream;
   const bool wide = aligned_to(y, 32) && aligned_to(q, 16) && aligned_to(a8, 4);
+  const int sms = device_sms();
+  if (sms <= 0) return BX_ELAUNCH;
   // Many rows: one persistent CTA per SM, 2^-f table in shared memory (copied in about 4 us); up to 128 rows a row over a
   // cluster, with gathers from L2 (us, cluster : persistent, FF 8192: 64 rows 8.0 : 10.4, 100 rows 10.7 : 10.8, 200 rows 18.8 : 17.5;
   // FF 4096: 64 rows 5.4 : 9.4, 256 rows 13.8 : 11.8; FF 14336: 64 rows 13.8 : 15.4).
@@ -717,17 +726,14 @@ int bx_exact_silu_quant(const int64_t* y, const int64_t* lut, int32_t* q, int64_
           return e;
         }) != BX_OK)
       return BX_ELAUNCH;
-    const int sms = device_sms();
-    if (sms <= 0) return BX_ELAUNCH;
-    // rows at a time in a CTA: as many as its threads can hold, but no more than the rows there are for an SM
-    const int room = FF <= 4096 ? 4 : FF <= 8192 ? 2 : 1, groups = N > 2 * sms ? room : N > sms && room > 2 ? 2 : N > sms ? room : 1;
+    const int groups = silu_groups(N, FF, sms);
     auto* kernel = FF > 8192 ? silu_persistent_kernel<1024, 4> : FF > 4096 ? (groups == 2 ? silu_persistent_kernel<512, 4> : silu_persistent_kernel<1024, 2>)
                    : groups == 4 ? silu_persistent_kernel<256, 4> : groups == 2 ? silu_persistent_kernel<512, 2> : silu_persistent_kernel<1024, 2>;
     return launch_chained(kernel, dim3(even_grid((N + groups - 1) / groups, sms)), SILU_P_THREADS, smem, st, 0, (const i64*)y, (const i64*)lut, q,
                           (i64*)sh, a8, flag, N, FF, wide);
   }
   if (FF % 4 == 0 && FF >= 1024) {     // decode batches: a row over a cluster
-    const int cl = N * 8 <= 148 ? 8 : 4, per = (FF / 4 + cl - 1) / cl;
+    const int cl = N * 8 <= sms ? 8 : 4, per = (FF / 4 + cl - 1) / cl;
     return launch_chained(per <= SILU_CL_THREADS ? silu_cluster_kernel<1> : per <= 2 * SILU_CL_THREADS ? silu_cluster_kernel<2> : silu_cluster_kernel<4>,
                           dim3(cl * N), SILU_CL_THREADS, 0, st, cl, (const i64*)y, (const i64*)lut, q, (i64*)sh, a8, flag, N, FF, wide);
   }
@@ -1107,9 +1113,20 @@ int bx_int8_norm(int mode, const void* xin, const int64_t* yin, const int64_t* i
   if ((mode == 0 && !ids) || (mode == 1 && !yin) || (do_norm && (!gamma || !a8 || !mant || !e))) return BX_EARG;
   if (M == 0) return BX_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  return launch_chained(mode == 0 ? i8::int8_norm_kernel<0> : mode == 1 ? i8::int8_norm_kernel<1> : i8::int8_norm_kernel<2>, dim3(M),
-                        NORM_THREADS, 0, st, 0, xin, (const i64*)yin, (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant,
-                        (i64*)e, flag, M, D, do_norm);
+  const int sms = device_sms();
+  if (sms <= 0) return BX_ELAUNCH;
+  const bool wide = D % 4 == 0 && aligned_to(xin, 32) && aligned_to(yin, 32) && aligned_to(gamma, 32) && aligned_to(xo, 32) && aligned_to(a8, 4);
+#define BX_NORM_LAUNCH(MODE, NT, Q) \
+  return launch_chained(i8::int8_norm_kernel<MODE, NT, Q>, dim3(even_grid(M, sms * (1024 / NT))), NT, 0, st, 0, xin, (const i64*)yin, \
+                        (const i64*)ids, (const i64*)gamma, (i64*)xo, a8, (i64*)mant, (i64*)e, flag, M, D, do_norm, wide)
+#define BX_NORM_MODES(NT, Q) \
+  if (mode == 0) BX_NORM_LAUNCH(0, NT, Q); else if (mode == 1) BX_NORM_LAUNCH(1, NT, Q); else BX_NORM_LAUNCH(2, NT, Q)
+  if (D <= 512) { BX_NORM_MODES(128, 1); }
+  else if (D <= 1024) { BX_NORM_MODES(256, 1); }
+  else if (D <= 2048) { BX_NORM_MODES(512, 1); }
+  else { BX_NORM_MODES(512, 2); }
+#undef BX_NORM_MODES
+#undef BX_NORM_LAUNCH
 }
 
 int bx_int8_qkv(const int64_t* y, const int64_t* cos, const int64_t* sin, const int64_t* pos, const int64_t* slot,
@@ -1131,7 +1148,12 @@ int bx_int8_attn_out(const int64_t* num, const int64_t* den, int8_t* a8, int64_t
       K2 / HD > AO_MAXH)
     return BX_EARG;
   if (N == 0) return BX_OK;
-  return launch_chained(i8::int8_attn_out_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, (const i64*)num, (const i64*)den, a8, (i64*)mant, (i64*)e, N, K2, HD);
+  const i64 *nm = (const i64*)num, *dn = (const i64*)den;
+  if (HD % 4)
+    return launch_chained(i8::int8_attn_out_any_kernel, dim3(N), AO_THREADS, 0, (cudaStream_t)stream, 0, nm, dn, a8, (i64*)mant, (i64*)e, N, K2, HD);
+  const bool wide = aligned_to(num, 32) && aligned_to(a8, 4);
+  return launch_chained(K2 <= 1024 ? i8::int8_attn_out_kernel<256, 1> : K2 <= 2048 ? i8::int8_attn_out_kernel<512, 1> : i8::int8_attn_out_kernel<512, 2>,
+                        dim3(N), K2 <= 1024 ? 256 : 512, 0, (cudaStream_t)stream, 0, nm, dn, a8, (i64*)mant, (i64*)e, N, K2, HD, wide);
 }
 
 int bx_int8_silu_quant(const int64_t* y, const int64_t* lut, int8_t* a8, int64_t* mant, int64_t* e, int64_t* scr,
@@ -1143,6 +1165,42 @@ int bx_int8_silu_quant(const int64_t* y, const int64_t* lut, int8_t* a8, int64_t
   const int ept = (FF + SILU_THREADS - 1) / SILU_THREADS;
   return launch_chained(ept <= 4 ? i8::int8_silu_kernel<4> : ept <= 16 ? i8::int8_silu_kernel<16> : i8::int8_silu_kernel<28>, dim3(N),
                         SILU_THREADS, 0, st, 0, (const i64*)y, (const i64*)lut, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF);
+}
+
+int bx_int8_silu_quant_tab(const int64_t* y, const int64_t* lut, const uint16_t* compact, int8_t* a8, int64_t* mant, int64_t* e, int64_t* scr,
+                           int N, int FF, void* stream) {
+  if (!compact || !aligned16(compact) || FF % 4 || FF < 1024) return bx_int8_silu_quant(y, lut, a8, mant, e, scr, N, FF, stream);
+  if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
+  if (!y || !lut || !a8 || !mant || !e || N < 0 || FF > SILU_THREADS * 28) return BX_EARG;
+  if (N == 0) return BX_OK;
+  const bool wide = aligned_to(y, 32) && aligned_to(a8, 4);
+  cudaStream_t st = (cudaStream_t)stream;
+  const int sms = device_sms();
+  if (sms <= 0) return BX_ELAUNCH;
+  if (N > 128) {
+    static PerDevice configured;
+    const int smem = i8::SC_BYTES;
+    if (once_per_device(configured, [smem] {
+          cudaError_t r = cudaSuccess;
+          for (auto* k : {i8::int8_silu_persistent_kernel<256, 4>, i8::int8_silu_persistent_kernel<512, 2>, i8::int8_silu_persistent_kernel<512, 4>,
+                          i8::int8_silu_persistent_kernel<1024, 2>, i8::int8_silu_persistent_kernel<1024, 4>})
+            if (r == cudaSuccess) r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+          return r;
+        }) != BX_OK)
+      return BX_ELAUNCH;
+    const int groups = silu_groups(N, FF, sms);
+    auto* kernel = FF > 8192 ? i8::int8_silu_persistent_kernel<1024, 4>
+                   : FF > 4096 ? (groups == 2 ? i8::int8_silu_persistent_kernel<512, 4> : i8::int8_silu_persistent_kernel<1024, 2>)
+                   : groups == 4 ? i8::int8_silu_persistent_kernel<256, 4> : groups == 2 ? i8::int8_silu_persistent_kernel<512, 2>
+                                                                                         : i8::int8_silu_persistent_kernel<1024, 2>;
+    return launch_chained(kernel, dim3(even_grid((N + groups - 1) / groups, sms)), SILU_P_THREADS, smem, st, 0, (const i64*)y, (const i64*)lut,
+                          compact, a8, (i64*)mant, (i64*)e, (i64*)scr, N, FF, wide);
+  }
+  const int cl = N * 8 <= sms ? 8 : 4, per = (FF / 4 + cl - 1) / cl;
+  return launch_chained(per <= SILU_CL_THREADS ? i8::int8_silu_cluster_kernel<1> : per <= 2 * SILU_CL_THREADS ? i8::int8_silu_cluster_kernel<2>
+                                                                                                  : i8::int8_silu_cluster_kernel<4>,
+                        dim3(cl * N), SILU_CL_THREADS, 0, st, cl, (const i64*)y, (const i64*)lut, compact, a8, (i64*)mant, (i64*)e, (i64*)scr, N,
+                        FF, wide);
 }
 
 int bx_int8_silu_prod(const int64_t* y, const int64_t* lut, int64_t* h, int64_t* rowmax, int64_t* scr, int N, int FFl,

@@ -630,8 +630,7 @@ attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int32_
     for (int j = 0; j < 4; ++j) {
       v[k][j] = 0;
       if (d[k] != 0) {
-        const double hi = __hiloint2double(0x43300000, (int)(o[k][j] >> 32) ^ (int)0x80000000) - 4503601774854144.0;
-        const double y = fma(hi, 4294967296.0, u32_to_f64((uint32_t)o[k][j])) * inv;
+        const double y = fma(s32_to_f64((int)(o[k][j] >> 32)), 4294967296.0, u32_to_f64((uint32_t)o[k][j])) * inv;
         const double t = __dadd_rd(y, F2I), e = (y - (t - F2I)) - 0.5;
         const int eh = __double2hiint(e);
         v[k][j] = __double2loint(t) + 1 + (eh >> 31);

@@ -27,6 +27,7 @@ __device__ __forceinline__ i64 f64_to_int(double t) {
   return ((i64)(__double2hiint(t) - F2I_HI) << 32) | (u64)(uint32_t)__double2loint(t);
 }
 __device__ __forceinline__ double u32_to_f64(uint32_t x) { return __hiloint2double(0x43300000, (int)x) - 4503599627370496.0; }
+__device__ __forceinline__ double s32_to_f64(int x) { return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0; }
 // 2^e, -1022 <= e <= 1023.
 __device__ __forceinline__ double pow2_f64(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 // Bit length of the largest |v| from the largest high word of |v| as a double (0 for 0).

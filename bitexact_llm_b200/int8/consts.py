@@ -52,6 +52,20 @@ def silu_table():
     return torch.round(x / (1.0 + torch.exp(-x)) * (1 << FR)).long()
 
 
+def silu_compact(lut):
+    """The stage kernels' form of a SiLU table: max(x, 0) - silu(x) for |x| <= 8 as 16 bits (uint16 values in an int16 tensor,
+    padded to 16 bytes); None where an entry does not fit."""
+    half = 8 << FA
+    mid = SILU_LIM << FA
+    x = torch.arange(-half, half + 1, dtype=torch.int64, device=lut.device) << (FR - FA)
+    d = x.clamp(min=0) - lut[mid - half:mid + half + 1]
+    if lut.shape[0] != 2 * mid + 1 or bool(((d < 0) | (d > 65535)).any()):
+        return None
+    out = torch.zeros((d.shape[0] + 7) // 8 * 8, dtype=torch.int16, device=lut.device)
+    out[:d.shape[0]] = torch.where(d > 32767, d - 65536, d).to(torch.int16)
+    return out
+
+
 def weight_table(lut, fp=20):
     """Attention weight table rsh(exp table, FE - FP) as int32 (src/bitexact/vllm_plugin/tri_paged.py:351-356)."""
     return ((lut + (1 << (FE - fp - 1))) >> (FE - fp)).to(torch.int32).contiguous()

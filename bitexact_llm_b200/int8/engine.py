@@ -9,6 +9,7 @@ from .. import _native as nv
 from .. import attn_table
 from ..engine_base import TokenRowEngine
 from ..vllm_plugin import tri_fuse, tri_paged, tri_prefill
+from .consts import silu_compact
 from .gemm_skinny import linear_post
 
 
@@ -32,6 +33,7 @@ class IntEngine(TokenRowEngine):
                        for i in range(self.L)]
         self.gf, self.lm = t("gf"), lin("lm")
         self.silu_t, self.cos, self.sin, self.ln = t("silu"), t("cos"), t("sin"), t("ln")
+        self.silu_c = silu_compact(self.silu_t)              # the stage kernels' form of it
         self.ptab = tri_paged.weight_table(t("exp"))
         self.compact = attn_table.to(attn_table.int8(self.ptab), self.dev)                # the decode kernels' form of it
         self.fl = torch.zeros(1, dtype=torch.int32, device=self.dev)
@@ -69,7 +71,8 @@ class IntEngine(TokenRowEngine):
             else:
                 num, den = tri_paged.attend(q, qpos, kvs[i], bt, self.ptab, rmap=rmap, compact=self.compact)
             x, *pre = fz.add_norm(self, self._lin(fz.attn_out(self, num, den), ly["wo"]), None, None, None, x, ly["gm"])
-            a8, mant, e, _ = fz.silu_quant(self, self._lin(pre, ly["wgu"]), None, None, None, self.silu_t, scr=self.scr[i])
+            a8, mant, e, _ = fz.silu_quant(self, self._lin(pre, ly["wgu"]), None, None, None, self.silu_t, scr=self.scr[i],
+                                           compact=self.silu_c)
             nxt = self.layers[i + 1]["ga"] if i + 1 < self.L else None
             x, *pre = fz.add_norm(self, self._lin((a8, mant, e), ly["wd"]), None, None, None, x, nxt)
         fz.flag_end(self, self.scr)

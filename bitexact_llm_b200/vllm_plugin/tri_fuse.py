@@ -85,10 +85,11 @@ def attn_out(m, num, den):
     return q, mant, e
 
 
-def silu_quant(m, c, lin, mant, e, lut, scr=None):
+def silu_quant(m, c, lin, mant, e, lut, scr=None, compact=None):
     """gate_up linear output -> (limbs, mant', e', flag) of silu_mul (table SiLU, h = rsh(sg u, 16), 2-limb rows).
     scr int64 [2] (zeroed): the maxima of |sg|, |u| go there (atomic maxima) and flag is None; without scr the
-    product-bound flag is returned as a 0-d bool tensor."""
+    product-bound flag is returned as a 0-d bool tensor. compact: `int8.consts.silu_compact(lut)`, made once by a caller that
+    keeps its table (the same integers, faster)."""
     y = _y(m, c, lin, mant, e).contiguous()
     N, FF = y.shape[0], y.shape[1] // 2
     q = torch.empty(2 * N, FF, dtype=torch.int8, device=m.dev)
@@ -97,9 +98,9 @@ def silu_quant(m, c, lin, mant, e, lut, scr=None):
     own = scr is None
     if own:
         scr = torch.zeros(2, dtype=torch.long, device=m.dev)
-    rc = nv.lib().bx_int8_silu_quant(y.data_ptr(), lut.data_ptr(), q.data_ptr(), mant2.data_ptr(), e2.data_ptr(),
-                                     scr.data_ptr(), N, FF, nv.stream())
-    nv.check(rc, "bx_int8_silu_quant")
+    rc = nv.lib().bx_int8_silu_quant_tab(y.data_ptr(), lut.data_ptr(), nv.ptr(compact), q.data_ptr(), mant2.data_ptr(), e2.data_ptr(),
+                                         scr.data_ptr(), N, FF, nv.stream())
+    nv.check(rc, "bx_int8_silu_quant_tab")
     return q, mant2, e2, ((scr[0] * scr[1] >= 1 << 62) if own else None)
 
 

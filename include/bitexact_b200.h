@@ -332,6 +332,11 @@ int bx_int8_attn_out(const int64_t* num, const int64_t* den, int8_t* a8, int64_t
  * clears scr (tri_fuse.flag_end, src/bitexact/vllm_plugin/tri_fuse.py:248-265). */
 int bx_int8_silu_quant(const int64_t* y, const int64_t* lut, int8_t* a8, int64_t* mant, int64_t* e, int64_t* scr,
                        int N, int FF, void* stream);
+/* The same with the table's compact form (may be NULL): uint16 [65537] on a 16-byte boundary, readable up to 131088 bytes,
+ * max(x, 0) - lut for |x| <= 8 in steps of 2^-12 (bitexact_llm_b200.int8.consts.silu_compact). Taken where FF is a multiple of
+ * four from 1024 on; it must describe lut. */
+int bx_int8_silu_quant_tab(const int64_t* y, const int64_t* lut, const uint16_t* compact, int8_t* a8, int64_t* mant, int64_t* e, int64_t* scr,
+                           int N, int FF, void* stream);
 int bx_int8_flag_end(int64_t* scr, int32_t* flag, int L, void* stream);
 
 /* h = rsh(silu_table(gate) * up, 16) and pre_plain(h) in two steps, for a gate / up projection sharded by output column

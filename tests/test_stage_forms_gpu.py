@@ -8,6 +8,7 @@ import torch
 
 from bitexact_llm_b200 import _native as nv
 from oracle import exact as ox
+from oracle import int8 as o8
 
 pytestmark = pytest.mark.gpu
 RNG = np.random.RandomState
@@ -135,3 +136,106 @@ def test_attention_division(H, HD, N, off):
     q, a8, sh = empty((N, K2), torch.int32, off), empty((3, N, K2), torch.int8, off), empty((N,), torch.int64, 0)
     nv.check(nv.lib().bx_exact_attn_out(tn.data_ptr(), td.data_ptr(), q.data_ptr(), sh.data_ptr(), a8.data_ptr(), N, K2, HD, nv.stream()), "out")
     same(q, a8, sh, wq, wsh)
+
+
+def same8(a8, mant, e, M, want):
+    wq, wm, we = want
+    a = a8.cpu().numpy().reshape(2, M, -1).astype(np.int64)
+    assert np.array_equal(mant.cpu().numpy(), wm) and np.array_equal(e.cpu().numpy(), we)
+    assert np.array_equal(a[0] + (a[1] << 8), wq)
+
+
+@pytest.mark.parametrize("D,M,off", [(7, 3, 0), (30, 2, 0), (256, 1, 0), (700, 5, 0), (1024, 700, 0), (2048, 301, 1), (3000, 4, 0), (4096, 300, 0)])
+def test_int8_norm(D, M, off):
+    rng = RNG(D + M)
+    x = (rng.randn(M, D) * 2.0 ** rng.uniform(2, 34, (M, 1))).round().astype(np.int64)
+    y = (rng.randn(M, D) * 2.0 ** 12).round().astype(np.int64)
+    x[0], y[0] = 1 << 16, 0
+    if M > 2:
+        x[1] = y[1] = 0
+        x[2], y[2] = spread(rng, D, 50), 0                        # beyond the flag, and beyond the fast form
+    for gamma in ((4096 * (1 + 0.3 * rng.randn(D))).round().astype(np.int64), rng.randint(-(1 << 24), 1 << 24, D).astype(np.int64)):
+        if D < 256 and abs(gamma).max() > 1 << 20:
+            x[2 % M] >>= 20
+        flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+        a8, mant, e, xo = empty((2, M, D), torch.int8, off), empty((M,), torch.int64, 0), empty((M,), torch.int64, 0), empty((M, D), torch.int64, off)
+        tx, ty, tg = T(x, off), T(y, off), T(gamma, off)
+        nv.check(nv.lib().bx_int8_norm(1, tx.data_ptr(), ty.data_ptr(), None, tg.data_ptr(), xo.data_ptr(), a8.data_ptr(), mant.data_ptr(),
+                                       e.data_ptr(), flag.data_ptr(), M, D, 1, nv.stream()), "bx_int8_norm")
+        assert np.array_equal(xo.cpu().numpy(), x + y)
+        ok = [m for m in range(M) if abs(x[m] + y[m]).max() * float(abs(gamma).max()) < 2.0 ** 62]       # the oracle's own range
+        wq, wm, we = o8.pre_norm((x + y)[ok], gamma)
+        same8(a8.view(2, M, D)[:, ok], mant[ok], e[ok], len(ok), (wq, wm, we))
+
+
+@pytest.mark.parametrize("bad,want", [((1 << 42) - 1, 0), (1 << 42, 1), (-(1 << 60), 1)])
+def test_int8_sum_flag(bad, want):
+    x = np.zeros((3, 64), np.int64)
+    x[1, 17] = bad
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tx, ty, xo = T(x), T(np.zeros_like(x)), empty(x.shape, torch.int64, 0)
+    nv.check(nv.lib().bx_int8_norm(1, tx.data_ptr(), ty.data_ptr(), None, None, xo.data_ptr(), None, None, None, flag.data_ptr(), 3, 64, 0,
+                                   nv.stream()), "bx_int8_norm")
+    assert flag.item() == want and np.array_equal(xo.cpu().numpy(), x)
+
+
+@pytest.mark.parametrize("FF,N,off", [(1000, 3, 0), (1028, 2, 0), (4096, 140, 0), (4096, 400, 0), (4096, 200, 1), (8192, 1, 0), (8192, 40, 1),
+                                      (8192, 130, 0), (8192, 310, 0), (14336, 20, 0), (14336, 150, 0)])
+def test_int8_silu(FF, N, off):
+    from bitexact_llm_b200.int8.consts import silu_compact
+    rng = RNG(FF + N)
+    y = (rng.randn(N, 2 * FF) * 2.0 ** rng.uniform(8, 19, (N, 1))).round().astype(np.int64)
+    edge = 8 << 16
+    y[0, :9] = [0, edge, edge - 1, -edge, -edge - 1, -edge + 1, 32 << 16, (1 << 33) + 5, -(1 << 33)]     # the table's ends, and beyond
+    y[0, FF:FF + 9] = [(1 << 30) - 1, 1 << 30, -(1 << 30), -(1 << 30) - 1, 1 << 31, 7, -(1 << 20), 1 << 20, 3]
+    if N > 2:
+        y[1, :FF] = np.arange(FF) * (edge // 997) - 3 * edge
+        y[2] = 0
+        y[N - 1, 5], y[N - 1, FF + 5] = 32 << 16, 1 << 41                        # h beyond 2^45, in one row
+    if N > 5:
+        y[4, 9], y[4, FF + 9] = 1 << 36, -(1 << 26)                              # and 2^46
+    lut = o8.silu_table()
+    wq, wm, we, _ = o8.silu_mul(y, lut)
+    ty, tl = T(y, off), T(lut)
+    tab = silu_compact(tl)
+    a8, mant, e, scr = empty((2, N, FF), torch.int8, off), empty((N,), torch.int64, 0), empty((N,), torch.int64, 0), torch.zeros(2, dtype=torch.long, device="cuda")
+    nv.check(nv.lib().bx_int8_silu_quant_tab(ty.data_ptr(), tl.data_ptr(), tab.data_ptr(), a8.data_ptr(), mant.data_ptr(), e.data_ptr(),
+                                             scr.data_ptr(), N, FF, nv.stream()), "silu")
+    same8(a8, mant, e, N, (wq, wm, we))
+    assert scr.tolist() == [int(abs(o8.silu(y[:, :FF], lut)).max()), int(abs(y[:, FF:]).max())]
+
+
+def test_int8_silu_of_products_beyond_doubles():
+    """h of 2^51 and more: the row takes the integer rules, its neighbours do not."""
+    from bitexact_llm_b200.int8.consts import silu_compact
+    rng = RNG(0)
+    lut = o8.silu_table()
+    tl = T(lut)
+    tab = silu_compact(tl)
+    for N in (2, 300):
+        y = rng.randint(-(1 << 18), 1 << 18, (N, 8192)).astype(np.int64)
+        y[1, 70], y[1, 4096 + 70] = 1 << 36, 1 << 32                              # silu(g) = g there: h = 2^52
+        wq, wm, we, _ = o8.silu_mul(y, lut)
+        ty = T(y)
+        a8, mant, e = empty((2, N, 4096), torch.int8, 0), empty((N,), torch.int64, 0), empty((N,), torch.int64, 0)
+        nv.check(nv.lib().bx_int8_silu_quant_tab(ty.data_ptr(), tl.data_ptr(), tab.data_ptr(), a8.data_ptr(), mant.data_ptr(), e.data_ptr(), None,
+                                                 N, 4096, nv.stream()), "silu")
+        assert 2 ** 51 < (1 << 36) * (1 << 32) >> 16
+        same8(a8, mant, e, N, (wq, wm, we))
+
+
+@pytest.mark.parametrize("H,HD,N,off", [(16, 64, 1, 0), (32, 64, 3, 0), (32, 64, 500, 1), (32, 128, 9, 0), (64, 64, 2, 0), (4, 30, 3, 0)])
+def test_int8_attention_division(H, HD, N, off):
+    rng = RNG(H + N)
+    num = spread(rng, (N, H, HD), 55)
+    den = rng.randint(1 << 29, 1 << 36, (N, H, 1)).astype(np.int64)
+    num[0, 0] = 64 * (den[0, 0] // 64) * np.arange(HD) // 64
+    den[0, 1], num[0, 1] = 1 << 30, (np.arange(HD) * 2 + 1) << 27
+    if N > 2:
+        den[1] = 1 << 22                                                          # quotients from 2^29 on: the integer rules
+        den[2] = (1 << 35) - rng.randint(0, 5, (H, 1))
+    K2 = H * HD
+    tn, td = T(num, off), T(den)
+    a8, mant, e = empty((2, N, K2), torch.int8, off), empty((N,), torch.int64, 0), empty((N,), torch.int64, 0)
+    nv.check(nv.lib().bx_int8_attn_out(tn.data_ptr(), td.data_ptr(), a8.data_ptr(), mant.data_ptr(), e.data_ptr(), N, K2, HD, nv.stream()), "out")
+    same8(a8, mant, e, N, o8.attn_out(num, den))
