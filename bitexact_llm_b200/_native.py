@@ -47,6 +47,7 @@ _SIGNATURES = {
     "bx_attention_stream_pairs": (I, []),
     "bx_attention_plan": (I, [I, I, I, I, I, I]),
     "bx_attention_scratch_bytes": (Z, [I, I]),
+    "bx_attention_workspace": (Z, [I, I, I, I, I]),
     "bx_exact_attention_ws": (I, [P, P, P, P, L, L, L, L, I, P, I, L, I, P, P, L, P, P, I, I, I, I, I, I, P, Z, P]),
     "bx_int8_attention_ws": (I, [P, P, P, L, L, L, L, I, P, I, L, I, P, P, P, P, I, I, I, I, I, I, P, Z, P]),
     "bx_exact_attention_tab": (I, [P, P, P, P, L, L, L, L, I, P, I, L, I, P, P, L, P, P, I, I, I, I, I, I, P, Z, P, P]),

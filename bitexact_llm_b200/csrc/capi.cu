@@ -15,6 +15,7 @@
 #include "int8_linear_splitk.cuh"
 #include "int8_stages.cuh"
 #include "elementwise.cuh"
+#include "attention_split.cuh"
 #include "paged_attention.cuh"
 #include "prefill_attention.cuh"
 #include "sampler.cuh"
@@ -849,6 +850,59 @@ static int run_attention_stream(const StreamPlan& plan, const int32_t* q, const 
                         spill_keys);
 }
 
+// Scratch of the even split (variant 7): scores of every 64-key unit that the block tables can hold, and the pieces' maxima.
+static size_t split_bytes(int64_t pairs, int64_t max_keys, int sms) {
+  return (size_t)pairs * ((max_keys + SPL_KEYS - 1) / SPL_KEYS) * SPL_KEYS * 32 + (size_t)(pairs + 2 * sms) * 32 + (size_t)2 * sms * 16;
+}
+static int64_t split_cta_pages(int64_t pairs, int64_t max_keys, int bs, int sms) {
+  const int64_t units = pairs * ((max_keys + SPL_KEYS - 1) / SPL_KEYS);
+  return ((units + 2 * sms - 1) / (2 * sms)) * (SPL_KEYS / bs);
+}
+static bool split_can(int64_t R, int64_t HKV, int64_t max_keys, int bs, int sms) {
+  return R <= SPL_MAXREQ && bs >= 8 && SPL_KEYS % bs == 0 && split_cta_pages(R * HKV, max_keys, bs, sms) <= SPL_MAXPAGES;
+}
+
+// Where the automatic choice splits evenly, by what the host knows: pairs and the width of the block tables. The two kernels cost about
+// 9 us more than one on the smallest batches and serve every mix of lengths alike (us, before : split, 8 KV heads: 32 sequences of
+// 64 .. 8192 keys 223 : 110, 64 of 16 .. 4096 145 : 119, 100 of 100 .. 1500 111 : 84, 256 of 500 .. 1400 254 : 184, 256 of
+// 512 .. 768 145 : 138; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27). Narrower tables stay with the kernels that give
+// a pair to a CTA or a cluster (64 of 16 .. 600 37 : 45, 256 of 16 .. 200 59 : 70), and so do few pairs of up to 3072 keys (4 of 2000 25 : 27).
+// Contexts much shorter than wide tables pay for it (64 of 16 .. 100 keys in 4096 25 : 30, 32 of the same 47 : 25).
+static bool split_auto(int64_t pairs, int64_t max_keys) {
+  return max_keys > (pairs >= 1024 ? 640 : pairs >= 192 ? 896 : pairs >= 128 ? 1280 : pairs >= 64 ? 2048 : 3072);
+}
+
+static int run_attention_split(const int8_t* cache, int64_t nb, AttnParams p, int R, void* scratch, int sms, cudaStream_t st) {
+  static PerDevice configured;
+  if (once_per_device(configured, [] {
+        cudaError_t e = cudaFuncSetAttribute(attention_scores_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, split_scores_smem(SPL_MAXPAGES));
+        return e != cudaSuccess ? e
+                                : cudaFuncSetAttribute(attention_values_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, split_values_smem(SPL_MAXPAGES));
+      }) != BX_OK)
+    return BX_ELAUNCH;
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return BX_ELAUNCH;
+  CUtensorMap tk, tv;
+  cuuint64_t dims[4] = {512, (cuuint64_t)p.bs, (cuuint64_t)p.HKV, (cuuint64_t)nb};
+  cuuint64_t strides[3] = {(cuuint64_t)p.sc_bs, (cuuint64_t)p.sc_h, (cuuint64_t)p.sc_nb};
+  cuuint32_t boxk[4] = {ATT2_HALF, (cuuint32_t)p.bs, 1, 1}, boxv[4] = {128, (cuuint32_t)p.bs, 1, 1}, estr[4] = {1, 1, 1, 1};
+  if (fn(&tk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t*>(cache), dims, strides, boxk, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+      fn(&tv, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<int8_t*>(cache), dims, strides, boxv, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return BX_ELAUNCH;
+  SplitParams sp;
+  sp.a = p;
+  sp.pmax = (i64*)scratch;                               // pieces first, so that both parts are aligned
+  sp.fits = (int*)(sp.pmax + ((int64_t)R * p.HKV + 2 * sms) * 4);
+  sp.scores = (i64*)(sp.fits + 4 * 2 * sms);
+  sp.nreq = R;
+  const int pages = (int)split_cta_pages((int64_t)R * p.HKV, (int64_t)p.nblk * p.bs, p.bs, sms);
+  const int rc = launch_chained(attention_scores_kernel, dim3(2 * sms), 32 * (SPL_WARPS + 1), split_scores_smem(pages), st, 0, tk, sp);
+  if (rc != BX_OK) return rc;
+  return launch_chained(attention_values_kernel, dim3(2 * sms), 32 * (SPL_WARPS + 2), split_values_smem(pages), st, 0, tv, sp);
+}
+
 static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
                          int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
                          int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e,
@@ -867,7 +921,16 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
   const bool tma_ok = (bs % 8 == 0) && (ATT2_STAGE_KEYS % bs == 0) && sc_bs % 16 == 0 && sc_h % 16 == 0 &&
                       sc_nb % 16 == 0 && sc_bs >= 384 && aligned16(cache);
   if (variant >= 2 && !tma_ok) return BX_EARG;
-  if (variant < 0 || variant > 6 || (variant == 4 && bs > 32)) return BX_EARG;
+  if (variant < 0 || variant > 7 || (variant == 4 && bs > 32)) return BX_EARG;
+  if (variant == 7 || (variant == 0 && cluster_size == 0 && tma_ok && split_auto((int64_t)R * HKV, max_keys))) {
+    const int sms = device_sms();
+    if (sms <= 0) return BX_ELAUNCH;
+    if (split_can(R, HKV, max_keys, bs, sms) && spill && aligned16(spill) && aligned16(num) && spill_bytes >= split_bytes((int64_t)R * HKV, max_keys, sms))
+      return run_attention_split(cache, nb, AttnParams{q, (const i64*)sh, (const i64*)qpos, cache, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt,
+                                 nblk, (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, 0, ptab, ct}, R, spill, sms,
+                                 (cudaStream_t)stream);
+    if (variant == 7) return BX_EARG;
+  }
   if (variant == 5 || variant == 6 || (variant == 0 && tma_ok)) {
     const int NW = variant == 5 ? 8 : 4;
     if (variant != 0 && !stream_page_ok(NW, bs)) return BX_EARG;
@@ -988,6 +1051,18 @@ size_t bx_attention_scratch_bytes(int nblk, int bs) {
   if (nblk <= 0 || bs <= 0) return 0;
   const size_t keys = ((size_t)nblk * bs + 63) / 64 * 64;
   return (size_t)4 * 148 * keys * 32;
+}
+
+size_t bx_attention_workspace(int R, int HKV, int nblk, int bs, int variant) {
+  const int sms = device_sms();
+  if (R <= 0 || HKV <= 0 || nblk <= 0 || bs <= 0 || sms <= 0) return 0;
+  const int64_t pairs = (int64_t)R * HKV, keys = (int64_t)nblk * bs;
+  if ((variant == 7 || (variant == 0 && split_auto(pairs, keys))) && split_can(R, HKV, keys, bs, sms)) {
+    // room for the streaming kernel too: a cache that no tensor map can describe, or a forced cluster size, takes another kernel
+    const size_t even = split_bytes(pairs, keys, sms), other = bx_attention_scratch_bytes(nblk, bs);
+    return variant == 7 || pairs < STREAM_PAIRS || even > other ? even : other;
+  }
+  return keys <= 896 || pairs < STREAM_PAIRS ? 0 : bx_attention_scratch_bytes(nblk, bs);
 }
 
 int bx_exact_attention_ws(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,

@@ -2,7 +2,6 @@
 (src/bitexact/vllm_plugin/tri_exact_attn.py:138-165)."""
 
 import ctypes
-import functools
 
 import torch
 
@@ -10,19 +9,10 @@ from .. import _native as nv
 from .. import attn_table
 
 
-@functools.lru_cache(maxsize=None)
-def stream_pairs():
-    """(request, KV head) pairs from which the streaming kernel runs: with fewer the cluster kernels do."""
-    return nv.lib().bx_attention_stream_pairs()
-
-
-def _scratch(device, pairs, nblk, bs):
-    """Scratch for the scores of contexts beyond the shared-memory buffer of the streaming kernel: only when the
-    block table is wide enough to need it and there are enough (request, KV head) pairs for that kernel."""
-    if nblk * bs <= 896 or pairs < stream_pairs():
-        return None, 0
-    n = nv.lib().bx_attention_scratch_bytes(nblk, bs)
-    return torch.empty(n, dtype=torch.uint8, device=device), n
+def _scratch(device, R, HKV, nblk, bs, variant):
+    """Scratch for scores that do not stay in shared memory, as the kernels want it that this call takes."""
+    n = nv.lib().bx_attention_workspace(R, HKV, nblk, bs, variant)
+    return (torch.empty(n, dtype=torch.uint8, device=device), n) if n else (None, 0)
 
 
 def attend(q, sh, qpos, cache, bt, rmap, lut, l2e, nsplit=None, bn=64, warps=4, variant=0, compact=None):
@@ -45,12 +35,12 @@ def attend(q, sh, qpos, cache, bt, rmap, lut, l2e, nsplit=None, bn=64, warps=4, 
         cs = 1
         while cs < min(int(nsplit), 8):
             cs *= 2
-    ws, ws_bytes = _scratch(q.device, R * HKV, bt.shape[1], cache.shape[2])
+    ws, ws_bytes = _scratch(q.device, R, HKV, bt.shape[1], cache.shape[2], variant)
     args = (q.data_ptr(), sh.data_ptr(), qpos.data_ptr(), cache.data_ptr(), cache.shape[0], cache.stride(0), cache.stride(1),
             cache.stride(2), cache.shape[2], bt.data_ptr(), int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
             nv.ptr(rmap.long().contiguous() if rmap is not None else None), lut.data_ptr(), int(l2e), num.data_ptr(),
             den.data_ptr(), R, HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes)
-    if compact is None or (variant == 0 and R * HKV < stream_pairs()):   # the cluster kernels use none
+    if compact is None:
         nv.check(nv.lib().bx_exact_attention_ws(*args, nv.stream()), "bx_exact_attention_ws")
     else:
         form = attn_table.native(compact)                       # lives until the call has read it

@@ -61,13 +61,13 @@ def attend(q, qpos, cache, bt, ptab, nsplit=None, bm=None, bn=None, warps=4, rma
         cs = 1
         while cs < min(int(nsplit), 8):
             cs *= 2
-    from .tri_exact_attn import _scratch, stream_pairs
-    ws, ws_bytes = _scratch(q.device, R * HKV, bt.shape[1], cache.shape[2])
+    from .tri_exact_attn import _scratch
+    ws, ws_bytes = _scratch(q.device, R, HKV, bt.shape[1], cache.shape[2], variant)
     args = (q32.data_ptr(), qpos.data_ptr(), cache.data_ptr(), cache.shape[0], cache.stride(0), cache.stride(1), cache.stride(2),
             cache.shape[2], bt.data_ptr(), int(bt.dtype == torch.int64), bt.stride(0), bt.shape[1],
             nv.ptr(rmap.long().contiguous() if rmap is not None else None), ptab.data_ptr(), num.data_ptr(), den.data_ptr(), R,
             HKV, M, HD, cs, variant, nv.ptr(ws), ws_bytes)
-    if compact is None or (variant == 0 and R * HKV < stream_pairs()):   # the cluster kernels use none
+    if compact is None:
         nv.check(nv.lib().bx_int8_attention_ws(*args, nv.stream()), "bx_int8_attention_ws")
     else:
         form = attn_table.native(compact)                       # lives until the call has read it

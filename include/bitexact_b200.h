@@ -229,6 +229,11 @@ int bx_exact_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos,
  * whose scores do not fit in shared memory (it keeps them in the scratch, one slice per CTA, and runs its second sweep
  * in chunks of 512 keys). The buffer carries nothing between calls. NULL scratch = bx_exact_attention. */
 size_t bx_attention_scratch_bytes(int nblk, int bs);
+/* Scratch that lets the automatic choice (variant 0) take any of its kernels for R x HKV pairs, the even split over the chip
+ * included (variant 7: two kernels with the scores in scratch between them; at most 512 requests, and 1024 pages per CTA: with pages
+ * of 16 about 4.8 million keys over all pairs by table width); 0: none is of use. With less, or with scratch or num off a 16-byte
+ * boundary, the kernels described above run. */
+size_t bx_attention_workspace(int R, int HKV, int nblk, int bs, int variant);
 int bx_exact_attention_ws(const int32_t* q, const int64_t* sh, const int64_t* qpos, const int8_t* cache, int64_t nb,
                           int64_t sc_nb, int64_t sc_h, int64_t sc_bs, int bs, const void* bt, int bt_is_int64,
                           int64_t sbt, int nblk, const int64_t* rmap, const int64_t* lut, int64_t l2e, int64_t* num,
