@@ -33,7 +33,7 @@ struct ProductTable {
   double slope;         // exact: (2^-(1 / 16384) - 1) / 4096
 };
 __device__ __forceinline__ double exp2_entry(const i64* lut, int i) { return (double)__ldg(lut + i) * 8.673617379884035e-19; }      // 2^-60
-__device__ __forceinline__ void fill_products(const AttnParams& p, ProductTable& pt, double* t, int tid, int n) {
+__device__ __forceinline__ void load_products(const AttnParams& p, ProductTable& pt, double* t, int tid, int n) {
   pt.t = t;
   pt.slope = 0.0;
   if (p.ptab) {
@@ -298,7 +298,7 @@ attention_scores_kernel(const __grid_constant__ CUtensorMap tmap_k, const SplitP
 
   {
     ProductTable pt;
-    fill_products(p, pt, sm->products, threadIdx.x, 32 * SPL_WARPS);
+    load_products(p, pt, sm->products, threadIdx.x, 32 * SPL_WARPS);
     asm volatile("bar.sync 1, %0;" ::"n"(32 * SPL_WARPS) : "memory");
     const bool fits = check_products(p, pt.t, blockIdx.x, gridDim.x, threadIdx.x, 32 * SPL_WARPS);
     const bool all = split_and(fits);
@@ -437,7 +437,7 @@ attention_values_kernel(const __grid_constant__ CUtensorMap tmap_v, const SplitP
   // wait: what it reads (positions, block table, cache, tables) is complete. Its scores, maxima and cleared outputs are not before
   // the wait of the weight warps.
   ProductTable pt;
-  fill_products(p, pt, sm->products, threadIdx.x, blockDim.x);
+  load_products(p, pt, sm->products, threadIdx.x, blockDim.x);
   split_starts(p, sp.nreq, sm->start, sm->keys);
   tc_fence_before();
   __syncthreads();
@@ -490,7 +490,8 @@ attention_values_kernel(const __grid_constant__ CUtensorMap tmap_v, const SplitP
     }
     __syncwarp();
   } else {
-    // ---------------- weight warps ----------------
+    // ---------------- weight warps: from here on, what the first kernel writes ----------------
+    wait_previous();
     bool ok = true;
     const int g = lane & 3;                                            // this lane's query
     uint32_t piece = 0, wave = 0;
@@ -580,7 +581,6 @@ attention_values_kernel(const __grid_constant__ CUtensorMap tmap_v, const SplitP
         if (whole) *o = x; else add_i64(o, x);
       }
     };
-    wait_previous();
     const uint32_t l2e = (uint32_t)p.l2e;
     i64 sc[4];
     Piece q, last{};

@@ -46,7 +46,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // whoever wrote them may be the kernel in front, and its writes are visible only then (also where it permits nothing and
 // this kernel starts at its very end). The weights of a linear may be read ahead of it where the caller says that the
 // kernel in front is the stage that made the activations (`early`); for that to hold for all that ran before the stage,
-// a stage calls `launch_next` only after its own `wait_previous`. (The float library reads weights ahead in every product
+// a stage calls `launch_next` only after its own `wait_previous`. The second kernel of the split decode attention reads its inputs,
+// cache and tables ahead for the same reason: the first one is always in front of it, launched by the same call. (The float library reads weights ahead in every product
 // and permits first: include/bitexact_float.h.)
 //
 // In the integer library the row-local stages permit it: the linear or attention kernel behind them does its set-up, its

@@ -81,3 +81,32 @@ def test_split_refuses_what_it_cannot_hold():
     tri_exact_attn.attend(*[a[:512] if torch.is_tensor(a) and a.shape[0] == R else a for a in args], variant=7)
     torch.cuda.synchronize()
     assert nv.device_status() == 0
+
+
+def test_inputs_rewritten_on_the_stream():
+    """Positions, pages, keys and the weight table are overwritten by the kernels right in front of the call: the second kernel, which
+    reads them before the first one has ended, sees the newest."""
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn
+    rng = np.random.RandomState(3)
+    R, HKV, M, bs, nblk = 24, 8, 4, 16, 20
+    caches = [T(cache_planes(rng, 40, HKV, bs, 1 << 16)) for _ in range(2)]
+    bts = [T(rng.randint(1, 40, (R, nblk)).astype(np.int32)) for _ in range(2)]
+    poss = [T(np.repeat(rng.randint(0, nblk * bs, (R, 1)), M, 1).astype(np.int64)) for _ in range(2)]
+    luts = [T(ox.exp2_table()), T(ox.exp2_table() // 3)]                             # the second is no table of products
+    q, sh = T(rng.randint(-(1 << 20), 1 << 20, (R, HKV, M, HD)), torch.int32), T(rng.randint(-26, -16, (R, HKV, M)))
+    call = lambda c, b, p, l, v: tri_exact_attn.attend(q, sh, p, c, b, None, l, ox.L2E28, variant=v)
+    want = {}
+    for i in range(16):
+        pick = [x[i >> k & 1] for k, x in enumerate((caches, bts, poss, luts))]
+        want[i] = call(*pick, 3)
+    live = [x[0].clone() for x in (caches, bts, poss, luts)]
+    torch.cuda.synchronize()
+    got = []
+    for i in rng.randint(0, 16, 60):
+        for k in rng.permutation(4):
+            live[k].copy_((caches, bts, poss, luts)[k][i >> k & 1])
+        got.append((i, call(*live, 7)))
+    torch.cuda.synchronize()
+    for i, (num, den) in got:
+        assert torch.equal(num, want[i][0]) and torch.equal(den, want[i][1])
+    assert nv.device_status() == 0
