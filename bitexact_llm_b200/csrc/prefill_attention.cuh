@@ -62,7 +62,7 @@ struct PrefillParams {
   const int32_t* q;     // [N, HKV, G, 64]
   const i64* sh;        // [N, HKV, G] (exact mode; null with ptab)
   const i64* pos;       // [N] query position of each token
-  const int32_t* tiles; // [T, 3] (block-table row, first token, tokens <= 32 / G)
+  const int32_t* tiles; // [T, 3] (block-table row, first token, tokens; more than 32 / G are taken 32 / G at a time)
   const void* bt;
   int bt64;
   int64_t sbt;
@@ -153,6 +153,14 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
     *fail = 1;
   };
   auto item = [&](int64_t w) { return p.work - 1 - w; };
+  // Pieces of 32 / G tokens of work item w. Every role reads it from the list itself, so that all go through the same number
+  // of rounds (and barriers) whatever a wait came to.
+  const int per = PF_ROWS / p.G;
+  auto pieces = [&](int64_t w) -> int {
+    if (w >= p.work) return 1;
+    const int n = p.tiles[3 * (item(w) / p.HKV) + 2];
+    return n > per ? (n + per - 1) / per : 1;
+  };
 
   if (warp == PF_WARPS) {
     // ---------------- producer warp ----------------
@@ -161,12 +169,14 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
     int slot = 0, round = 0, issued = 0;
     uint32_t k = 0;
     const bool start = ok;
-    for (int64_t w = blockIdx.x; w < p.work && ok; w += gridDim.x, ++k) {
+    int piece = 0;
+    for (int64_t w = blockIdx.x; w < p.work && ok; ++k) {
       const int64_t it = item(w);
       const int h = (int)(it % p.HKV);
       const int32_t* tl = p.tiles + 3 * (it / p.HKV);
-      const int64_t brow = tl[0], tok0 = tl[1];
-      const int ntok = tl[2];
+      const int64_t brow = tl[0], tok0 = tl[1] + (int64_t)piece * per;
+      const int rest = tl[2] - piece * per, ntok = min(rest, per);
+      if (rest > per) ++piece; else { piece = 0; w += gridDim.x; }
       // ---- the tile's rows, one per lane ----
       if (k >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&sm->info_empty[k & 1], ((k >> 1) - 1) & 1));
       if (!ok) break;
@@ -258,7 +268,12 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
         ++v;
         pv_k2v0 = -1;
       };
-      for (int64_t w = blockIdx.x; w < p.work && ok; w += gridDim.x, ++k) {
+      int left = pieces(blockIdx.x);
+      for (int64_t w = blockIdx.x; w < p.work && ok; ++k) {
+        if (--left == 0) {
+          w += gridDim.x;
+          left = pieces(w);
+        }
         ok = mbar_wait(&sm->info_full[k & 1], (k >> 1) & 1);
         const int nb = ok ? sm->tile[k & 1].nb : 0;
         mbar_arrive(&sm->info_empty[k & 1]);
@@ -350,12 +365,17 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const Prefill
     const bool fits = sm->bad_table == 0;
     const uint32_t l2e = (uint32_t)p.w.l2e;
     uint32_t k = 0, s = 0, v = 0;
-    for (int64_t w = blockIdx.x; w < p.work && start; w += gridDim.x, ++k) {
+    int left = pieces(blockIdx.x);
+    for (int64_t w = blockIdx.x; w < p.work && start; ++k) {
+      if (--left == 0) {
+        w += gridDim.x;
+        left = pieces(w);
+      }
       const PrefillTile& ti = sm->tile[k & 1];
       if (ok) ok = mbar_wait(&sm->info_full[k & 1], (k >> 1) & 1);
       ok = __all_sync(0xffffffffu, ok && *fail == 0);
       const int nb = ok ? ti.nb : 0;
-      const bool last_tile = w + gridDim.x >= p.work;
+      const bool last_tile = w >= p.work;              // w is already that of the next piece
       int qmin = 0x7fffffff;                             // keys up to here are visible to the warp's 8 rows
 #pragma unroll
       for (int j = 0; j < 8; ++j) qmin = min(qmin, ti.qp[8 * group + j]);

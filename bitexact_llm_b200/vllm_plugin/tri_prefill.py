@@ -24,20 +24,6 @@ def tile_table(pre, G, bm=BM):
                         dtype=torch.int32).reshape(-1, 3)
 
 
-def _fit(tiles, G, rows):
-    """Tiles taller than the kernel's `rows` query rows are cut into pieces of rows // G tokens (on the device)."""
-    per = max(1, rows // G)
-    if tiles.shape[0] == 0 or int(tiles[:, 2].max()) <= per:
-        return tiles.contiguous()
-    t = tiles.long()
-    pieces = (t[:, 2] + per - 1) // per
-    idx = torch.repeat_interleave(torch.arange(t.shape[0], device=t.device), pieces)
-    first = torch.cumsum(pieces, 0) - pieces
-    k = torch.arange(idx.shape[0], device=t.device) - first[idx]
-    out = torch.stack([t[idx, 0], t[idx, 1] + k * per, torch.minimum(t[idx, 2] - k * per, torch.full_like(k, per))], 1)
-    return out.to(torch.int32).contiguous()
-
-
 def _run(q32, sh, pos, cache, bt, tiles, lut, l2e, ptab, num, den, rows=None):
     N, HKV, G, HD = q32.shape
     rows = ROWS if rows is None else rows
@@ -45,7 +31,7 @@ def _run(q32, sh, pos, cache, bt, tiles, lut, l2e, ptab, num, den, rows=None):
     assert HD == 64 and BM % G == 0 and cache.shape[1] == HKV and cache.shape[3] == 8 * HD and cache.stride(3) == 1
     assert bt.shape[1] * cache.shape[2] < 43690 and bt.dtype in (torch.int32, torch.int64) and bt.stride(1) == 1
     assert num.is_contiguous() and den.is_contiguous() and q32.is_contiguous() and tiles.dtype == torch.int32
-    tiles = _fit(tiles, G, rows)
+    tiles = tiles.contiguous()                               # the kernel takes taller tiles 32 // G tokens at a time
     if tiles.shape[0] == 0:
         return
     rc = nv.lib().bx_prefill_attention(q32.data_ptr(), nv.ptr(sh), pos.data_ptr(), tiles.data_ptr(), tiles.shape[0],

@@ -272,7 +272,7 @@ int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table);
 int bx_attention_stream_pairs(void);
 
 /* ---- prefill attention (both weight rules) -------------------------------------------------------------------------
- * Attention of whole TILES of prompt tokens: a tile is up to tile_rows / G consecutive tokens of one request. One
+ * Attention of whole TILES of prompt tokens: a tile is a run of consecutive tokens of one request. One
  * persistent CTA per SM walks the (tile, KV head) list, stages every K / V row once for the tile's query rows (token x G
  * query heads), runs both integer sweeps and has the limb products (scores and p.V) on tcgen05 with TMEM accumulators.
  * tile_rows: 32 (0 selects it) or 16, kept for callers with tables of shorter tiles: half of the kernel's rows stay empty,
@@ -280,7 +280,8 @@ int bx_attention_stream_pairs(void);
  *   q      int32 [N, HKV, G, 64] token-major (|q| <= 2^22 exact mode; within three limbs int8 mode), 16-byte aligned
  *   sh     int64 [N, HKV, G] row exponents (exact mode; NULL with ptab)
  *   pos    int64 [N] position of each token: key s is visible iff s <= pos
- *   tiles  int32 [n_tiles, 3] = (block-table row, first token, tokens <= tile_rows / G), on the device
+ *   tiles  int32 [n_tiles, 3] = (block-table row, first token, tokens), on the device; of more than 32 / G tokens a tile takes
+ *          32 / G at a time
  *   cache, bt, nblk, bs as bx_exact_attention (bs one of 8, 16, 32, 64, 128); lut / l2e: exact weight rule;
  *   ptab: int8-mode weight table (then lut may be NULL)
  *   num int64 [N, HKV, G, 64], den int64 [N, HKV, G]: the rows of the tiles' tokens are written, others untouched.
