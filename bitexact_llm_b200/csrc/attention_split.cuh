@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(32 * (SPL_WARPS + 2), 2)
 attention_values_kernel(const __grid_constant__ CUtensorMap tmap_v, const SplitParams sp) {
   extern __shared__ __align__(128) uint8_t att_smem[];
   const AttnParams& p = sp.a;
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(att_smem);
   uint8_t* ptile = ring + SPL_V_STAGES * SPL_V_STAGE;                  // [2 waves][8 groups][512]
   SplitValuesSmall* sm = reinterpret_cast<SplitValuesSmall*>(ptile + 2 * SPL_WAVE * SPL_PTILE);
   int* list = reinterpret_cast<int*>(sm + 1);

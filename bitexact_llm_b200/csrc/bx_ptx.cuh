@@ -24,6 +24,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The next 1024-byte boundary of dynamic shared memory, by an offset: rounded as an integer, the pointer would lose its address
+// space, and every access through it would be a generic one with a 64-bit address.
+__device__ __forceinline__ uint8_t* align_smem(uint8_t* p) { return p + ((0u - smem_u32(p)) & 1023u); }
+
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));

@@ -214,7 +214,7 @@ exact_linear_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   using Cfg = RowsCfg<TN, DBL>;
   constexpr int EPI_WARPS = 4 * EPI_GROUPS;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   PairShared* sh = reinterpret_cast<PairShared*>(ring + Cfg::STAGES * Cfg::STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5;

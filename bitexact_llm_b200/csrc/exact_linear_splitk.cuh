@@ -106,7 +106,7 @@ __device__ __forceinline__ void limb_splitk(const CUtensorMap& tmap_w, const CUt
   constexpr int NW = Epi::NW, NA = Epi::NA, NBLK = NW + NA - 1;
   using Cfg = GemmCfg<NW, NA, TA>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   GemmShared* sh = reinterpret_cast<GemmShared*>(ring + Cfg::STAGES * Cfg::STAGE_BYTES);
   i64* partial = reinterpret_cast<i64*>(ring);                        // after the main loops: [S sources][owned column][128]
 

@@ -82,7 +82,7 @@ fl_paged_attention_tc_kernel(const __grid_constant__ CUtensorMap mq, const __gri
                              const PagedAttn a, const LatentTc c) {
   constexpr int TCOLS = PARTS == 2 ? 256 : 512;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* qs = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* qs = align_smem(smem_raw);
   const int q_box = c.qrows * 128;                       // bytes of a column block of the queries
   uint8_t* ring = qs + c.kcols * q_box;
   const int stage_bytes = c.cols * LT_KEYS * 128;

@@ -223,7 +223,7 @@ fl_gemm_kernel(const __grid_constant__ CUtensorMap mw, const __grid_constant__ C
   constexpr int TCOLS = Cfg::tmem_cols(Cfg::COLS);
   static_assert(Epi::stash_bytes(TA) <= Cfg::RING_BYTES, "the epilogue's stash lies in the idle ring");
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   FlShared* sh = reinterpret_cast<FlShared*>(ring + Cfg::RING_BYTES);
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -321,7 +321,7 @@ fl_gemm_persistent_kernel(const __grid_constant__ CUtensorMap mw, const __grid_c
   static_assert(2 * Cfg::COLS <= 512 && Epi::PLANES == 1, "two accumulator buffers");
   constexpr int TCOLS = Cfg::tmem_cols(2 * Cfg::COLS);
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   FlShared* sh = reinterpret_cast<FlShared*>(ring + Cfg::RING_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total = s.n_tiles * s.m_tiles * (s.counts ? 1 : s.groups), nkb = (s.K + KE - 1) / KE;

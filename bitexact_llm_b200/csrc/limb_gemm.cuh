@@ -60,7 +60,7 @@ __device__ __forceinline__ void limb_gemm_tile(const CUtensorMap* tmap_w, const 
                                                int kb0, int kb1, const typename Epi::Params& ep, bool early = false) {
   using Cfg = GemmCfg<NW, NA, TA>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   GemmShared* sh = reinterpret_cast<GemmShared*>(ring + Cfg::STAGES * Cfg::STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void limb_gemm_persistent(const CUtensorMap* tmap_w, 
   auto w_origin = [&](int tile) { return (W_FASTEST ? tile % n_tiles : tile / m_tiles) * WROWS; };
   auto a_origin = [&](int tile) { return (W_FASTEST ? tile / n_tiles : tile % m_tiles) * TA; };
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(smem_raw);
   GemmSharedP* sh = reinterpret_cast<GemmSharedP*>(ring + Cfg::STAGES * Cfg::STAGE_BYTES);
 
   const int warp = threadIdx.x >> 5;

@@ -716,7 +716,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   constexpr int STAGE_BYTES = KEYS * 256;       // [V0|V1] tile + [V1|V2] tile (the K half uses 192 B per key)
   constexpr int CTHREADS = 32 * NW;             // consumer threads
   extern __shared__ __align__(128) uint8_t att_smem[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(att_smem);
   i64* scores = reinterpret_cast<i64*>(ring + ATT3_NS * STAGE_BYTES);   // later, in place: the p-limb tiles
   Attn3Small* sm = reinterpret_cast<Attn3Small*>(reinterpret_cast<uint8_t*>(scores) + (size_t)p.chunk_cap * 32);
 
@@ -1110,7 +1110,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
   constexpr int STAGE_BYTES = KEYS * 256;       // two V tiles of 128-byte rows (the K sweep uses 192 B per key)
   constexpr int CTHREADS = 32 * NW;             // consumer threads
   extern __shared__ __align__(128) uint8_t att_smem[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(att_smem);
   i64* scores = reinterpret_cast<i64*>(ring + (size_t)NS * STAGE_BYTES);   // later, in place: the p-limb tiles
   Attn6Small* sm = reinterpret_cast<Attn6Small*>(reinterpret_cast<uint8_t*>(scores) + (size_t)p.chunk_cap * 32);
   uint16_t* order = reinterpret_cast<uint16_t*>(sm + 1);             // requests, longest context first (or unused)

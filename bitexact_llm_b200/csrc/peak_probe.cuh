@@ -18,7 +18,7 @@ struct PeakShared {
 
 __global__ void __launch_bounds__(128, 1) i8_peak_kernel(int iters) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* base = align_smem(smem_raw);
   uint8_t* a_tile = base;                              // 128 rows x 128 bytes (four K slices), 128-byte swizzle
   uint8_t* b_tile = base + 128 * 128;                  // 256 rows x 128 bytes
   PeakShared* sh = reinterpret_cast<PeakShared*>(base + (128 + PEAK_N) * 128);

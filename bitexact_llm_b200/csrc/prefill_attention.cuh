@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1)
 prefill_attention_kernel(const __grid_constant__ CUtensorMap tmap, const PrefillParams p) {
   constexpr int NBOX = pf_boxes(EXACT);
   extern __shared__ uint8_t pf_raw[];
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pf_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = align_smem(pf_raw);
   uint8_t* qtile = ring + NBOX * PF_BOX;
   uint8_t* ptile = qtile + PF_QTILE;
   uint8_t* table = ptile + 2 * PF_PTILE;
