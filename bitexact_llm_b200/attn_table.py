@@ -6,7 +6,7 @@ memory, from which a weight is known to within a small window, and goes to the f
 lies in the window. The window is a property of the full table, worked out here over all of its entries; a table that
 such a form cannot stand for gets none (None), and the kernels then read the full table for every weight.
 
-compact = (int32 tensor of the entries, window, slack, factor from a row distance to t, its left shift, 2^(top + 1)):
+compact = (int32 tensor of the entries, in exact mode with the products of doubles behind them, window, slack, factor from a row distance to t, its left shift, 2^(top + 1)):
 window in units
 of the interpolated entry, slack (for a table that was itself rounded) in units of 2^-32 of a weight."""
 
@@ -16,6 +16,7 @@ import torch
 
 T_BITS, W_BITS = 26, 31                # fractional bits of t, bits of an entry
 STEP = 1 << 14                         # t steps per segment: 4096 segments
+ENTRIES = 4097
 
 
 class Native(ctypes.Structure):
@@ -25,7 +26,24 @@ class Native(ctypes.Structure):
 
 def native(compact):
     tab, window, slack, factor, shift, mtop = compact
-    return Native(tab.data_ptr(), window, slack, factor, mtop, shift)
+    return Native(tab.data_ptr(), window, slack, factor, mtop, shift | (256 if tab.shape[0] > ENTRIES else 0))
+
+
+def products(lut):
+    """The doubles of which the entries of a 2^-f table (int64 [16385]) are products: 2^-(i / 128), 2^-(i / 16384) and the slope between
+    entries; None where an entry is not, by the bound that csrc/attn_weight_products.cuh rounds weights by."""
+    e = lut.detach().cpu().double() * 2.0 ** -60
+    t = torch.cat([e[0:16384:128], e[:128], ((e[1] - 1.0) / 4096)[None]])
+    w = (t[:128, None] * t[None, 128:256]).reshape(-1)
+    ok = float(t[0]) == 1.0 and bool(((e[:-1] - w).abs() <= 2.0 ** -50).all()) and abs(float(e[-1]) - 0.5) <= 2.0 ** -50
+    return t if ok else None
+
+
+def _with_products(tab, lut):
+    """The entries, and behind them (from byte 16400 on) the products, with a 1 in front of them where the table has such."""
+    t = products(lut)
+    word = torch.tensor([0, 0, 0 if t is None else 1], dtype=torch.int32)
+    return torch.cat([tab, word, (torch.zeros(257, dtype=torch.float64) if t is None else t).view(torch.int32)])
 
 
 def to(compact, device):
@@ -56,7 +74,7 @@ def exact(lut, l2e):
     tab = a + (lo - 2)                 # one for the floor of the kernel's product, one for the rounding of the table's rule
     if not _fits(tab) or hi - lo > 60:
         return None
-    return tab.to(torch.int32), hi - lo + 3, 0, int(l2e) * 8, 1, 1 << 23
+    return _with_products(tab.to(torch.int32), v), hi - lo + 3, 0, int(l2e) * 8, 1, 1 << 23
 
 
 def int8(ptab):

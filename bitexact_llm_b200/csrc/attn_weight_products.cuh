@@ -3,13 +3,14 @@
 // Both weight tables are exponentials, so an entry is the product of two of 128 (exact rule: 2^-f in steps of 2^-7 and 2^-14) or of
 // 512 and 256 (int8 rule: e^z in steps of 2^-4 and 2^-12) doubles in shared memory, 2 and 6 KB for 131 and 524, and a weight
 // is known to 2^-27 (exact rule) or to the 2^-11 that its table was rounded by before (int8 rule). Nearer to a rounding boundary than
-// 2^-21 / 2^-10 the table itself decides. The kernels hold every entry of the caller's table against the products (the split decode
-// attention a slice per CTA of its first kernel, the prefill kernel all of the exact rule's in every CTA), so the form serves any
-// caller, and a table of another kind takes the general rule.
+// 2^-21 / 2^-10 the table itself decides. A table is known to be of this kind because every entry was held against the products: by the
+// caller that prepared them (attn_table.py, the kernels that give a pair to a CTA or a cluster), or by the first kernel of the split
+// decode attention, a slice per CTA. A table of another kind takes the general rule.
+// Measured in the second kernel of the split attention, 32 sequences of 64 .. 8192 keys: 85 us with the 4097 entries of
+// attn_weight_tables.cuh, which leave 1 % of the weights near the maximum undecided (most warps then gather from L2), 66 us so.
 #pragma once
 
 #include "attn_weight_tables.cuh"
-#include "paged_attention.cuh"
 #include "stage_math.cuh"
 
 namespace bx {
@@ -18,38 +19,46 @@ constexpr int PW_EXACT = 128, PW_INT8 = 512, PW_DOUBLES = 768;
 constexpr int PW_LAST = 131072;                                        // int8 rule: entry of z = 0
 
 struct ProductTable {
-  double* t;            // shared memory: exact 2^-(i / 128), 2^-(i / 16384); int8 ptab[last] e^-(i / 16), e^-(i / 4096)
+  const double* t;      // shared memory: exact 2^-(i / 128), 2^-(i / 16384); int8 ptab[last] e^-(i / 16), e^-(i / 4096)
   double slope;         // exact: (2^-(1 / 16384) - 1) / 4096
 };
 __device__ __forceinline__ double exp2_entry(const i64* lut, int i) { return (double)__ldg(lut + i) * 8.673617379884035e-19; }      // 2^-60
-__device__ __forceinline__ void load_products(const AttnParams& p, ProductTable& pt, double* t, int tid, int n) {
+__device__ __forceinline__ void load_products(const i64* lut, const int32_t* ptab, ProductTable& pt, double* t, int tid, int n) {
   pt.t = t;
   pt.slope = 0.0;
-  if (p.ptab) {
-    const double top = (double)__ldg(p.ptab + PW_LAST);
+  if (ptab) {
+    const double top = (double)__ldg(ptab + PW_LAST);
     for (int i = tid; i < PW_INT8 + 256; i += n) t[i] = i < PW_INT8 ? top * exp(-i / 16.0) : exp(-(i - PW_INT8) / 4096.0);
   } else {
-    for (int i = tid; i < 2 * PW_EXACT; i += n) t[i] = exp2_entry(p.lut, i < PW_EXACT ? i * PW_EXACT : i - PW_EXACT);
-    pt.slope = (exp2_entry(p.lut, 1) - 1.0) * (1.0 / 4096);
+    for (int i = tid; i < 2 * PW_EXACT; i += n) t[i] = exp2_entry(lut, i < PW_EXACT ? i * PW_EXACT : i - PW_EXACT);
+    pt.slope = (exp2_entry(lut, 1) - 1.0) * (1.0 / 4096);
   }
 }
+// The same of the exact rule from a caller's copy that says whether it has found them to be its table's (bitexact_llm_b200/attn_table.py):
+// the slope behind them, and in front of them a word that is 1 where they are; otherwise pt.t is null.
+__device__ __forceinline__ void copy_products(const double* src, ProductTable& pt, double* t, int tid, int n) {
+  for (int i = tid; i < 2 * PW_EXACT; i += n) t[i] = __ldg(src + i);
+  pt.t = __ldg(reinterpret_cast<const int*>(src) - 1) == 1 ? t : nullptr;
+  pt.slope = __ldg(src + 2 * PW_EXACT);
+}
+constexpr int PW_EXACT_BYTES = 8 * 2 * PW_EXACT;
 // Entries [part of parts) of the caller's table against the products.
-__device__ __forceinline__ bool check_products(const AttnParams& p, const double* t, int part, int parts, int tid, int n) {
+__device__ __forceinline__ bool check_products(const i64* lut, const int32_t* ptab, i64 l2e, const double* t, int part, int parts, int tid,
+                                               int n) {
   bool ok = true;
-  if (p.ptab) {
+  if (ptab) {
 #pragma unroll 4
     for (int i = part * n + tid; i <= PW_LAST; i += parts * n) {
-      const int v = __ldg(p.ptab + (PW_LAST - i));
+      const int v = __ldg(ptab + (PW_LAST - i));
       const double w = i < PW_LAST ? t[i >> 8] * t[PW_INT8 + (i & 255)] : 0.0;
       ok &= v >= 0 && v <= (1 << 22) && fabs((double)v - w) <= 0.50048828125;              // 1/2 + 2^-11
     }
   } else {
-#pragma unroll 8
     for (int i = part * n + tid; i <= 1 << EXP2_BITS; i += parts * n) {
       const double w = i < 1 << EXP2_BITS ? t[i >> 7] * t[PW_EXACT + (i & 127)] : 0.5;
-      ok &= fabs(exp2_entry(p.lut, i) - w) <= 8.881784197001252e-16;                       // 2^-50
+      ok &= fabs(exp2_entry(lut, i) - w) <= 8.881784197001252e-16;                       // 2^-50
     }
-    ok &= t[0] == 1.0 && p.l2e >= (1ll << 28) && p.l2e < (1ll << 29);
+    ok &= t[0] == 1.0 && l2e >= (1ll << 28) && l2e < (1ll << 29);
   }
   return ok;
 }

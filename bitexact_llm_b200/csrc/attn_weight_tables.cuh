@@ -111,6 +111,7 @@ __device__ __forceinline__ uint32_t int8_weight(i64 zz, bool live, const uint8_t
 // 45, of which the two 32-bit gathers from shared memory take 14.
 struct CompactTable {
   const uint32_t* tab;          // null: none
+  const double* products;       // attn_weight_products.cuh, in place of tab (null: none)
   uint32_t window, slack, factor, mtop;
   int shift;
 };

@@ -757,7 +757,8 @@ struct StreamPlan {
 };
 
 // chunked: scores of contexts beyond `cap` in the caller's scratch; else in shared memory for the widest context.
-static StreamPlan stream_plan(int NW, int64_t max_keys, bool chunked, bool table) {
+// table: bytes of the weight table's form in shared memory, 0: none.
+static StreamPlan stream_plan(int NW, int64_t max_keys, bool chunked, int table) {
   const int KEYS = 8 * NW, STAGE = KEYS * 256;
   StreamPlan p{NW, 0, 0, chunked, false, chunked ? BX_ATT_CHUNK : (max_keys + KEYS - 1) / KEYS * KEYS, 0};  // chunks: a multiple of 32 NW keys
   if (p.cap / 32 > ATT6_MAXGROUPS) return p;
@@ -771,9 +772,9 @@ static StreamPlan stream_plan(int NW, int64_t max_keys, bool chunked, bool table
   // The compact weight table where it costs neither a CTA nor the ring: 256 sequences of 512 .. 768 keys 155 -> 133 us; a
   // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %. With
   // pages of 16 keys that is: tables of up to 64 keys, 592 .. 832, 1360 .. 1888, and all that are chunked.
-  p.table = table && stages(fixed + CT_BYTES) >= 4;
+  p.table = table && stages(fixed + table) >= 4;
   if (p.table) {
-    fixed += CT_BYTES;
+    fixed += table;
     p.stages = stages(fixed);
   }
   if (p.stages > ATT6_MAXNS) p.stages = ATT6_MAXNS;
@@ -787,7 +788,7 @@ static bool stream_page_ok(int NW, int bs) { return bs <= 8 * NW && 8 * NW % bs 
 
 // The automatic choice, by CTAs that fit on an SM beside the score buffer: four 4-warp CTAs, else two 8-warp CTAs, else two or
 // three 4-warp CTAs, else, with scratch, chunks; per_sm 0: the cluster kernels (they stream better than one CTA per SM).
-static StreamPlan stream_auto(int64_t pairs, int64_t max_keys, int bs, bool scratch, bool table) {
+static StreamPlan stream_auto(int64_t pairs, int64_t max_keys, int bs, bool scratch, int table) {
   const StreamPlan none{};
   if (pairs < STREAM_PAIRS) return none;
   const int tries[3][2] = {{4, 4}, {8, 2}, {4, 2}};
@@ -805,6 +806,12 @@ static StreamPlan stream_auto(int64_t pairs, int64_t max_keys, int bs, bool scra
   const int NW = !table && pairs >= 1024 ? 4 : 8;
   const StreamPlan p = stream_plan(NW, max_keys, true, table);
   return stream_page_ok(NW, bs) && p.per_sm >= 2 ? p : none;
+}
+
+// shift: bit 8 says that the products lie behind the entries.
+static CompactTable compact_table(const bx_compact_table* c) {
+  const double* products = c->shift & 256 ? reinterpret_cast<const double*>(c->tab + CT_BYTES / 4) : nullptr;
+  return CompactTable{c->tab, products, c->window, c->slack, c->factor, c->mtop, c->shift & 255};
 }
 
 static int run_attention_stream(const StreamPlan& plan, const int32_t* q, const int64_t* sh, const int64_t* qpos,
@@ -865,11 +872,11 @@ static bool split_can(int64_t R, int64_t HKV, int64_t max_keys, int bs, int sms)
 // Where the automatic choice splits evenly, by what the host knows: pairs and the width of the block tables. The two kernels cost about
 // 9 us more than one on the smallest batches and serve every mix of lengths alike (us, before : split, 8 KV heads: 32 sequences of
 // 64 .. 8192 keys 223 : 110, 64 of 16 .. 4096 145 : 119, 100 of 100 .. 1500 111 : 84, 256 of 500 .. 1400 254 : 184, 256 of
-// 512 .. 768 145 : 138; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27). Narrower tables stay with the kernels that give
+// 512 .. 768 145 : 138, of 500 .. 620 129 : 119; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27). Narrower tables stay with the kernels that give
 // a pair to a CTA or a cluster (64 of 16 .. 600 37 : 45, 256 of 16 .. 200 59 : 70), and so do few pairs of up to 3072 keys (4 of 2000 25 : 27).
 // Contexts much shorter than wide tables pay for it (64 of 16 .. 100 keys in 4096 25 : 30, 32 of the same 47 : 25).
 static bool split_auto(int64_t pairs, int64_t max_keys) {
-  return max_keys > (pairs >= 1024 ? 640 : pairs >= 192 ? 896 : pairs >= 128 ? 1280 : pairs >= 64 ? 2048 : 3072);
+  return max_keys > (pairs >= 1024 ? 512 : pairs >= 192 ? 896 : pairs >= 128 ? 1280 : pairs >= 64 ? 2048 : 3072);
 }
 
 static int run_attention_split(const int8_t* cache, int64_t nb, AttnParams p, int R, void* scratch, int sms, cudaStream_t st) {
@@ -909,7 +916,12 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
                          const int32_t* ptab, int64_t* num, int64_t* den, int R, int HKV, int M, int HD,
                          int cluster_size, int variant, const CompactTable& given, void* spill, size_t spill_bytes,
                          void* stream) {
-  const CompactTable ct = aligned16(given.tab) ? given : CompactTable{};
+  CompactTable ct = aligned16(given.tab) ? given : CompactTable{};
+  // The products of the exact rule (2 KB) everywhere; an int8 weight is one entry of its table, which the 16 KB form serves better than
+  // 6 KB of products do (us, 64 sequences of 16 .. 600 keys 35 : 37, 4 of 16 .. 2000 20 : 22).
+  if (ptab) ct.products = nullptr;
+  if (ct.products) ct.tab = nullptr;
+  const int table = ct.products ? PW_EXACT_BYTES : ct.tab ? CT_BYTES : 0;
   if (!q || !qpos || !cache || !bt || !num || !den) return BX_EARG;
   if (!ptab && (!sh || !lut)) return BX_EARG;
   if (R < 0 || HKV <= 0 || M < 1 || M > 4 || HD != ATT_HD || bs <= 0 || nblk <= 0 || nb <= 0) return BX_EARG;
@@ -934,8 +946,8 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
   if (variant == 5 || variant == 6 || (variant == 0 && tma_ok)) {
     const int NW = variant == 5 ? 8 : 4;
     if (variant != 0 && !stream_page_ok(NW, bs)) return BX_EARG;
-    const StreamPlan plan = variant == 0 ? stream_auto((int64_t)R * HKV, max_keys, bs, spill != nullptr, ct.tab != nullptr)
-                                         : stream_plan(NW, max_keys, spill != nullptr, ct.tab != nullptr);
+    const StreamPlan plan = variant == 0 ? stream_auto((int64_t)R * HKV, max_keys, bs, spill != nullptr, table)
+                                         : stream_plan(NW, max_keys, spill != nullptr, table);
     int rc = BX_ENOFIT;
     if (plan.per_sm > 0)
       rc = run_attention_stream(plan, q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
@@ -948,7 +960,7 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
   const int kind = variant != 0 ? variant : (tma_ok ? ((bs <= 32 && (int64_t)R * HKV >= 64) ? 4 : 3) : 1);
   const int nw = kind == 4 ? 4 : 8;
   const bool use_tma = kind >= 2;
-  const int64_t fixed = kind >= 3 ? 1024 + (int64_t)ATT3_NS * (8 * nw * 256) + (int64_t)sizeof(Attn3Small)
+  const int64_t fixed = kind >= 3 ? 1024 + (int64_t)ATT3_NS * (8 * nw * 256) + (int64_t)sizeof(Attn3Small) + (ct.products ? table : 0)
                         : kind == 2 ? (int64_t)ATT2_NS * ATT2_STAGE_BYTES + (int64_t)sizeof(Attn2Small)
                                     : (int64_t)sizeof(AttnShared);
   const int64_t gran = kind >= 3 ? 8 * nw : use_tma ? ATT2_STAGE_KEYS : 8;
@@ -967,7 +979,7 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
   if (chunk_cap > cap_limit) return BX_EARG;
   const size_t smem = (size_t)fixed + (size_t)chunk_cap * 32;
   AttnParams p{q, (const i64*)sh, (const i64*)qpos, cache, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk,
-               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, chunk_cap, ptab, CompactTable{}};
+               (const i64*)rmap, (const i64*)lut, (i64)l2e, (i64*)num, (i64*)den, M, HKV, chunk_cap, ptab, kind >= 3 && ct.products ? ct : CompactTable{}};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((int64_t)cs * R * HKV), 1, 1);
   cfg.blockDim = dim3(kind == 4 ? 160 : use_tma ? ATT2_THREADS : ATT_THREADS, 1, 1);
@@ -1041,7 +1053,7 @@ int bx_exact_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos,
 
 int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table) {
   if (R < 0 || HKV <= 0 || nblk <= 0 || bs <= 0) return BX_EARG;
-  const StreamPlan p = stream_auto((int64_t)R * HKV, (int64_t)nblk * bs, bs, scratch != 0, table != 0);
+  const StreamPlan p = stream_auto((int64_t)R * HKV, (int64_t)nblk * bs, bs, scratch != 0, table ? CT_BYTES : 0);
   return p.per_sm == 0 ? 0 : 1000 * p.chunked + 100 * p.warps + 10 * p.per_sm + p.table;
 }
 
@@ -1103,7 +1115,7 @@ int bx_exact_attention_tab(const int32_t* q, const int64_t* sh, const int64_t* q
                            size_t scratch_bytes, const bx_compact_table* compact, void* stream) {
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!sh || !lut || !compact) return BX_EARG;
-  const CompactTable ct{compact->tab, compact->window, compact->slack, compact->factor, compact->mtop, compact->shift};
+  const CompactTable ct = compact_table(compact);
   return run_attention(q, sh, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, lut, l2e,
                        nullptr, num, den, R, HKV, M, HD, cluster_size, variant, ct, scratch, scratch_bytes, stream);
 }
@@ -1115,7 +1127,7 @@ int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* c
                           const bx_compact_table* compact, void* stream) {
   if (g_status_seen.load(std::memory_order_relaxed)) return BX_EDEVICE;
   if (!ptab || !compact) return BX_EARG;
-  const CompactTable ct{compact->tab, compact->window, compact->slack, compact->factor, compact->mtop, compact->shift};
+  const CompactTable ct = compact_table(compact);
   return run_attention(q, nullptr, qpos, cache, nb, sc_nb, sc_h, sc_bs, bs, bt, bt_is_int64, sbt, nblk, rmap, nullptr,
                        0, ptab, num, den, R, HKV, M, HD, cluster_size, variant, ct, scratch, scratch_bytes, stream);
 }

@@ -20,6 +20,7 @@
 
 #include <cooperative_groups.h>
 
+#include "attn_weight_products.cuh"
 #include "attn_weight_tables.cuh"
 #include "bx_ptx.cuh"
 #include "bx_rules.cuh"
@@ -54,7 +55,7 @@ struct AttnParams {
   int M, HKV;
   int chunk_cap;        // score slots per query row in shared memory (multiple of 8)
   const int32_t* ptab;  // int8 mode: weight table rsh(e^z table, 10), 131073 entries; null = exact mode
-  CompactTable ct;      // shared-memory form of either table (the streaming kernel); tab null: none
+  CompactTable ct;      // shared-memory form of either table (streaming and tcgen05 cluster kernels); both null: none
 };
 
 struct AttnShared {
@@ -126,23 +127,26 @@ __device__ __forceinline__ i64 fragment_score(const int (&acc)[3][4], int lane) 
 struct WeightRow {
   i64 mx, mxh, rowshift;      // maximum; with the rounding term of the row shift
   int c, hs;
-  bool fast;                  // the compact table serves the row
+  bool fast;                  // the compact table or the products serve the row
 };
-__device__ __forceinline__ WeightRow weight_row(const AttnParams& p, i64 mx, i64 rowshift) {
+__device__ __forceinline__ WeightRow weight_row(const AttnParams& p, const ProductTable& prod, i64 mx, i64 rowshift) {
   WeightRow r;
   r.mx = mx;
   r.rowshift = rowshift;
-  r.fast = p.ct.tab != nullptr && (p.ptab || (rowshift >= 1 && rowshift <= 31));
+  r.fast = (p.ct.tab || prod.t) && (p.ptab || (rowshift >= 1 && rowshift <= 31));
   r.c = p.ptab ? WT_INT8_SHIFT : r.fast ? (int)rowshift : 1;
   r.hs = p.ptab ? 4 : r.c - 1;
   r.mxh = mx + (p.ptab ? (1ll << (WT_INT8_SHIFT - 1)) - 1 : 1ll << (r.c - 1));
   return r;
 }
 // The weights of 4 keys (live: visible) of one query from their scores.
-__device__ __forceinline__ void four_weights(const AttnParams& p, const WeightRow& row, const uint32_t* tab, const i64 (&sc)[4],
-                                             const bool (&live)[4], uint32_t (&pv)[4]) {
+__device__ __forceinline__ void four_weights(const AttnParams& p, const WeightRow& row, const uint32_t* tab, const ProductTable& prod,
+                                             const i64 (&sc)[4], const bool (&live)[4], uint32_t (&pv)[4]) {
   bool redo[4];
-  if (row.fast) {
+  if (row.fast && prod.t) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) pv[j] = product_weight(prod, (uint32_t)p.l2e, row.mxh - sc[j], row.c, live[j], redo[j]);
+  } else if (row.fast) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) pv[j] = compact_weight(p.ct, tab, row.mxh - sc[j], row.c, row.hs, live[j], redo[j]);
   } else {
@@ -719,6 +723,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   uint8_t* ring = align_smem(att_smem);
   i64* scores = reinterpret_cast<i64*>(ring + ATT3_NS * STAGE_BYTES);   // later, in place: the p-limb tiles
   Attn3Small* sm = reinterpret_cast<Attn3Small*>(reinterpret_cast<uint8_t*>(scores) + (size_t)p.chunk_cap * 32);
+  double* products = reinterpret_cast<double*>(sm + 1);                 // the weight products, if there are any
 
   cg::cluster_group cluster = cg::this_cluster();
   const int CS = (int)cluster.num_blocks();
@@ -745,6 +750,8 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     tmem_relinquish();
   }
   wait_previous();
+  ProductTable prod{};
+  if (p.ct.products) copy_products(p.ct.products, prod, products, threadIdx.x, blockDim.x);
   i64 kend = 0;
   for (int g = 0; g < p.M; ++g) kend = imax(kend, p.qpos[r * p.M + g] + 1);
   kend = imin(kend, (i64)p.nblk * p.bs);
@@ -906,7 +913,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const bool gok = g2 < p.M;
   const i64 qp2 = gok ? p.qpos[r * p.M + g2] : -1;
   const i64 rowshift = (gok && p.sh) ? (i64)(FK + 3 - FZ) - p.sh[pz * p.M + g2] : 0;
-  const WeightRow wrow = weight_row(p, mx, rowshift);
+  const WeightRow wrow = weight_row(p, prod, mx, rowshift);
   i64 den = 0;
   const int ngroups = (int)((hi - lo + 31) / 32);
   for (int grp = warp; grp < ngroups; grp += NW) {
@@ -922,7 +929,7 @@ exact_attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
       const i64 key = lo + (i64)grp * 32 + 8 * j + (lane >> 2);
       live[j] = key < hi && key <= qp2;
     }
-    four_weights(p, wrow, nullptr, sc, live, pv);
+    four_weights(p, wrow, nullptr, prod, sc, live, pv);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int kl = 8 * j + (lane >> 2);
@@ -1114,7 +1121,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
   i64* scores = reinterpret_cast<i64*>(ring + (size_t)NS * STAGE_BYTES);   // later, in place: the p-limb tiles
   Attn6Small* sm = reinterpret_cast<Attn6Small*>(reinterpret_cast<uint8_t*>(scores) + (size_t)p.chunk_cap * 32);
   uint16_t* order = reinterpret_cast<uint16_t*>(sm + 1);             // requests, longest context first (or unused)
-  uint32_t* ctab = reinterpret_cast<uint32_t*>(order + 512);         // the compact weight table, if there is one
+  uint32_t* ctab = reinterpret_cast<uint32_t*>(order + 512);         // the compact weight table or the products, if there are any
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int C = p.chunk_cap;                                          // keys whose scores / p tiles fit in shared memory
   const int GPC = C / 32;                                             // 32-key groups per chunk (a multiple of NW)
@@ -1142,6 +1149,8 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     return imin(imax(kend, 0), (i64)p.nblk * p.bs);
   };
   if (p.ct.tab && threadIdx.x == 0) fetch_compact(ctab, p.ct, &sm->table_full);
+  ProductTable prod{};
+  if (p.ct.products) copy_products(p.ct.products, prod, reinterpret_cast<double*>(ctab), threadIdx.x, blockDim.x);
   if (ranked) {
     // Requests by context length, longest first, in buckets of 128 keys (ties by index): a counting sort whose
     // placement step runs in one warp over 32 requests at a time (match_any gives each lane its place among the lanes
@@ -1421,7 +1430,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
     const bool gok = g2 < p.M;
     const i64 qp2 = gok ? p.qpos[r * p.M + g2] : -1;
     const i64 rowshift = (gok && p.sh) ? (i64)(FK + 3 - FZ) - p.sh[pz * p.M + g2] : 0;
-    const WeightRow wrow = weight_row(p, mx, rowshift);
+    const WeightRow wrow = weight_row(p, prod, mx, rowshift);
     i64 den = 0;
     const int ngroups = (int)((hi + 31) / 32);
     const int nchunks = (ngroups + GPC - 1) / GPC;
@@ -1451,7 +1460,7 @@ exact_attention_stream_kernel(const __grid_constant__ CUtensorMap tmap_k, const 
           const i64 key = (i64)grp * 32 + 8 * j + (lane >> 2);
           live[j] = key < hi && key <= qp2;
         }
-        four_weights(p, wrow, ctab, sc, live, pv);
+        four_weights(p, wrow, ctab, prod, sc, live, pv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int kl = 8 * j + (lane >> 2);

@@ -248,7 +248,9 @@ int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* ca
  * a weight is read off it where that decides the weight, and off the full table elsewhere, so the results are the same
  * for any table the form was made from (bitexact_llm_b200/attn_table.py: `exact`, `int8`). shift is the left shift of a
  * row distance before the product with factor; window, slack and mtop as described there. A tab that does not start on a
- * 16-byte boundary is not used. */
+ * 16-byte boundary is not used. Bit 8 of shift (exact rule): from byte 16400 of tab on lie the 257 doubles of which every table
+ * entry is a product (`products` there), which the kernels use in place of the entries where the 32-bit word in front of them is 1,
+ * and the full table where it is not. */
 typedef struct {
   const uint32_t* tab;
   uint32_t window, slack, factor, mtop;

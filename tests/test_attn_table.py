@@ -147,3 +147,19 @@ def test_many_pairs_in_chunks_without_a_table():
     for var in (3, 5):
         other = run(var)
         assert torch.equal(num, other[0]) and torch.equal(den, other[1])
+
+
+def test_products_are_the_tables_they_stand_for():
+    """The doubles behind a compact table: every entry within the bound that weights are rounded by, and the mark of a table that
+    is none of products."""
+    lut = exp2_table("cpu").long()
+    t = attn_table.products(lut)
+    i = torch.arange(16384)
+    for rr in (0, 1, 2048, 4095):
+        v = lut[i].double() * 2.0 ** -60 + (lut[i + 1] - lut[i]).double() * rr * 2.0 ** -72
+        w = t[i >> 7] * t[128 + (i & 127)]
+        assert bool(((w + w * (t[256] * rr) - v).abs() <= 2.0 ** -49).all())      # a weight of 22 bits to 2^-27
+    other = (lut >> 1) + (1 << 58)
+    assert attn_table.products(other) is None
+    a, b = attn_table.exact(lut, L2E)[0], attn_table.exact(other, L2E)[0]
+    assert a.shape == b.shape and int(a[4099]) == 1 and int(b[4099]) == 0
