@@ -55,6 +55,9 @@ _SIGNATURES = {
     "bx_exact_attention": (I, [P, P, P, P, L, L, L, L, I, P, I, L, I, P, P, L, P, P, I, I, I, I, I, I, P]),
     "bx_int8_attention": (I, [P, P, P, L, L, L, L, I, P, I, L, I, P, P, P, P, I, I, I, I, I, I, P]),
     "bx_prefill_attention": (I, [P, P, P, P, I, P, L, L, L, L, I, P, I, L, I, P, L, P, P, P, I, I, I, I, P]),
+    "bx_forward_bytes": (Z, [I, I, I, I, I, I, I, I, I, I]),
+    "bx_exact_forward": (I, [P, P, P]),
+    "bx_int8_forward": (I, [P, P, P]),
     "bx_int8_norm": (I, [I, P, P, P, P, P, P, P, P, P, I, I, I, P]),
     "bx_int8_qkv": (I, [P, P, P, P, P, P, L, L, L, I, P, P, P, I, I, I, I, P]),
     "bx_int8_attn_out": (I, [P, P, P, P, P, I, I, I, P]),
@@ -93,6 +96,13 @@ _SIGNATURES = {
     "bx_logp_finish": (I, [P, P, P, P, I, I, P]),
 }
 
+
+
+class Step(ctypes.Structure):
+    """bx_step."""
+    _fields_ = [(n, P) for n in ("emb", "ids", "pos", "qpos", "slot", "bt", "rmap", "tiles", "cos", "sin", "lut", "ptab", "silu", "silu_compact",
+                                 "scr", "compact", "num", "den", "x", "flag", "work")] + \
+               [(n, L) for n in ("layers", "N", "D", "H", "HKV", "HD", "FF", "bs", "bt64", "sbt", "nblk", "l2e", "n_tiles", "work_bytes")]
 
 
 class Epilogue(ctypes.Structure):

@@ -1787,3 +1787,5 @@ int bx_exact_linear_static(const int32_t* q, int64_t ldq, const int64_t* sh, con
 }
 
 }  // extern "C"
+
+#include "forward.cuh"

@@ -3,6 +3,8 @@ reference's plugin (src/bitexact/vllm_plugin/graph.py:69-87 `_decode_fused`, vll
 rules of `IntLlama` (src/bitexact/int8/model.py:25-133). Nine kernels per layer: fused int8 linear (GEMM + post),
 qkv, attention, attn_out, linear, add_norm, linear, silu_quant, linear, add_norm."""
 
+import ctypes
+
 import torch
 
 from .. import _native as nv
@@ -24,6 +26,7 @@ class IntEngine(TokenRowEngine):
         self.H = cfg.get("num_attention_heads", 32)
         self.HKV = cfg.get("num_key_value_heads", 8)
         self.HD = cfg.get("head_dim") or self.D // self.H
+        self.FF = cfg.get("intermediate_size", 8192)
         self.L = c["n_layers"] if n_layers is None else n_layers
         t = lambda k: c[k].to(self.dev).contiguous()
         self.emb = t("emb")
@@ -57,8 +60,11 @@ class IntEngine(TokenRowEngine):
         """Same contract as ExactEngine.forward; returns the residual stream int64 [N, D] at 16 bits."""
         fz = tri_fuse
         N, G = ids.shape[0], self.H // self.HKV
-        pos = pos.long()
-        slot = torch.where(slot < 0, torch.zeros_like(slot), slot).long()
+        pos = pos.long().contiguous()
+        slot = torch.where(slot < 0, torch.zeros_like(slot), slot).long().contiguous()
+        x = self._forward_native(kvs, ids.long(), pos, slot, bt, rmap, tiles)
+        if x is not None:
+            return x
         qpos = pos.view(-1, 1).expand(-1, G).contiguous()
         x, *pre = fz.embed_norm(self, ids, self.layers[0]["ga"])
         for i in range(self.L):
@@ -77,6 +83,21 @@ class IntEngine(TokenRowEngine):
             x, *pre = fz.add_norm(self, self._lin((a8, mant, e), ly["wd"]), None, None, None, x, nxt)
         fz.flag_end(self, self.scr)
         return x
+
+    def _forward_native(self, kvs, ids, pos, slot, bt, rmap, tiles):
+        if self.timer is not None or rmap is None:               # a timer brackets every linear by itself
+            return None
+        rows = []
+        for ly in self.layers[:self.L]:
+            row = []
+            for n in ("wqkv", "wo", "wgu", "wd"):
+                w, mul, fmsh = ly[n]
+                row += (w.data_ptr(), mul.data_ptr(), int(fmsh), w.shape[0], w.shape[1])
+            rows.append(row + [ly["ga"].data_ptr(), ly["gm"].data_ptr()])
+        form = None if self.compact is None else attn_table.native(self.compact)       # lives until the call has read it
+        fields = dict(ptab=self.ptab.data_ptr(), silu=self.silu_t.data_ptr(), silu_compact=nv.ptr(self.silu_c), scr=self.scr.data_ptr(),
+                      compact=None if form is None else ctypes.addressof(form))
+        return self.forward_native("bx_int8_forward", False, fields, rows, kvs, ids, pos, slot, bt, rmap, tiles)
 
     def logits(self, h):
         """Final residual rows [M, D] -> int64 logits [M, V] at 16 bits."""

@@ -442,6 +442,59 @@ int bx_sample(const int64_t* logits, int64_t ld, const int64_t* rows, const int6
 int bx_sample_shard(const int64_t* logits, int64_t ld, const int64_t* rows, const int64_t* lnt, void* scratch,
                     int64_t* best, int64_t* idx, int M, int V_local, int64_t v_offset, int bits, void* stream);
 
+/* ---- all layers of a forward call ---------------------------------------------------------------------------------
+ * The stages, linears and attention calls above for every layer, in the order of ExactEngine.forward and IntEngine.forward
+ * (bitexact_llm_b200/vllm_plugin/exact_run.py, int8/engine.py), from one call: x int64 [N, D] receives the residual rows. Every pointer
+ * is one that the single calls take; work: bx_forward_bytes(..) bytes on a 256-byte boundary, which carry nothing between
+ * calls. N rows: ids, pos, slot [N], qpos [N, H / HKV] and rmap [N] (decode attention; rmap may be NULL), or tiles [n_tiles, 3] with
+ * num [N, H, HD] and den [N, H] that hold what rows outside the tiles are to have (0 and 1). HD 64. The weights of a layer must be
+ * complete before the call. Errors of a single call are returned as they are; what was launched before them runs. */
+typedef struct {
+  const int8_t* limbs;
+  const int64_t *d, *g;
+  const int32_t *cnt, *ec;
+  const int64_t* ev;
+  int64_t R, N, K, tile_rows;
+} bx_exact_lin;
+typedef struct {
+  bx_exact_lin wqkv, wo, wgu, wd;
+  const int64_t *ga_m, *ga_e, *gm_m, *gm_e;
+  int8_t* cache;
+  int64_t nb, sc_nb, sc_h, sc_bs;
+} bx_exact_layer;
+typedef struct {
+  const int8_t* w;
+  const int64_t* mul;
+  int64_t fmsh, N, K;
+} bx_int8_lin;
+typedef struct {
+  bx_int8_lin wqkv, wo, wgu, wd;
+  const int64_t *ga, *gm;
+  int8_t* cache;
+  int64_t nb, sc_nb, sc_h, sc_bs;
+} bx_int8_layer;
+typedef struct {
+  const int32_t* emb;
+  const int64_t *ids, *pos, *qpos, *slot;
+  const void* bt;
+  const int64_t* rmap;
+  const int32_t* tiles;
+  const int64_t *cos, *sin, *lut;          /* lut: exact mode */
+  const int32_t* ptab;                     /* ptab, silu, silu_compact (may be NULL), scr [layers, 2]: int8 mode */
+  const int64_t* silu;
+  const uint16_t* silu_compact;
+  int64_t* scr;
+  const bx_compact_table* compact;         /* may be NULL */
+  int64_t *num, *den;                      /* with tiles */
+  int64_t* x;
+  int32_t* flag;
+  void* work;
+  int64_t layers, N, D, H, HKV, HD, FF, bs, bt64, sbt, nblk, l2e, n_tiles, work_bytes;
+} bx_step;
+size_t bx_forward_bytes(int exact, int N, int D, int H, int HKV, int HD, int FF, int nblk, int bs, int tiles);
+int bx_exact_forward(const bx_step* step, const bx_exact_layer* layers, void* stream);
+int bx_int8_forward(const bx_step* step, const bx_int8_layer* layers, void* stream);
+
 /* ---- weight preparation (load time) ----------------------------------------------------------------------------
  * bf16 weights w [N, K] (raw 16-bit patterns, row stride ldw) -> the constants of the exact-mode linear layer:
  * limbs int8 [3][N][K], per-row grid exponent g and residual depth d (int64 [N]), cnt int32 [N] = residual entries
