@@ -87,9 +87,17 @@ class Session:
                     i += 1
             if not runs:
                 continue
-            seq = torch.cat([torch.full((len(t),), s) for _, s, _, t in runs]).to(dev)
-            pos = torch.cat([torch.arange(n, n + len(t)) for _, _, n, t in runs]).to(dev)
-            ids = torch.cat([t for _, _, _, t in runs]).to(dev)
+            # everything that the step has to know of its rows goes over in one copy
+            many = torch.tensor([[s, n, len(t)] for _, s, n, t in runs])
+            counts = many[:, 2]
+            first = torch.cumsum(counts, 0) - counts
+            table = torch.empty(3, at, dtype=torch.long)
+            table[0] = torch.repeat_interleave(many[:, 0], counts)
+            table[1] = torch.arange(at) + torch.repeat_interleave(many[:, 1] - first, counts)
+            torch.cat([t.cpu() for _, _, _, t in runs], out=table[2])
+            ends = torch.cat([many[:, 0], many[:, 1] + counts])
+            both = torch.cat([table.reshape(-1), ends]).to(dev)
+            seq, pos, ids = both[:3 * at].view(3, at)
             tt, row = [], 0
             for _, s, n, t in runs:
                 tt.append((s, row, len(t), n + len(t)))
@@ -99,11 +107,11 @@ class Session:
             x = self.eng.forward(self.kvs, ids, pos, self._slots(seq, pos), self.bt, seq,
                                  tiles=None if tt is None else tt.to(dev))
             row = 0
-            for e, s, n, t in runs:
+            for e, _, _, t in runs:
                 out[e].append(x[row:row + len(t)])
                 row += len(t)
-                self.lens[s] = n + len(t)
-        return [torch.cat(o) if o else torch.empty(0, self.eng.D, device=dev) for o in out]
+            self.lens[both[3 * at:3 * at + len(runs)]] = both[3 * at + len(runs):]
+        return [o[0] if len(o) == 1 else torch.cat(o) if o else torch.empty(0, self.eng.D, device=dev) for o in out]
 
     def _slots(self, seq, pos):
         return self.bt[seq, pos // self.bs].long() * self.bs + pos % self.bs

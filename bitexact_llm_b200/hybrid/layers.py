@@ -14,6 +14,7 @@ import torch
 
 from .. import _native as nv
 from . import ops
+from ..vllm_plugin.tri_prefill import cut_runs
 
 
 @dataclass
@@ -49,8 +50,6 @@ class Tiles:
     @classmethod
     def of(cls, runs, sizes):
         """runs = [(table row, first token row, tokens, context length)], sizes: the tile heights in use."""
-        table = lambda n: torch.tensor([[r, t0 + s, min(n, ql - s)] for r, t0, ql, _ in runs for s in range(0, ql, n)],
-                                       dtype=torch.int32).reshape(-1, 3)
         size = cls.SEGMENT if sum(ql for _, _, ql, _ in runs) >= 4096 else cls.SEGMENT // 2
         per_run, chunks, segments, spans = [], [], [], []
         for _, t0, ql, _ in runs:
@@ -59,11 +58,20 @@ class Tiles:
             segments += [[t0 + s, min(size, ql - s), len(chunks) + s // cls.CHUNK] for s in range(0, ql, size)]
             chunks += [[t0 + s, min(cls.CHUNK, ql - s)] for s in range(0, ql, cls.CHUNK)]
         tensor = lambda rows, n: torch.tensor(rows, dtype=torch.int32).reshape(-1, n)
-        return cls({n: table(n) for n in sizes}, tensor(per_run, 3), tensor(chunks, 2), tensor(segments, 3), tensor(spans, 3))
+        return cls({n: cut_runs(runs, n) for n in sizes}, tensor(per_run, 3), tensor(chunks, 2), tensor(segments, 3), tensor(spans, 3))
 
     def to(self, dev):
-        return Tiles({n: t.to(dev) for n, t in self.attention.items()},
-                     *(t.to(dev) for t in (self.runs, self.chunks, self.segments, self.spans)))
+        every = [*self.attention.values(), self.runs, self.chunks, self.segments, self.spans]
+        at = [0]
+        for t in every:
+            at.append(at[-1] + (t.numel() + 31) // 32 * 32)         # each on a boundary of its own
+        packed = torch.empty(at[-1], dtype=torch.int32)
+        for t, o in zip(every, at):
+            packed[o:o + t.numel()] = t.reshape(-1)
+        packed = packed.to(dev)                                     # one copy
+        moved = [packed[o:o + t.numel()].view(t.shape) for t, o in zip(every, at)]
+        n = len(self.attention)
+        return Tiles(dict(zip(self.attention, moved[:n])), *moved[n:])
 
     def chunked(self, K, V, rows):
         """Whether a recurrence of these sizes runs in chunks: portions of a few rows are shorter row by row."""

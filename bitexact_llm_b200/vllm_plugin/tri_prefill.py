@@ -19,9 +19,20 @@ ROWS = 32   # query rows of a tile (16: tiles of half the height fill half of th
 def tile_table(pre, G, bm=BM):
     """[T, 3] int32 (request, first token, tokens) of the bm // G-token tiles of the prefill requests
     pre = [(req, tok0, qlen, seq_len)], on the host."""
-    bt_ = max(1, min(bm, 32) // G)
-    return torch.tensor([[r, t0 + s, min(bt_, ql - s)] for r, t0, ql, _ in pre for s in range(0, ql, bt_)],
-                        dtype=torch.int32).reshape(-1, 3)
+    return cut_runs(pre, max(1, min(bm, 32) // G))
+
+
+def cut_runs(pre, n):
+    """[T, 3] int32 (request, first token, tokens): the runs of pre = [(req, tok0, qlen, ..)] in pieces of n tokens."""
+    if len(pre) == 0:
+        return torch.empty(0, 3, dtype=torch.int32)
+    run = torch.tensor([p[:3] for p in pre], dtype=torch.int32)
+    pieces = (run[:, 2] + n - 1) // n
+    out = torch.repeat_interleave(run, pieces, dim=0)
+    at = n * (torch.arange(out.shape[0], dtype=torch.int32) - torch.repeat_interleave(torch.cumsum(pieces, 0).int() - pieces, pieces))
+    out[:, 1] += at
+    out[:, 2] = torch.clamp(out[:, 2] - at, max=n)
+    return out
 
 
 def _run(q32, sh, pos, cache, bt, tiles, lut, l2e, ptab, num, den, rows=None):
