@@ -1407,7 +1407,7 @@ static void logp_plan(int M, int V, int& ch, int& nch) {
 }
 
 size_t bx_logp_scratch_bytes(int M, int V) {
-  return (size_t)2 * 8 * (size_t)(M > 0 ? M : 0) * sample_chunks(M, V > 0 ? V : 1);
+  return (size_t)(2 * 8 + 4) * (size_t)(M > 0 ? M : 0) * sample_chunks(M, V > 0 ? V : 1);      // maxima, sums, and a word per CTA
 }
 
 static bool logp_args_ok(const void* lg, int64_t ld, const void* scratch, int M, int V) {
@@ -1429,7 +1429,7 @@ int bx_logp_rowmax(const int64_t* logits, int64_t ld, void* scratch, int64_t* ro
   logp_plan(M, V, ch, nch);
   cudaStream_t st = (cudaStream_t)stream;
   i64* pmax = (i64*)scratch;
-  logp_max_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, pmax, V, ch, nch);
+  logp_max_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, pmax, V, ch, nch, nullptr, nullptr);
   logp_rowfold_kernel<<<(M + 127) / 128, 128, 0, st>>>(pmax, nch, (i64*)rowmax, M, 0);
   return launched(2);
 }
@@ -1446,7 +1446,7 @@ int bx_logp_rowsum(const int64_t* logits, int64_t ld, const int64_t* rowmax, con
   cudaStream_t st = (cudaStream_t)stream;
   i64* psum = (i64*)scratch;
   logp_sum_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, (const i64*)rowmax, nullptr, 0, nullptr,
-                                                        (const longlong2*)tab2, psum, V, ch, nch, fr);
+                                                        (const longlong2*)tab2, nullptr, psum, V, ch, nch, fr);
   logp_rowfold_kernel<<<(M + 127) / 128, 128, 0, st>>>(psum, nch, (i64*)S, M, 1);
   return launched(2);
 }
@@ -1473,10 +1473,12 @@ int bx_int_logp(const int64_t* logits, int64_t ld, const int64_t* tok, const int
   const int nch0 = sample_chunks(M, V);
   i64* pmax = (i64*)scratch;                       // chunk maxima, then (entry 0 of each row) the row maximum
   i64* psum = pmax + (size_t)M * nch0;
-  logp_max_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, pmax, V, ch, nch);
+  // below about eight table lengths of logits, checking the table costs what the gathers do
+  int* fits = (i64)M * V >= (i64)8 * LSE_LAST ? (int*)(psum + (size_t)M * nch0) : nullptr;
+  logp_max_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, pmax, V, ch, nch, (const longlong2*)tab2, fits);
   // the row maxima go to out[], which the last kernel overwrites after reading them
   logp_sum_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, nullptr, pmax, nch, (i64*)out,
-                                                        (const longlong2*)tab2, psum, V, ch, nch, fr);
+                                                        (const longlong2*)tab2, fits, psum, V, ch, nch, fr);
   logp_finish_kernel<<<(M + 127) / 128, 128, 0, st>>>(psum, nch, nullptr, (const i64*)logits, ld, (const i64*)tok,
                                                       (const i64*)out, (const i64*)lnt, (i64*)out, M, V, fr);
   return launched(3);

@@ -47,6 +47,30 @@ def test_seeded_rows_vs_oracle(M, V, fr):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("M,V,fr,table", [(6, 250001, 16, "exp"), (37, 36001, 24, "exp"), (1100, 1200, 13, "exp"),
+                                          (37, 36001, 16, "last"), (37, 36001, 16, "first")])
+def test_terms_as_products(M, V, fr, table):
+    """Rows long enough that the terms come from products of doubles: arguments next to the maximum and down to the clamp and past 32 bits,
+    every table entry met, remainders of the chunks; and tables with one entry off by one, whose terms are gathered. Integers: equal."""
+    from bitexact_llm_b200 import _native as nv
+    g = np.random.default_rng(M + V + fr)
+    lg = -(g.integers(0, 41 << fr, (M, V), dtype=np.int64) >> g.integers(0, 12, (M, V)))
+    lg[:, ::7] = lg[:, ::7] >> (fr - 12) << (fr - 12)                              # whole steps: no interpolation
+    lg[:, 1::11] -= 1 << 33
+    tab = ol.lse_table()
+    if table != "exp":
+        tab[-1 if table == "last" else 0] += 1 if table == "first" else -1
+    tok, lnt = g.integers(0, V, M, dtype=np.int64), ox.ln_table(40)
+    lib, d, w, t, l = nv.lib(), T(tab), T(lg), T(tok), T(lnt)
+    pair = torch.empty(tab.shape[0], 2, dtype=torch.long, device="cuda")
+    scratch = torch.empty(lib.bx_logp_scratch_bytes(M, V), dtype=torch.uint8, device="cuda")
+    out = torch.empty(M, dtype=torch.long, device="cuda")
+    nv.check(lib.bx_logp_pair_table(d.data_ptr(), tab.shape[0], pair.data_ptr(), nv.stream()), "pair_table")
+    nv.check(lib.bx_int_logp(w.data_ptr(), V, t.data_ptr(), l.data_ptr(), pair.data_ptr(), tab.shape[0], scratch.data_ptr(),
+                             out.data_ptr(), M, V, fr, nv.stream()), "int_logp")
+    assert np.array_equal(out.cpu().numpy(), ol.int_logp_q(lg, tok, lnt, tab, fr))
+
+
 def test_token_out_of_range_gives_nan():
     from bitexact_llm_b200.vllm_plugin import rl
     lg = torch.randint(-(1 << 20), 1 << 20, (3, 500), device="cuda")
