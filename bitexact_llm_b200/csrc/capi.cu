@@ -1363,7 +1363,7 @@ static int run_sample(const int64_t* logits, int64_t ld, const int64_t* rows, co
   const int rc = launch_chained(sample_part_kernel, dim3(nch, M), SAMPLE_THREADS, 0, st, 0, (const i64*)logits, ld, (const i64*)rows,
                                 (const i64*)lnt, pmax, pidx, V, ch, nch, bits, (i64)voff);
   if (rc != BX_OK) return rc;
-  return launch_chained(sample_combine_kernel, dim3((M + 127) / 128), 128, 0, st, 0, pmax, pidx, (i64*)tok, (i64*)omax, M, nch);
+  return launch_chained(sample_combine_kernel, dim3((M + 3) / 4), 128, 0, st, 0, pmax, pidx, (i64*)tok, (i64*)omax, M, nch);
 }
 
 int bx_sample(const int64_t* logits, int64_t ld, const int64_t* rows, const int64_t* lnt, void* scratch,

@@ -12,6 +12,7 @@
 
 #include "bx_rules.cuh"
 #include "elementwise.cuh"
+#include "stage_math.cuh"
 
 namespace bx {
 
@@ -100,20 +101,32 @@ __device__ inline u128 pcg_advance(u128 state, u128 inc, u64 delta) {
   return add128(mul128(acc_mult, state), acc_plus);
 }
 
-// (mult, plus) of `delta` LCG steps at once: state -> mult * state + plus.
-__device__ inline void pcg_jump(u128 inc, u64 delta, u128& mult, u128& plus) {
-  u128 cur_mult = {PCG_MULT_HI, PCG_MULT_LO}, cur_plus = inc;
-  mult = u128{0, 1};
-  plus = u128{0, 0};
-  while (delta) {
-    if (delta & 1) {
-      mult = mul128(mult, cur_mult);
-      plus = add128(mul128(plus, cur_mult), cur_plus);
-    }
-    cur_plus = mul128(add128(cur_mult, u128{0, 1}), cur_plus);
-    cur_mult = mul128(cur_mult, cur_mult);
-    delta >>= 1;
+// n LCG steps at once: state -> mult state + sum inc with mult = M^n and sum = 1 + M + .. + M^(n-1), which depend on n alone:
+// n = 0 .. N - 1 (each thread of a CTA takes its own), or n = 2^0 .. 2^(N-1).
+struct alignas(16) PcgSteps {
+  u64 mult_lo, mult_hi, sum_lo, sum_hi;
+};
+template <int N>
+struct PcgTable {
+  PcgSteps e[N];
+};
+template <int N>
+constexpr PcgTable<N> pcg_table(bool powers) {
+  using W = unsigned __int128;
+  const W one = ((W)PCG_MULT_HI << 64) | PCG_MULT_LO;
+  PcgTable<N> t{};
+  W mult = powers ? one : 1, sum = powers ? 1 : 0;
+  for (int i = 0; i < N; ++i) {
+    t.e[i] = PcgSteps{(u64)mult, (u64)(mult >> 64), (u64)sum, (u64)(sum >> 64)};
+    sum = powers ? (mult + 1) * sum : sum * one + 1;
+    mult *= powers ? mult : one;
   }
+  return t;
+}
+__device__ const PcgTable<SAMPLE_THREADS + 1> PCG_STEPS = pcg_table<SAMPLE_THREADS + 1>(false);
+__constant__ PcgTable<64> PCG_POWERS = pcg_table<64>(true);
+__device__ __forceinline__ u128 pcg_steps(const PcgSteps& n, u128 state, u128 inc) {
+  return add128(mul128(u128{n.mult_hi, n.mult_lo}, state), mul128(u128{n.sum_hi, n.sum_lo}, inc));
 }
 
 // XSL-RR output of a state.
@@ -208,9 +221,12 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
                    const i64* __restrict__ lnt, i64* __restrict__ pmax, i64* __restrict__ pidx, int V, int ch,
                    int nch, int bits, i64 voff) {
   __shared__ i64 smax[SAMPLE_THREADS / 32], sidx[SAMPLE_THREADS / 32];
-  __shared__ i64 gtab[41];
+  __shared__ double gtab[41];
+  __shared__ u128 seeded[3];
+  __shared__ int reached;                  // the CTA's best value: a float rounded down, as a whole number of its order
   const int64_t row = blockIdx.y;
   const int chunk = blockIdx.x;
+  const PcgSteps own = PCG_STEPS.e[threadIdx.x];
   wait_previous();
   launch_next();
   const i64 tn = rows[4 * row + 2], td = rows[4 * row + 3];
@@ -229,24 +245,51 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
     // for 1 - u in (2^-j, 2^-(j-1)] it is at most gtab[j] = g at 1 - u = 2^-j (taken with the same function). An
     // entry whose scaled logit plus that bound stays below a value some entry of the row already reached cannot be
     // the first maximum; only the others (a few per cent) pay for the two table logarithms and the division.
-    // The bound every lane prunes with is the warp's best value, refreshed every fourth entry; the comparison is
-    // strict, so equal values (which the first-index rule must see) are always evaluated.
-    if (threadIdx.x >= 1 && threadIdx.x <= 40) {
-      const u64 t = (1ull << 53) - (1ull << (53 - threadIdx.x));
-      gtab[threadIdx.x] = gumbel_q((i64)(t << 11), lnt, bits);
+    // The comparison is made in doubles on the safe side (2 and 2^-50 of the scaled logit above it, more than the
+    // roundings and the 1/2 of rdiv): a double operation takes a quarter of a 64-bit integer comparison.
+    // The bound every lane prunes with is the best value so far of its warp, and every fourth entry of the CTA, as a float
+    // rounded down (some value of the row that was reached, whatever the order of the warps); the comparison is strict,
+    // so equal values (which the first-index rule must see) are always evaluated.
+    // The first warp seeds and advances to the chunk once, the threads step on from there. Rows of 128256, with the combine kernel:
+    // 68 us for 19 and 92 for 64 with every thread doing both, 38 and 68 so; pruned in doubles 38 and 64 (1000 rows 641 -> 518);
+    // with the bound shared in the CTA and refreshed at once 29 and 48 (1000 rows 445, 256 rows 214 -> 136).
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+      u128 st, inc;
+      pcg_seed((u64)rows[4 * row], (u64)rows[4 * row + 1], st, inc);
+      const u64 n = (u64)(voff + c0) + 1;                      // the state whose output is the word of entry c0
+      for (u64 left = n, k = 0; left; left >>= 1, ++k)
+        if (left & 1) st = pcg_steps(PCG_POWERS.e[k], st, inc);
+      if (lane == 0) {
+        reached = (int)0x80000000;
+        seeded[0] = st;
+        seeded[1] = inc;
+        seeded[2] = mul128(u128{PCG_STEPS.e[SAMPLE_THREADS].sum_hi, PCG_STEPS.e[SAMPLE_THREADS].sum_lo}, inc);
+      }
+    } else if (threadIdx.x > 64 && threadIdx.x <= 64 + 40) {
+      const int j = threadIdx.x - 64;
+      const u64 t = (1ull << 53) - (1ull << (53 - j));
+      gtab[j] = 2.0 + (double)gumbel_q((i64)(t << 11), lnt, bits);
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    u128 st, inc, jm, jp;
-    pcg_seed((u64)rows[4 * row], (u64)rows[4 * row + 1], st, inc);
-    st = pcg_advance(st, inc, (u64)(voff + e0) + 1);           // the state whose output is the word of entry e0
-    pcg_jump(inc, SAMPLE_THREADS, jm, jp);
+    u128 st = pcg_steps(own, seeded[0], seeded[1]);
+    const u128 jm = {PCG_STEPS.e[SAMPLE_THREADS].mult_hi, PCG_STEPS.e[SAMPLE_THREADS].mult_lo}, jp = seeded[2];
     const u64 dv = (u64)(2 * tn);
     const u64 inv = ~0ull / dv;
-    const bool prunable = dv < (1ull << 31);
-    i64 wb = (i64)0x8000000000000000ull;
+    // logits below 2^51 (a whole double) and 2^60 / td in size: |2 l td + tn| does not wrap
+    const bool prunable = tn > 0 && tn < (1ll << 30) && td >= 0 && td < (1ll << 27);
+    const int bound = prunable ? min(51, 60 - bitlen(td)) - 32 : 0;
+    const double ratio = (double)td / (double)tn;
+    int mine = (int)0x80000000;
+    const auto order = [](int b) { return b ^ (b >> 31 & 0x7fffffff); };      // a float's bits <-> a whole number of its order
+    double floor_ = -__longlong_as_double(0x7ff0000000000000ll);
     // Four entries per round: their logits are loaded first (independent loads in flight), then each is processed.
     for (int64_t eb = c0 + (threadIdx.x & ~31); eb < c1; eb += 4 * SAMPLE_THREADS) {
+      const int other = *(volatile int*)&reached;
+      if (other > mine) {
+        mine = other;
+        floor_ = __int_as_float(order(mine));
+      }
       i64 lg[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -260,18 +303,17 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
         const bool act = e < c1;
         const u64 w = pcg_output(st);
         st = add128(mul128(jm, st), jp);
-        const i64 U = iclamp((i64)((w >> 11) & ((1ull << 53) - 1)), UMIN, (1ll << 53) - UMIN);
-        const int j = __clzll((1ll << 53) - U) - 10;           // 1 - u in (2^-j, 2^-(j-1)], 1 <= j <= 40
-        // rdiv(l * td, tn) = floor((2 l td + tn) / (2 tn))
-        const i64 a = 2 * lg[k] * td + tn;
+        const uint32_t ones = ~(uint32_t)(w >> 32);
+        const int j = ones ? __clz(ones) + 1 : 40;             // 1 - u in [2^-j, 2^-(j-1)), or below 2^-32
         bool pass = act;
-        const i64 lb = imax(best, wb);
-        if (act && prunable && lb > -(1ll << 61)) {
-          const i64 m = lb - gtab[j];                          // floor(a / dv) + gtab[j] < lb  <=>  a < m dv
-          if (m > -(1ll << 31) && m < (1ll << 31)) pass = !(a < m * (i64)dv);
+        if (prunable && (uint32_t)(lg[k] >> 32) + (1u << bound) < 2u << bound) {
+          const double t = to_f64(lg[k]) * ratio;
+          pass &= !(fma(fabs(t), 8.881784197001252e-16, t) + gtab[j] < floor_);
         }
         if (__any_sync(0xffffffffu, pass)) {
           if (pass) {
+            // rdiv(l * td, tn) = floor((2 l td + tn) / (2 tn))
+            const i64 a = 2 * lg[k] * td + tn;
             const i64 g = gumbel_q((i64)w, lnt, bits);
             u64 rem;
             const u64 qd = uqr_recip((u64)iabs(a), dv, inv, rem);
@@ -279,9 +321,14 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
             const i64 v = fq + g;
             if (v > best) { best = v; bidx = voff + e; }
           }
+          const int top = __reduce_max_sync(0xffffffffu, order(__float_as_int(__ll2float_rd(best))));
+          if (top > mine) {
+            mine = top;
+            floor_ = __int_as_float(order(mine));
+            if (lane == 0) atomicMax(&reached, mine);
+          }
         }
       }
-      wb = warp_max(best);
     }
   }
   // first index of the maximum: larger value wins, then the smaller index
@@ -302,20 +349,28 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
   }
 }
 
-// tok[row] = first index of the maximum over the chunks; omax (may be null) receives the maximum itself.
+// tok[row] = first index of the maximum over the chunks; omax (may be null) receives the maximum itself. A warp per row: one thread
+// walking a row's chunks took 7 us more for one row.
 __global__ void sample_combine_kernel(const i64* __restrict__ pmax, const i64* __restrict__ pidx,
                                       i64* __restrict__ tok, i64* __restrict__ omax, int M, int nch) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   wait_previous();
   launch_next();
   if (row >= M) return;
-  i64 best = pmax[(int64_t)row * nch], bidx = pidx[(int64_t)row * nch];
-  for (int c = 1; c < nch; ++c) {
+  i64 best = (i64)0x8000000000000000ull, bidx = 0x7fffffffffffffffll;
+  for (int c = lane; c < nch; c += 32) {
     const i64 v = pmax[(int64_t)row * nch + c], i = pidx[(int64_t)row * nch + c];
     if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
   }
-  tok[row] = bidx;
-  if (omax) omax[row] = best;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const i64 v = __shfl_xor_sync(0xffffffffu, best, o), i = __shfl_xor_sync(0xffffffffu, bidx, o);
+    if (v > best || (v == best && i < bidx)) { best = v; bidx = i; }
+  }
+  if (lane == 0) {
+    tok[row] = bidx;
+    if (omax) omax[row] = best;
+  }
 }
 
 }  // namespace bx

@@ -368,6 +368,42 @@ def test_sharded_sampler_pairs_combine_to_the_full_row_token():
     assert torch.equal(tok, want) and int(tok[2]) in (100, int(want[2]))
 
 
+@pytest.mark.parametrize("V,tn,td,shift,voff", [(1, 7, 10, 0, 0), (255, 1, 100, 0, 3), (257, 7, 10, 26, 0), (2049, 3, 1, 20, (1 << 33) + 5),
+                                                (5003, (1 << 30) - 1, 1 << 26, 0, 1 << 40), (5003, 7, 1 << 27, 0, 0)])
+def test_sampler_steps_to_its_words(V, tn, td, shift, voff):
+    """Chunk and thread starts at odd sizes and far offsets, keys of one and two words, logits on both sides of the limit of the
+    comparison in doubles (shift), ratios on both sides of its rule: against the generator in whole numbers. Equal."""
+    import oracle.sampler as osm
+    from bitexact_llm_b200 import _native as nv
+    from bitexact_llm_b200.exact.consts import ln_table
+    lib, lnt = nv.lib(), ln_table(device="cuda")
+    rng = np.random.RandomState(V)
+    keys = [(5, 9), ((1 << 40) + 3, 1), (2, (1 << 35) + 7)]
+    li = rng.randint(-(25 << 24), 25 << 24, (len(keys), V)).astype(np.int64) << shift
+    want = []
+    for (s, t), row in zip(keys, li):
+        state, inc = osm.pcg_state(s, t)
+        m, p, n, am, ap = osm.PCG_MULT, inc, voff, 1, 0
+        while n:                                                    # n steps as one: doubling
+            if n & 1:
+                am, ap = am * m & osm.M128, (ap * m + p) & osm.M128
+            m, p, n = m * m & osm.M128, (m + 1) * p & osm.M128, n >> 1
+        state, words = (am * state + ap) & osm.M128, []
+        for _ in range(V):
+            state = (state * osm.PCG_MULT + inc) & osm.M128
+            x, rot = (state >> 64 ^ state) & ((1 << 64) - 1), state >> 122
+            words.append((x >> rot | x << (64 - rot & 63)) & ((1 << 64) - 1))
+        g = osm.gumbel(np.array(words, dtype=np.uint64).view(np.int64), ox.ln_table(), 24)
+        want.append(voff + int(osm.sample(row, tn, td, g)))
+    rows = torch.tensor([[s, t, tn, td] for s, t in keys], device="cuda")
+    d = torch.from_numpy(li).cuda()
+    best, idx = torch.empty(3, dtype=torch.long, device="cuda"), torch.empty(3, dtype=torch.long, device="cuda")
+    scratch = torch.empty(lib.bx_sample_scratch_bytes(3, V), dtype=torch.uint8, device="cuda")
+    assert lib.bx_sample_shard(d.data_ptr(), V, rows.data_ptr(), lnt.data_ptr(), scratch.data_ptr(), best.data_ptr(), idx.data_ptr(),
+                               3, V, voff, 24, nv.stream()) == 0
+    assert idx.tolist() == want
+
+
 def test_sampler_pruning_keeps_the_first_maximum():
     """Rows built to stress the exact pruning of the sampler: flat logits (the noise alone decides), a narrow band,
     a dominant logit, huge spread, duplicated maxima of logit + noise, 16 and 24 fractional bits, many temperatures,
