@@ -1473,7 +1473,8 @@ int bx_int_logp(const int64_t* logits, int64_t ld, const int64_t* tok, const int
   const int nch0 = sample_chunks(M, V);
   i64* pmax = (i64*)scratch;                       // chunk maxima, then (entry 0 of each row) the row maximum
   i64* psum = pmax + (size_t)M * nch0;
-  // below about eight table lengths of logits, checking the table costs what the gathers do
+  // below about eight table lengths of logits, checking the table costs what the gathers do (both 34 .. 39 us at 16 rows of 128256;
+  // 64 rows 80 -> 66 us)
   int* fits = (i64)M * V >= (i64)8 * LSE_LAST ? (int*)(psum + (size_t)M * nch0) : nullptr;
   logp_max_kernel<<<dim3(nch, M), LOGP_THREADS, 0, st>>>((const i64*)logits, ld, pmax, V, ch, nch, (const longlong2*)tab2, fits);
   // the row maxima go to out[], which the last kernel overwrites after reading them
