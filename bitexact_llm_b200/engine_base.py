@@ -28,15 +28,19 @@ class TokenRowEngine:
             return None
         return tri_prefill.tile_table(runs, G, tri_prefill.ROWS)
 
-    def forward_native(self, call, exact, fields, layers, kvs, ids, pos, slot, bt, rmap, tiles):
+    def forward_native(self, call, exact, fields, layers, shapes, kvs, ids, pos, slot, bt, rmap, tiles):
         """All layers' kernels from one call of the library (`bx_exact_forward`, `bx_int8_forward`): fields of bx_step beside the common
-        ones, layers a flat list of what a bx_*_layer holds in front of its cache, one list per layer. Returns the residual rows, or
-        None where the call's geometry is not what that entry takes (the engines then run their own loop)."""
+        ones, layers a flat list of what a bx_*_layer holds in front of its cache, one list per layer, shapes the (rows, columns) of its
+        four matrices. Returns the residual rows, or None where the call's geometry is not what that entry takes (the engines then run
+        their own loop)."""
         import ctypes
 
         from . import _native as nv
         N, G, dev = ids.shape[0], self.H // self.HKV, ids.device
         if N == 0 or self.HD != 64 or G > 4 and tiles is None or len(kvs) < self.L or tiles is not None and tiles.shape[0] == 0:
+            return None
+        FF = shapes[0][2][0] // 2                                # of the weights: a config need not name it
+        if any(sh != [((self.H + 2 * self.HKV) * self.HD, self.D), (self.D, self.H * self.HD), (2 * FF, self.D), (self.D, FF)] for sh in shapes):
             return None
         bs, flat = kvs[0].shape[2], []
         for c, layer in zip(kvs, layers):
@@ -47,12 +51,12 @@ class TokenRowEngine:
             flat += (c.data_ptr(), c.shape[0], c.stride(0), c.stride(1), c.stride(2))
         assert bt.shape[1] * bs < 43690 and bt.dtype in (torch.int32, torch.int64) and bt.stride(1) == 1
         x = torch.empty(N, self.D, dtype=torch.long, device=dev)
-        n = nv.lib().bx_forward_bytes(int(exact), N, self.D, self.H, self.HKV, self.HD, self.FF, bt.shape[1], bs, int(tiles is not None))
+        n = nv.lib().bx_forward_bytes(int(exact), N, self.D, self.H, self.HKV, self.HD, FF, bt.shape[1], bs, int(tiles is not None))
         work = torch.empty(n, dtype=torch.uint8, device=dev)
         keep = [ids.contiguous(), rmap.long().contiguous()]
         s = nv.Step(ids=keep[0].data_ptr(), pos=pos.data_ptr(), slot=slot.data_ptr(), bt=bt.data_ptr(), rmap=keep[1].data_ptr(), cos=self.cos.data_ptr(),
                     sin=self.sin.data_ptr(), emb=self.emb.data_ptr(), x=x.data_ptr(), flag=self.fl.data_ptr(), work=work.data_ptr(), layers=self.L, N=N,
-                    D=self.D, H=self.H, HKV=self.HKV, HD=self.HD, FF=self.FF, bs=bs, bt64=int(bt.dtype == torch.int64), sbt=bt.stride(0),
+                    D=self.D, H=self.H, HKV=self.HKV, HD=self.HD, FF=FF, bs=bs, bt64=int(bt.dtype == torch.int64), sbt=bt.stride(0),
                     nblk=bt.shape[1], work_bytes=n, **fields)
         if tiles is None:
             keep.append(pos.view(-1, 1).expand(-1, G).contiguous())

@@ -26,7 +26,6 @@ class IntEngine(TokenRowEngine):
         self.H = cfg.get("num_attention_heads", 32)
         self.HKV = cfg.get("num_key_value_heads", 8)
         self.HD = cfg.get("head_dim") or self.D // self.H
-        self.FF = cfg.get("intermediate_size", 8192)
         self.L = c["n_layers"] if n_layers is None else n_layers
         t = lambda k: c[k].to(self.dev).contiguous()
         self.emb = t("emb")
@@ -87,17 +86,19 @@ class IntEngine(TokenRowEngine):
     def _forward_native(self, kvs, ids, pos, slot, bt, rmap, tiles):
         if self.timer is not None or rmap is None:               # a timer brackets every linear by itself
             return None
-        rows = []
+        rows, shapes = [], []
         for ly in self.layers[:self.L]:
-            row = []
+            row, sh = [], []
             for n in ("wqkv", "wo", "wgu", "wd"):
                 w, mul, fmsh = ly[n]
                 row += (w.data_ptr(), mul.data_ptr(), int(fmsh), w.shape[0], w.shape[1])
+                sh.append((w.shape[0], w.shape[1]))
+            shapes.append(sh)
             rows.append(row + [ly["ga"].data_ptr(), ly["gm"].data_ptr()])
         form = None if self.compact is None else attn_table.native(self.compact)       # lives until the call has read it
         fields = dict(ptab=self.ptab.data_ptr(), silu=self.silu_t.data_ptr(), silu_compact=nv.ptr(self.silu_c), scr=self.scr.data_ptr(),
                       compact=None if form is None else ctypes.addressof(form))
-        return self.forward_native("bx_int8_forward", False, fields, rows, kvs, ids, pos, slot, bt, rmap, tiles)
+        return self.forward_native("bx_int8_forward", False, fields, rows, shapes, kvs, ids, pos, slot, bt, rmap, tiles)
 
     def logits(self, h):
         """Final residual rows [M, D] -> int64 logits [M, V] at 16 bits."""

@@ -95,7 +95,7 @@ class ExactEngine(TokenRowEngine):
         layers = self.layers[:self.L]
         if self.D & (self.D - 1) or not 32 <= self.D <= 4096 or rmap is None or any(ly[n].timer is not None for ly in layers for n in ("wqkv", "wo", "wgu", "wd")):
             return None                                          # a timer brackets every linear by itself
-        ptr, rows = nv.ptr, []
+        ptr, rows, shapes = nv.ptr, [], []
         for ly in layers:
             row = []
             for n in ("wqkv", "wo", "wgu", "wd"):
@@ -103,9 +103,10 @@ class ExactEngine(TokenRowEngine):
                 row += (w.limbs.data_ptr(), w.d.data_ptr(), w.g.data_ptr(), ptr(w.cnt) or 0, ptr(w.ec) or 0, ptr(w.ev) or 0, w.R, w.N, w.K, w.cfg or 0)
             row += (ly["ga"][0].data_ptr(), ly["ga"][1].data_ptr(), ly["gm"][0].data_ptr(), ly["gm"][1].data_ptr())
             rows.append(row)
+            shapes.append([(ly[n].N, ly[n].K) for n in ("wqkv", "wo", "wgu", "wd")])
         form = None if self.compact is None else attn_table.native(self.compact)       # lives until the call has read it
         fields = dict(lut=self.exp2.data_ptr(), l2e=int(self.l2e), compact=None if form is None else ctypes.addressof(form))
-        return self.forward_native("bx_exact_forward", True, fields, rows, kvs, ids, pos, slot, bt, rmap, tiles)
+        return self.forward_native("bx_exact_forward", True, fields, rows, shapes, kvs, ids, pos, slot, bt, rmap, tiles)
 
     def logits(self, h):
         """Final residual rows [M, D] -> int64 logits [M, V] at 24 bits."""

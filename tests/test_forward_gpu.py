@@ -11,17 +11,17 @@ from bitexact_llm_b200 import _native as nv
 pytestmark = pytest.mark.gpu
 
 
-def engine(mode, width, layers):
+def engine(mode, width, layers, edit=lambda c: c):
     from bitexact_llm_b200.exact import consts
     cfg = dict(consts.LLAMA_1B, hidden_size=width, intermediate_size=4 * width, num_hidden_layers=layers, num_attention_heads=width // 64,
                num_key_value_heads=width // 256, head_dim=64, vocab_size=512)
     sd = consts.random_state_dict(cfg, seed=width, device="cuda", gamma_jitter=0.1)
     if mode == "exact":
         from bitexact_llm_b200.vllm_plugin.exact_run import ExactEngine
-        return ExactEngine(consts.build(cfg, sd, n_pos=700), "cuda")
+        return ExactEngine(edit(consts.build(cfg, sd, n_pos=700)), "cuda")
     from bitexact_llm_b200.int8 import consts as consts8
     from bitexact_llm_b200.int8.engine import IntEngine
-    return IntEngine(consts8.build(cfg, sd, n_pos=700), "cuda")
+    return IntEngine(edit(consts8.build(cfg, sd, n_pos=700)), "cuda")
 
 
 def step(eng, ses, seqs, lens, tiles, native, form=True):
@@ -86,3 +86,19 @@ def test_what_the_loop_alone_serves():
     work = nv.lib().bx_forward_bytes(1, 2, 256, 4, 1, 64, 1024, 4, 16, 0)
     assert work > 0 and nv.lib().bx_forward_bytes(1, 0, 256, 4, 1, 64, 1024, 4, 16, 0) == 0
     assert nv.lib().bx_exact_forward(None, None, None) == nv.BX_EARG and nv.lib().bx_int8_forward(None, None, None) == nv.BX_EARG
+
+
+@pytest.mark.parametrize("mode", ["exact", "int8"])
+def test_the_feed_forward_width_is_that_of_the_weights(mode):
+    """Constants whose config does not name it."""
+    from bitexact_llm_b200.decode import Session
+
+    def unnamed(c):
+        del c["cfg"]["intermediate_size"]
+        return c
+    for n in (1, 600):
+        got = []
+        for edit in (unnamed, lambda c: c):
+            eng = engine(mode, 256, 2, edit)
+            got.append(step(eng, Session(eng, 2, 640, perm_seed=1), [1], [n], n > 500, True))
+        assert torch.equal(got[0][0], got[1][0]) and got[0][3] == got[1][3]
