@@ -84,8 +84,8 @@ class IntEngine(TokenRowEngine):
         return x
 
     def _forward_native(self, kvs, ids, pos, slot, bt, rmap, tiles):
-        if self.timer is not None or rmap is None:               # a timer brackets every linear by itself
-            return None
+        if self.timer is not None or rmap is None or getattr(self._lin, "__func__", None) is not IntEngine._lin:
+            return None                                          # a timer brackets every linear, another _lin is to be called for each
         rows, shapes = [], []
         for ly in self.layers[:self.L]:
             row, sh = [], []

@@ -93,8 +93,10 @@ class ExactEngine(TokenRowEngine):
 
     def _forward_native(self, kvs, ids, pos, slot, bt, rmap, tiles):
         layers = self.layers[:self.L]
-        if self.D & (self.D - 1) or not 32 <= self.D <= 4096 or rmap is None or any(ly[n].timer is not None for ly in layers for n in ("wqkv", "wo", "wgu", "wd")):
-            return None                                          # a timer brackets every linear by itself
+        if self.D & (self.D - 1) or not 32 <= self.D <= 4096 or rmap is None:
+            return None
+        if any(type(ly[n]) is not FusedLin or ly[n].timer is not None for ly in layers for n in ("wqkv", "wo", "wgu", "wd")):
+            return None                                          # another callable, or a timer that brackets every linear by itself
         ptr, rows, shapes = nv.ptr, [], []
         for ly in layers:
             row = []

@@ -102,3 +102,45 @@ def test_the_feed_forward_width_is_that_of_the_weights(mode):
             eng = engine(mode, 256, 2, edit)
             got.append(step(eng, Session(eng, 2, 640, perm_seed=1), [1], [n], n > 500, True))
         assert torch.equal(got[0][0], got[1][0]) and got[0][3] == got[1][3]
+
+
+@pytest.mark.parametrize("layer", ["wqkv", "wo", "wgu", "wd"])
+def test_linears_of_another_kind_are_called(layer):
+    """A layer that is wrapped, or of a class of its own (exact mode); an engine's own _lin, of its class or its instance (int8 mode)."""
+    from bitexact_llm_b200.decode import Session
+    from bitexact_llm_b200.int8.engine import IntEngine
+    from bitexact_llm_b200.vllm_plugin.exact_gemm import FusedLin
+    seen = []
+
+    class Counted(FusedLin):
+        def __call__(self, *a, **k):
+            seen.append(self)
+            return super().__call__(*a, **k)
+
+    class Own(IntEngine):
+        def _lin(self, pre, lin):
+            seen.append(lin)
+            return super()._lin(pre, lin)
+
+    def run(eng):
+        return step(eng, Session(eng, 2, 64, perm_seed=1), [1], [3], False, True)
+    eng = engine("exact", 256, 2)
+    want, plain = run(eng), eng.layers[1][layer]
+    eng.layers[1][layer] = lambda *a, **k: (seen.append(a), plain(*a, **k))[1]
+    got = run(eng)
+    assert len(seen) == 1 and torch.equal(got[0], want[0])
+    eng.layers[1][layer] = plain
+    plain.__class__ = Counted
+    got = run(eng)
+    assert len(seen) == 2 and torch.equal(got[0], want[0])
+    plain.__class__ = FusedLin
+    eng = engine("int8", 256, 2)
+    want = run(eng)
+    assert len(seen) == 2
+    eng.__class__ = Own
+    got = run(eng)
+    assert len(seen) == 2 + 4 * eng.L and torch.equal(got[0], want[0])
+    eng.__class__ = IntEngine
+    eng._lin = lambda pre, lin: (seen.append(lin), IntEngine._lin(eng, pre, lin))[1]
+    got = run(eng)
+    assert len(seen) == 2 + 8 * eng.L and torch.equal(got[0], want[0])
