@@ -87,14 +87,15 @@ class Session:
                     i += 1
             if not runs:
                 continue
-            # everything that the step has to know of its rows goes over in one copy
+            # everything that the step has to know of its rows goes over in one copy, but tokens that are on a device already
+            host = [t.device.type == "cpu" for _, _, _, t in runs]
             many = torch.tensor([[s, n, len(t)] for _, s, n, t in runs])
             counts = many[:, 2]
             first = torch.cumsum(counts, 0) - counts
             table = torch.empty(3, at, dtype=torch.long)
             table[0] = torch.repeat_interleave(many[:, 0], counts)
             table[1] = torch.arange(at) + torch.repeat_interleave(many[:, 1] - first, counts)
-            torch.cat([t.cpu() for _, _, _, t in runs], out=table[2])
+            torch.cat([t if h else torch.zeros(len(t), dtype=torch.long) for h, (_, _, _, t) in zip(host, runs)], out=table[2])
             ends = torch.cat([many[:, 0], many[:, 1] + counts])
             both = torch.cat([table.reshape(-1), ends]).to(dev)
             seq, pos, ids = both[:3 * at].view(3, at)
@@ -102,6 +103,8 @@ class Session:
             for _, s, n, t in runs:
                 tt.append((s, row, len(t), n + len(t)))
                 row += len(t)
+            if not all(host):
+                ids = torch.cat([ids[r:r + n] if h else t.to(dev) for h, (_, r, n, _), (_, _, _, t) in zip(host, tt, runs)])
             longest = max(c for _, _, q, c in tt if q > 1) if any(q > 1 for _, _, q, _ in tt) else 0
             tt = self.eng.tile_table(tt, self.bs) if longest > self.eng.tiles_from else None
             x = self.eng.forward(self.kvs, ids, pos, self._slots(seq, pos), self.bt, seq,

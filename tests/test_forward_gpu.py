@@ -144,3 +144,33 @@ def test_linears_of_another_kind_are_called(layer):
     eng._lin = lambda pre, lin: (seen.append(lin), IntEngine._lin(eng, pre, lin))[1]
     got = run(eng)
     assert len(seen) == 2 + 8 * eng.L and torch.equal(got[0], want[0])
+
+
+def test_feed_of_device_tokens():
+    """A server's sampled tokens stay on the device: no more waits than for tokens on the host, the same rows, lengths and caches,
+    also beside entries on the host and portions cut by chunk_rows."""
+    import warnings
+
+    from bitexact_llm_b200.decode import Session
+    eng, rng = engine("exact", 256, 2), torch.Generator().manual_seed(3)
+    portions = [torch.randint(0, 512, (n,), generator=rng) for n in (1, 7, 1, 450, 1, 3)]
+
+    def run(place, chunk_rows):
+        ses = Session(eng, 6, 640, perm_seed=1)
+        entries = [(s, t.cuda() if place == "device" or place == "mixed" and s % 2 else t) for s, t in enumerate(portions)]
+        with warnings.catch_warnings(record=True) as waits:
+            warnings.simplefilter("always")
+            torch.cuda.set_sync_debug_mode("warn")
+            try:
+                rows = ses.feed(entries, chunk_rows)
+            finally:
+                torch.cuda.set_sync_debug_mode("default")
+        return torch.cat(rows), ses.lens.clone(), torch.stack(ses.kvs), sum("synchroniz" in str(w.message) for w in waits)
+    run("host", 4096)
+    for chunk_rows in (4096, 100):
+        want = run("host", chunk_rows)
+        assert want[3] > 0
+        for place in ("device", "mixed"):
+            got = run(place, chunk_rows)
+            assert all(torch.equal(a, b) for a, b in zip(want[:3], got[:3]))
+            assert got[3] <= want[3]
