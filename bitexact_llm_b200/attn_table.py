@@ -6,9 +6,12 @@ memory, from which a weight is known to within a small window, and goes to the f
 lies in the window. The window is a property of the full table, worked out here over all of its entries; a table that
 such a form cannot stand for gets none (None), and the kernels then read the full table for every weight.
 
-compact = (int32 tensor of the entries, in exact mode with the products of doubles behind them, window, slack, factor from a row distance to t, its left shift, 2^(top + 1)):
-window in units
-of the interpolated entry, slack (for a table that was itself rounded) in units of 2^-32 of a weight."""
+In exact mode the doubles of which the entries of a 2^-f table are products (2 KB, `products`) serve better and take the place of the
+entries where the table is one of products; any other table keeps the entries.
+
+compact = (int32 tensor of the entries, in exact mode with room for the products behind them, window, slack, factor from a row
+distance to t, its left shift (and ENTRIES_ONLY where there are no products behind the entries of exact mode), 2^(top + 1)): window in
+units of the interpolated entry, slack (for a table that was itself rounded) in units of 2^-32 of a weight."""
 
 import ctypes
 
@@ -17,6 +20,7 @@ import torch
 T_BITS, W_BITS = 26, 31                # fractional bits of t, bits of an entry
 STEP = 1 << 14                         # t steps per segment: 4096 segments
 ENTRIES = 4097
+ENTRIES_ONLY = 1 << 9                  # in `shift`: the room behind the entries is empty
 
 
 class Native(ctypes.Structure):
@@ -26,7 +30,8 @@ class Native(ctypes.Structure):
 
 def native(compact):
     tab, window, slack, factor, shift, mtop = compact
-    return Native(tab.data_ptr(), window, slack, factor, mtop, shift | (256 if tab.shape[0] > ENTRIES else 0))
+    products = tab.shape[0] > ENTRIES and not shift & ENTRIES_ONLY
+    return Native(tab.data_ptr(), window, slack, factor, mtop, (shift & 255) | (256 if products else 0))
 
 
 def products(lut):
@@ -39,9 +44,8 @@ def products(lut):
     return t if ok else None
 
 
-def _with_products(tab, lut):
-    """The entries, and behind them (from byte 16400 on) the products, with a 1 in front of them where the table has such."""
-    t = products(lut)
+def _with_products(tab, t):
+    """The entries, and behind them (from byte 16400 on) the products t, with a 1 in front of them; zeros for None."""
     word = torch.tensor([0, 0, 0 if t is None else 1], dtype=torch.int32)
     return torch.cat([tab, word, (torch.zeros(257, dtype=torch.float64) if t is None else t).view(torch.int32)])
 
@@ -74,7 +78,8 @@ def exact(lut, l2e):
     tab = a + (lo - 2)                 # one for the floor of the kernel's product, one for the rounding of the table's rule
     if not _fits(tab) or hi - lo > 60:
         return None
-    return _with_products(tab.to(torch.int32), v), hi - lo + 3, 0, int(l2e) * 8, 1, 1 << 23
+    t = products(v)
+    return _with_products(tab.to(torch.int32), t), hi - lo + 3, 0, int(l2e) * 8, 1 if t is not None else 1 | ENTRIES_ONLY, 1 << 23
 
 
 def int8(ptab):

@@ -808,7 +808,7 @@ static StreamPlan stream_auto(int64_t pairs, int64_t max_keys, int bs, bool scra
   return stream_page_ok(NW, bs) && p.per_sm >= 2 ? p : none;
 }
 
-// shift: bit 8 says that the products lie behind the entries.
+// shift: bit 8 says that the products lie behind the entries; without it those serve an exact table too.
 static CompactTable compact_table(const bx_compact_table* c) {
   const double* products = c->shift & 256 ? reinterpret_cast<const double*>(c->tab + CT_BYTES / 4) : nullptr;
   return CompactTable{c->tab, products, c->window, c->slack, c->factor, c->mtop, c->shift & 255};
@@ -875,7 +875,11 @@ static bool split_can(int64_t R, int64_t HKV, int64_t max_keys, int bs, int sms)
 // 512 .. 768 145 : 138, of 500 .. 620 129 : 119; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27). Narrower tables stay with the kernels that give
 // a pair to a CTA or a cluster (64 of 16 .. 600 37 : 45, 256 of 16 .. 200 59 : 70), and so do few pairs of up to 3072 keys (4 of 2000 25 : 27).
 // Contexts much shorter than wide tables pay for it (64 of 16 .. 100 keys in 4096 25 : 30, 32 of the same 47 : 25).
-static bool split_auto(int64_t pairs, int64_t max_keys) {
+// entries: the caller's exact table has a compact form but no products, which leaves every weight of the split to the full table; the
+// streaming kernel has the entries (us, stream : split: 64 sequences of 16 .. 4096 keys 137 : 167, 100 of 100 .. 1500 109 : 122, 256 of
+// 512 .. 768 138 : 175, of 500 .. 1400 254 : 247; 48 of 64 .. 8192 221 : 208).
+static bool split_auto(int64_t pairs, int64_t max_keys, bool entries) {
+  if (entries && pairs >= STREAM_PAIRS && max_keys <= 4096 + 64) return false;
   return max_keys > (pairs >= 1024 ? 512 : pairs >= 192 ? 896 : pairs >= 128 ? 1280 : pairs >= 64 ? 2048 : 3072);
 }
 
@@ -934,7 +938,7 @@ static int run_attention(const int32_t* q, const int64_t* sh, const int64_t* qpo
                       sc_nb % 16 == 0 && sc_bs >= 384 && aligned16(cache);
   if (variant >= 2 && !tma_ok) return BX_EARG;
   if (variant < 0 || variant > 7 || (variant == 4 && bs > 32)) return BX_EARG;
-  if (variant == 7 || (variant == 0 && cluster_size == 0 && tma_ok && split_auto((int64_t)R * HKV, max_keys))) {
+  if (variant == 7 || (variant == 0 && cluster_size == 0 && tma_ok && split_auto((int64_t)R * HKV, max_keys, !ptab && ct.tab))) {
     const int sms = device_sms();
     if (sms <= 0) return BX_ELAUNCH;
     if (split_can(R, HKV, max_keys, bs, sms) && spill && aligned16(spill) && aligned16(num) && spill_bytes >= split_bytes((int64_t)R * HKV, max_keys, sms))
@@ -1069,7 +1073,7 @@ size_t bx_attention_workspace(int R, int HKV, int nblk, int bs, int variant) {
   const int sms = device_sms();
   if (R <= 0 || HKV <= 0 || nblk <= 0 || bs <= 0 || sms <= 0) return 0;
   const int64_t pairs = (int64_t)R * HKV, keys = (int64_t)nblk * bs;
-  if ((variant == 7 || (variant == 0 && split_auto(pairs, keys))) && split_can(R, HKV, keys, bs, sms)) {
+  if ((variant == 7 || (variant == 0 && split_auto(pairs, keys, false))) && split_can(R, HKV, keys, bs, sms)) {
     // room for the streaming kernel too: a cache that no tensor map can describe, or a forced cluster size, takes another kernel
     const size_t even = split_bytes(pairs, keys, sms), other = bx_attention_scratch_bytes(nblk, bs);
     return variant == 7 || pairs < STREAM_PAIRS || even > other ? even : other;

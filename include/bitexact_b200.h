@@ -250,7 +250,7 @@ int bx_int8_attention_ws(const int32_t* q, const int64_t* qpos, const int8_t* ca
  * row distance before the product with factor; window, slack and mtop as described there. A tab that does not start on a
  * 16-byte boundary is not used. Bit 8 of shift (exact rule): from byte 16400 of tab on lie the 257 doubles of which every table
  * entry is a product (`products` there), which the kernels use in place of the entries where the 32-bit word in front of them is 1,
- * and the full table where it is not. */
+ * and the full table where it is not: to be set only for tables that are such products, others keep the entries. */
 typedef struct {
   const uint32_t* tab;
   uint32_t window, slack, factor, mtop;

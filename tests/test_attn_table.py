@@ -163,3 +163,44 @@ def test_products_are_the_tables_they_stand_for():
     assert attn_table.products(other) is None
     a, b = attn_table.exact(lut, L2E)[0], attn_table.exact(other, L2E)[0]
     assert a.shape == b.shape and int(a[4099]) == 1 and int(b[4099]) == 0
+
+
+def halved(lut):
+    """A table with a compact form that is none of products."""
+    return (lut >> 1) + (1 << 58)
+
+
+def test_tables_of_another_kind_keep_their_entries():
+    lut = exp2_table("cpu").long()
+    assert attn_table.native(attn_table.exact(lut, L2E)).shift == 257
+    form = attn_table.exact(halved(lut), L2E)
+    assert attn_table.native(form).shift == 1 and attn_table.native(attn_table.to(form, "cpu")).shift == 1
+    i, tab = torch.arange(16384), form[0][:attn_table.ENTRIES].long()
+    for rr in (0, 1, 2047, 4095):                                # the window holds for what the kernels then read
+        v = halved(lut)[i] + (((halved(lut)[i + 1] - halved(lut)[i]) * rr + (1 << 11)) >> 12)
+        w = attn_table._walk(tab, i * 4096 + rr)
+        assert bool((w << 29 <= v).all()) and bool((v <= w + form[1] << 29).all()), rr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("R,nblk", [(37, 4), (37, 37), (37, 85), (38, 150), (37, 261), (4, 261)])
+def test_entries_of_an_exact_table_that_is_none_of_products(R, nblk):
+    """The streaming kernel reads them, the others the full table; on both sides of where the split takes over."""
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
+    HKV, M, bs, nb = 8, 4, 16, 301
+    g = torch.Generator().manual_seed(R * nblk)
+    rng = lambda lo, hi, *n: torch.randint(lo, hi, n, generator=g)
+    cache = tri_paged.to_limbs((rng(-(1 << 18), 1 << 18, nb, HKV, bs, 128) >> rng(0, 4, nb, 1, 1, 1)).int()).cuda()
+    bt, pos = rng(1, nb, R, nblk).int().cuda(), rng(0, nblk * bs, R, 1)
+    pos[0] = nblk * bs - 1
+    qpos = (pos - rng(0, 3, R, M)).clamp(min=0).cuda()
+    q = (rng(-(1 << 20), 1 << 20, R, HKV, M, 64) >> rng(0, 6, R, HKV, M, 1)).int().cuda()
+    sh = (-6 - rng(10, 20, R, HKV, M)).cuda()
+    lut = halved(exp2_table("cuda").long())
+    form = attn_table.to(attn_table.exact(lut, L2E), "cuda")
+    run = lambda c, var: tri_exact_attn.attend(q, sh, qpos, cache, bt, None, lut, L2E, variant=var, compact=c)
+    want = run(None, 3)
+    for c, var in ((form, 0), (form, 5), (form, 6), (form, 3), (form, 7), (None, 0)):
+        got = run(c, var)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), var
+    assert want[1].unique().numel() > 1
