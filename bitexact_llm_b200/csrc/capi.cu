@@ -1057,7 +1057,10 @@ int bx_exact_attention(const int32_t* q, const int64_t* sh, const int64_t* qpos,
 
 int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table) {
   if (R < 0 || HKV <= 0 || nblk <= 0 || bs <= 0) return BX_EARG;
-  const StreamPlan p = stream_auto((int64_t)R * HKV, (int64_t)nblk * bs, bs, scratch != 0, table ? CT_BYTES : 0);
+  const int64_t pairs = (int64_t)R * HKV, keys = (int64_t)nblk * bs;
+  const int sms = device_sms();
+  if (scratch == 2 && R > 0 && split_auto(pairs, keys, table == 3) && split_can(R, HKV, keys, bs, sms > 0 ? sms : 148)) return 7;
+  const StreamPlan p = stream_auto(pairs, keys, bs, scratch != 0, table == 2 ? PW_EXACT_BYTES : table ? CT_BYTES : 0);
   return p.per_sm == 0 ? 0 : 1000 * p.chunked + 100 * p.warps + 10 * p.per_sm + p.table;
 }
 

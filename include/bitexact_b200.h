@@ -267,9 +267,12 @@ int bx_int8_attention_tab(const int32_t* q, const int64_t* qpos, const int8_t* c
                           int HD, int cluster_size, int variant, void* scratch, size_t scratch_bytes,
                           const bx_compact_table* compact, void* stream);
 
-/* What variant 0 of the attention calls runs for R x HKV (request, KV head) pairs and block tables of nblk pages of bs keys, with
- * `scratch` and the compact `table` or without, on a cache that tensor maps can describe: 0 the cluster kernels, else the
- * streaming kernel as 1000 (contexts in chunks, scores in scratch) + 100 x warps + 10 x CTAs per SM + 1 (it uses the table). bx_attention_stream_pairs: pairs below which it is always 0. */
+/* What variant 0 of the attention calls runs for R x HKV (request, KV head) pairs and block tables of nblk pages of bs keys, on a cache
+ * that tensor maps can describe: 7 the even split, 0 the cluster kernels, else the streaming kernel as 1000 (contexts in chunks, scores
+ * in scratch) + 100 x warps + 10 x CTAs per SM + 1 (its CTAs hold the table's form). scratch: 0 none, 1 enough for the streaming
+ * kernel's chunks and too little for the split, 2 what bx_attention_workspace asks for. table: 0 without a compact form, 1 int8 mode's
+ * entries, 2 the products of exact mode, 3 the entries of an exact table that is none of products.
+ * bx_attention_stream_pairs: pairs below which the streaming kernel is never chosen. */
 int bx_attention_plan(int R, int HKV, int nblk, int bs, int scratch, int table);
 int bx_attention_stream_pairs(void);
 

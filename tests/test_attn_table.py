@@ -82,12 +82,44 @@ def test_where_the_automatic_choice_uses_the_table():
     assert plan(36, 784, 1) == 0 and nv.lib().bx_attention_stream_pairs() == 296
 
 
+def test_where_the_automatic_choice_splits():
+    """With the scratch that bx_attention_workspace asks for: the split on both sides of its widths, what it cannot hold, and what
+    an exact table without products takes in its place; the products' 2 KB leave room where 16 KB do not."""
+    from bitexact_llm_b200 import _native as nv
+    plan = lambda R, keys, table, HKV=8, bs=16: nv.lib().bx_attention_plan(R, HKV, keys // bs, bs, 2, table)
+    assert [plan(37, keys, 1) for keys in (592, 832, 896, 912, 1360, 2400, 8192)] == [821, 821, 820, 7, 7, 7, 7]
+    assert [plan(128, keys, 1) for keys in (512, 528)] == [440, 7] and [plan(24, keys, 1) for keys in (896, 912)] == [0, 7]
+    assert [plan(16, keys, 1) for keys in (1280, 1296)] == [0, 7] and [plan(8, keys, 1) for keys in (2048, 2064)] == [0, 7]
+    assert [plan(1, keys, 0) for keys in (3072, 3088)] == [0, 7]
+    assert [plan(512, 1040, 1, 1), plan(513, 1040, 1, 1), plan(64, 43200, 1), plan(64, 2048, 1, 8, 128)] == [7, 820, 1821, 0]
+    assert [plan(37, keys, 3) for keys in (592, 1360, 2416, 4160, 4176)] == [821, 421, 1821, 1821, 7] and plan(36, 1360, 3) == 7
+    assert [plan(37, keys, 2) for keys in (64, 80, 512, 528, 592, 848, 896)] == [441, 441, 441, 440, 821, 821, 821]
+
+
+def only_streaming(monkeypatch):
+    """Variant 0 gets enough scratch for the streaming kernel's chunks, and less than the split asks for."""
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn
+
+    def scratch(device, R, HKV, nblk, bs, variant):
+        n = R * HKV * ((nblk * bs + 63) // 64) * 64 * 32
+        return torch.empty(n, dtype=torch.uint8, device=device), n
+    monkeypatch.setattr(tri_exact_attn, "_scratch", scratch)
+
+
+def launches(run):
+    from bitexact_llm_b200 import _native as nv
+    before = nv.lib().bx_launch_count()
+    out = run()
+    return out, nv.lib().bx_launch_count() - before
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("R,nblk", [(37, 1), (75, 4), (37, 37), (40, 52), (37, 85), (41, 118), (37, 151), (38, 300)])
 @pytest.mark.parametrize("mode", ["exact", "int8"])
-def test_streaming_kernel_with_the_table_equals_the_oracle(mode, R, nblk):
-    """Every form of the streaming kernel that uses the table by itself (both ends of each band of widths), and the forced
-    ones: the full table's integers for all pairs, the CPU oracle's for some; contexts of 1 key up to the whole table."""
+def test_streaming_kernel_with_the_table_equals_the_oracle(mode, R, nblk, monkeypatch):
+    """Every form of the streaming kernel that uses the table by itself (both ends of each band of widths), the forced ones, and what
+    the automatic choice runs with all its scratch: the full table's integers for all pairs, the CPU oracle's for some; contexts of
+    1 key up to the whole table."""
     from bitexact_llm_b200 import _native as nv
     from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
     from oracle import exact as ox
@@ -121,16 +153,24 @@ def test_streaming_kernel_with_the_table_equals_the_oracle(mode, R, nblk):
         compact = attn_table.int8(ptab)
         want = o8.paged_attention(q[pick].long().numpy(), *rows[1:], pick, o8.exp_table())
     compact = attn_table.to(compact, "cuda")
-    num, den = run(compact)
-    for other in (run(None), run(compact, 5), run(compact, 6), run(None, 3)):
+    (num, den), count = launches(lambda: run(compact))
+    table = 2 if mode == "exact" else 1
+    assert count == (2 if nv.lib().bx_attention_plan(R, HKV, nblk, bs, 2, table) == 7 else 1)
+    with monkeypatch.context() as m:
+        only_streaming(m)
+        assert nv.lib().bx_attention_plan(R, HKV, nblk, bs, 1, table) % 10 == 1
+        streamed, count = launches(lambda: run(compact))
+        assert count == 1
+    for other in (streamed, run(None), run(compact, 5), run(compact, 6), run(None, 3)):
         assert torch.equal(num, other[0]) and torch.equal(den, other[1])
     assert np.array_equal(num.cpu().numpy()[pick], want[0])
     assert np.array_equal(den.cpu().numpy()[pick].reshape(want[1].shape), want[1])
 
 
 @pytest.mark.gpu
-def test_many_pairs_in_chunks_without_a_table():
-    """From 1024 pairs on 4-warp CTAs serve wide block tables for callers without a compact table."""
+def test_many_pairs_in_chunks_without_a_table(monkeypatch):
+    """From 1024 pairs on 4-warp CTAs serve wide block tables for callers without a compact table, where the split has too little
+    scratch."""
     from bitexact_llm_b200 import _native as nv
     from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
     R, HKV, M, bs, nblk, nb = 129, 8, 4, 16, 160, 200
@@ -144,9 +184,43 @@ def test_many_pairs_in_chunks_without_a_table():
     q, sh = rng(-(1 << 20), 1 << 20, R, HKV, M, 64).int().cuda(), (-6 - rng(12, 20, R, HKV, M)).cuda()
     run = lambda var: tri_exact_attn.attend(q, sh, qpos, cache, bt, None, exp2_table("cuda").long(), L2E, variant=var)
     num, den = run(0)
-    for var in (3, 5):
+    for var in (3, 5, 6):
         other = run(var)
         assert torch.equal(num, other[0]) and torch.equal(den, other[1])
+    only_streaming(monkeypatch)
+    other, count = launches(lambda: run(0))
+    assert count == 1 and torch.equal(num, other[0]) and torch.equal(den, other[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["exact", "int8"])
+@pytest.mark.parametrize("R,HKV,nblk", [(520, 1, 70), (513, 1, 160), (64, 8, 2700)])
+def test_what_the_split_cannot_hold(mode, R, HKV, nblk):
+    """More than 512 requests, or more than 1024 pages a CTA by table width: variant 0 streams, with and without a compact table."""
+    from bitexact_llm_b200 import _native as nv
+    from bitexact_llm_b200.vllm_plugin import tri_exact_attn, tri_paged
+    M, bs, nb = 4, 16, 200
+    g = torch.Generator().manual_seed(R + nblk)
+    rng = lambda lo, hi, *n: torch.randint(lo, hi, n, generator=g)
+    cache = tri_paged.to_limbs((rng(-(1 << 18), 1 << 18, nb, HKV, bs, 128) >> rng(0, 5, nb, 1, 1, 1)).int()).cuda()
+    bt, pos = rng(1, nb, R, nblk).int().cuda(), rng(0, min(nblk * bs, 1500), R, 1)
+    pos[3] = min(nblk * bs, 5000) - 1
+    qpos = pos.expand(-1, M).contiguous().cuda()
+    q, sh = rng(-(1 << 20), 1 << 20, R, HKV, M, 64).int().cuda(), (-6 - rng(12, 20, R, HKV, M)).cuda()
+    if mode == "exact":
+        lut = exp2_table("cuda").long()
+        form = attn_table.to(attn_table.exact(lut, L2E), "cuda")
+        run = lambda c, var: tri_exact_attn.attend(q, sh, qpos, cache, bt, None, lut, L2E, variant=var, compact=c)
+    else:
+        q >>= 7
+        ptab = consts8.weight_table(consts8.exp_table()).cuda()
+        form = attn_table.to(attn_table.int8(ptab), "cuda")
+        run = lambda c, var: tri_paged.attend(q, qpos, cache, bt, ptab, variant=var, compact=c)
+    want = run(None, 3 if nblk < 1000 else 5)
+    for c, table in ((form, 2 if mode == "exact" else 1), (None, 0)):
+        assert nv.lib().bx_attention_plan(R, HKV, nblk, bs, 2, table) > 100
+        got, count = launches(lambda: run(c, 0))
+        assert count == 1 and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
 def test_products_are_the_tables_they_stand_for():
