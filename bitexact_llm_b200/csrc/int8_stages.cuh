@@ -579,7 +579,6 @@ int8_silu_persistent_kernel(const i64* __restrict__ y, const i64* __restrict__ l
   extern __shared__ __align__(16) uint8_t silu_smem[];
   const uint16_t* tab = reinterpret_cast<const uint16_t*>(silu_smem);
   __shared__ i64 red[GROUPS][2][32];
-  __shared__ uint32_t redb[GROUPS][2][32];
   __shared__ uint64_t table_full;
   const int group = threadIdx.x / GT, t = threadIdx.x % GT;
   int turn = 0;

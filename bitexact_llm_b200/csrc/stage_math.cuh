@@ -15,7 +15,6 @@ namespace bx {
 
 constexpr double F2I = 6755399441055744.0;            // 1.5 2^52: v + F2I has the integer v in its low mantissa bits
 constexpr int F2I_HI = 0x43380000;                    // its high word (the low word is 0)
-constexpr double SURE = 9.5367431640625e-7;           // 2^-20
 
 // |x| < 2^51, exact.
 __device__ __forceinline__ double to_f64(i64 x) {
