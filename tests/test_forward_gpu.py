@@ -11,17 +11,17 @@ from bitexact_llm_b200 import _native as nv
 pytestmark = pytest.mark.gpu
 
 
-def engine(mode, width, layers, edit=lambda c: c):
+def engine(mode, width, layers, edit=lambda c: c, n_pos=700):
     from bitexact_llm_b200.exact import consts
     cfg = dict(consts.LLAMA_1B, hidden_size=width, intermediate_size=4 * width, num_hidden_layers=layers, num_attention_heads=width // 64,
                num_key_value_heads=width // 256, head_dim=64, vocab_size=512)
     sd = consts.random_state_dict(cfg, seed=width, device="cuda", gamma_jitter=0.1)
     if mode == "exact":
         from bitexact_llm_b200.vllm_plugin.exact_run import ExactEngine
-        return ExactEngine(edit(consts.build(cfg, sd, n_pos=700)), "cuda")
+        return ExactEngine(edit(consts.build(cfg, sd, n_pos=n_pos)), "cuda")
     from bitexact_llm_b200.int8 import consts as consts8
     from bitexact_llm_b200.int8.engine import IntEngine
-    return IntEngine(edit(consts8.build(cfg, sd, n_pos=700)), "cuda")
+    return IntEngine(edit(consts8.build(cfg, sd, n_pos=n_pos)), "cuda")
 
 
 def step(eng, ses, seqs, lens, tiles, native, form=True):
@@ -174,3 +174,67 @@ def test_feed_of_device_tokens():
             got = run(place, chunk_rows)
             assert all(torch.equal(a, b) for a, b in zip(want[:3], got[:3]))
             assert got[3] <= want[3]
+
+
+@pytest.mark.parametrize("mode", ["exact", "int8"])
+@pytest.mark.parametrize("B,keys", [(3, 3300), (48, 1000)])
+def test_decoding_in_wide_tables(mode, B, keys):
+    """The even split, whose scratch lies in the call's workspace, layer after layer over filled caches: few pairs and many."""
+    from bitexact_llm_b200.decode import Session
+    from bitexact_llm_b200.vllm_plugin import tri_paged
+    eng = engine(mode, 1024, 3, n_pos=keys)
+    ses = Session(eng, B, keys, perm_seed=1)
+    assert nv.lib().bx_attention_plan(B, eng.HKV, ses.nblk, ses.bs, 2, 2 if mode == "exact" else 1) == 7
+    g = torch.Generator(device="cuda").manual_seed(B)
+    lens = torch.randint(0, keys, (B,), generator=g, device="cuda")
+    lens[0] = keys - 1
+    seq = torch.repeat_interleave(torch.arange(B, device="cuda"), lens)
+    at = torch.arange(seq.shape[0], device="cuda") - torch.repeat_interleave(torch.cumsum(lens, 0) - lens, lens)
+    bits = (17, 19) if mode == "exact" else (14, 14)
+    for cache in ses.kvs:
+        k, v = (torch.round(torch.randn(seq.shape[0], eng.HKV, 64, generator=g, device="cuda") * 2.0 ** b).long() for b in bits)
+        tri_paged.store(cache, ses._slots(seq, at), k, v)
+    ids, out = torch.arange(B, device="cuda") * 7 % 512, []
+    for native in (False, True):
+        kvs = [c.clone() for c in ses.kvs]
+        with pytest.MonkeyPatch.context() as m:
+            if not native:
+                m.setattr(type(eng), "_forward_native", lambda *a: None)
+            before = nv.lib().bx_launch_count()
+            out.append((eng.forward(kvs, ids, lens, ses._slots(ses.rows, lens), ses.bt, ses.rows), nv.lib().bx_launch_count() - before, kvs))
+    assert torch.equal(out[0][0], out[1][0]) and out[0][1] == out[1][1]
+    assert all(torch.equal(a, b) for a, b in zip(out[0][2], out[1][2]))
+    eng.check()
+
+
+@pytest.mark.parametrize("mode,bound", [("exact", "wqkv"), ("exact", "wgu"), ("exact", "wd"), ("int8", "keys"), ("int8", "products")])
+def test_a_bound_in_the_middle_layer_sets_the_flag(mode, bound):
+    """Keys, values or products beyond their bounds in one layer of three; the product bound of int8 mode, which only the end of the
+    call looks at, by itself. Without the edit there is no flag."""
+    from bitexact_llm_b200.decode import Session
+    from bitexact_llm_b200.vllm_plugin import tri_fuse
+    eng = engine(mode, 256, 3)
+    ses = Session(eng, 2, 64, perm_seed=1)
+    run = lambda native: step(eng, ses, [0, 1], [3, 5], False, native)
+    assert run(True)[2] == 0 and run(False)[2] == 0
+    ly = eng.layers[1]
+    if mode == "exact":
+        ly[bound].g += 30
+    elif bound == "keys":
+        ly["ga"] <<= 12
+    else:
+        w, mul, fmsh = ly["wd"]
+        ly["wd"], gamma = (w, mul, fmsh + 28), ly["gm"].clone()
+        with pytest.MonkeyPatch.context() as m:                  # the maxima at 2^12 times the gamma, and the gamma for 2^62.5
+            m.setattr(tri_fuse, "flag_end", lambda *a: None)
+            ly["gm"] = gamma << 12
+            assert run(False)[2] == 0
+            s, u = eng.scr[1].tolist()
+            ly["gm"] = gamma * int(2.0 ** 12 * (2.0 ** 62.5 / (s * u)) ** 0.5)
+            eng.scr.zero_()
+            assert run(False)[2] == 0                            # nothing else sets the flag
+            s, u = eng.scr[1].tolist()
+            assert 1 << 62 <= s * u < 1 << 63
+            eng.scr.zero_()
+    loop, native = run(False), run(True)
+    assert loop[2] == native[2] == 1 and torch.equal(loop[0], native[0])
