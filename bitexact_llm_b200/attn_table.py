@@ -10,8 +10,8 @@ In exact mode the doubles of which the entries of a 2^-f table are products (2 K
 entries where the table is one of products; any other table keeps the entries.
 
 compact = (int32 tensor of the entries, in exact mode with room for the products behind them, window, slack, factor from a row
-distance to t, its left shift (and ENTRIES_ONLY where there are no products behind the entries of exact mode), 2^(top + 1)): window in
-units of the interpolated entry, slack (for a table that was itself rounded) in units of 2^-32 of a weight."""
+distance to t, its left shift, 2^(top + 1)): window in units of the interpolated entry, slack (for a table that was itself rounded) in
+units of 2^-32 of a weight; an EntriesOnly where exact mode's table is none of products."""
 
 import ctypes
 
@@ -20,7 +20,10 @@ import torch
 T_BITS, W_BITS = 26, 31                # fractional bits of t, bits of an entry
 STEP = 1 << 14                         # t steps per segment: 4096 segments
 ENTRIES = 4097
-ENTRIES_ONLY = 1 << 9                  # in `shift`: the room behind the entries is empty
+
+
+class EntriesOnly(tuple):
+    """A compact form of exact mode without products: the room behind the entries is empty, and the kernels are told so."""
 
 
 class Native(ctypes.Structure):
@@ -30,8 +33,8 @@ class Native(ctypes.Structure):
 
 def native(compact):
     tab, window, slack, factor, shift, mtop = compact
-    products = tab.shape[0] > ENTRIES and not shift & ENTRIES_ONLY
-    return Native(tab.data_ptr(), window, slack, factor, mtop, (shift & 255) | (256 if products else 0))
+    products = tab.shape[0] > ENTRIES and not isinstance(compact, EntriesOnly)
+    return Native(tab.data_ptr(), window, slack, factor, mtop, shift | (256 if products else 0))
 
 
 def products(lut):
@@ -51,7 +54,7 @@ def _with_products(tab, t):
 
 
 def to(compact, device):
-    return None if compact is None else (compact[0].to(device), *compact[1:])
+    return None if compact is None else type(compact)((compact[0].to(device), *compact[1:]))
 
 
 def _walk(tab, t):
@@ -79,7 +82,8 @@ def exact(lut, l2e):
     if not _fits(tab) or hi - lo > 60:
         return None
     t = products(v)
-    return _with_products(tab.to(torch.int32), t), hi - lo + 3, 0, int(l2e) * 8, 1 if t is not None else 1 | ENTRIES_ONLY, 1 << 23
+    form = _with_products(tab.to(torch.int32), t), hi - lo + 3, 0, int(l2e) * 8, 1, 1 << 23
+    return form if t is not None else EntriesOnly(form)
 
 
 def int8(ptab):
