@@ -30,8 +30,8 @@ class TokenRowEngine:
 
     def forward_native(self, call, exact, fields, layers, shapes, kvs, ids, pos, slot, bt, rmap, tiles):
         """All layers' kernels from one call of the library (`bx_exact_forward`, `bx_int8_forward`): fields of bx_step beside the common
-        ones, layers a flat list of what a bx_*_layer holds in front of its cache, one list per layer, shapes the (rows, columns) of its
-        four matrices. Returns the residual rows, or None where the call's geometry is not what that entry takes (the engines then run
+        ones, layers a flat list of what a bx_*_layer holds in front of its cache, one list per layer, shapes the rows and columns of
+        its four matrices. Returns the residual rows, or None where the call's geometry is not what that entry takes (the engines then run
         their own loop)."""
         import ctypes
 
@@ -39,8 +39,8 @@ class TokenRowEngine:
         N, G, dev = ids.shape[0], self.H // self.HKV, ids.device
         if N == 0 or self.HD != 64 or G > 4 and tiles is None or len(kvs) < self.L or tiles is not None and tiles.shape[0] == 0:
             return None
-        FF = shapes[0][2][0] // 2                                # of the weights: a config need not name it
-        if any(sh != [((self.H + 2 * self.HKV) * self.HD, self.D), (self.D, self.H * self.HD), (2 * FF, self.D), (self.D, FF)] for sh in shapes):
+        FF = shapes[0][4] // 2                                   # of the weights: a config need not name it
+        if shapes.count(((self.H + 2 * self.HKV) * self.HD, self.D, self.D, self.H * self.HD, 2 * FF, self.D, self.D, FF)) < len(shapes):
             return None
         bs, flat = kvs[0].shape[2], []
         for c, layer in zip(kvs, layers):

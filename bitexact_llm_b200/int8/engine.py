@@ -88,12 +88,11 @@ class IntEngine(TokenRowEngine):
             return None                                          # a timer brackets every linear, another _lin is to be called for each
         rows, shapes = [], []
         for ly in self.layers[:self.L]:
-            row, sh = [], []
+            row = []
             for n in ("wqkv", "wo", "wgu", "wd"):
                 w, mul, fmsh = ly[n]
                 row += (w.data_ptr(), mul.data_ptr(), int(fmsh), w.shape[0], w.shape[1])
-                sh.append((w.shape[0], w.shape[1]))
-            shapes.append(sh)
+            shapes.append((row[3], row[4], row[8], row[9], row[13], row[14], row[18], row[19]))
             rows.append(row + [ly["ga"].data_ptr(), ly["gm"].data_ptr()])
         form = None if self.compact is None else attn_table.native(self.compact)       # lives until the call has read it
         fields = dict(ptab=self.ptab.data_ptr(), silu=self.silu_t.data_ptr(), silu_compact=nv.ptr(self.silu_c), scr=self.scr.data_ptr(),

@@ -92,20 +92,19 @@ class ExactEngine(TokenRowEngine):
         return x
 
     def _forward_native(self, kvs, ids, pos, slot, bt, rmap, tiles):
-        layers = self.layers[:self.L]
         if self.D & (self.D - 1) or not 32 <= self.D <= 4096 or rmap is None:
             return None
-        if any(type(ly[n]) is not FusedLin or ly[n].timer is not None for ly in layers for n in ("wqkv", "wo", "wgu", "wd")):
-            return None                                          # another callable, or a timer that brackets every linear by itself
         ptr, rows, shapes = nv.ptr, [], []
-        for ly in layers:
+        for ly in self.layers[:self.L]:
             row = []
             for n in ("wqkv", "wo", "wgu", "wd"):
                 w = ly[n]
+                if type(w) is not FusedLin or w.timer is not None:
+                    return None                                  # another callable, or a timer that brackets every linear by itself
                 row += (w.limbs.data_ptr(), w.d.data_ptr(), w.g.data_ptr(), ptr(w.cnt) or 0, ptr(w.ec) or 0, ptr(w.ev) or 0, w.R, w.N, w.K, w.cfg or 0)
             row += (ly["ga"][0].data_ptr(), ly["ga"][1].data_ptr(), ly["gm"][0].data_ptr(), ly["gm"][1].data_ptr())
             rows.append(row)
-            shapes.append([(ly[n].N, ly[n].K) for n in ("wqkv", "wo", "wgu", "wd")])
+            shapes.append((row[7], row[8], row[17], row[18], row[27], row[28], row[37], row[38]))
         form = None if self.compact is None else attn_table.native(self.compact)       # lives until the call has read it
         fields = dict(lut=self.exp2.data_ptr(), l2e=int(self.l2e), compact=None if form is None else ctypes.addressof(form))
         return self.forward_native("bx_exact_forward", True, fields, rows, shapes, kvs, ids, pos, slot, bt, rmap, tiles)
