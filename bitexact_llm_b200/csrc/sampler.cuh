@@ -276,9 +276,11 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
     const u128 jm = {PCG_STEPS.e[SAMPLE_THREADS].mult_hi, PCG_STEPS.e[SAMPLE_THREADS].mult_lo}, jp = seeded[2];
     const u64 dv = (u64)(2 * tn);
     const u64 inv = ~0ull / dv;
-    // logits below 2^51 (a whole double) and 2^60 / td in size: |2 l td + tn| does not wrap
+    // logits below 2^51 (a whole double) and 2^60 / td, and down to about -2^62 / td, where 2 l td + tn does not wrap: below -2^51 the
+    // bound takes -2^51 in their place (masked entries; evaluated one by one, 9 of 10 at -2^55 took 409 us for 256 rows, pruned 142)
     const bool prunable = tn > 0 && tn < (1ll << 30) && td >= 0 && td < (1ll << 27);
-    const int bound = prunable ? min(51, 60 - bitlen(td)) - 32 : 0;
+    const int width = prunable ? 28 - bitlen(td) : 0;
+    const uint32_t below = 4u << width, span = prunable ? below + (1u << min(width, 19)) : 0;
     const double ratio = (double)td / (double)tn;
     int mine = (int)0x80000000;
     const auto order = [](int b) { return b ^ (b >> 31 & 0x7fffffff); };      // a float's bits <-> a whole number of its order
@@ -306,8 +308,9 @@ sample_part_kernel(const i64* __restrict__ logits, int64_t ld, const i64* __rest
         const uint32_t ones = ~(uint32_t)(w >> 32);
         const int j = ones ? __clz(ones) + 1 : 40;             // 1 - u in [2^-j, 2^-(j-1)), or below 2^-32
         bool pass = act;
-        if (prunable && (uint32_t)(lg[k] >> 32) + (1u << bound) < 2u << bound) {
-          const double t = to_f64(lg[k]) * ratio;
+        const int hi = (int)(lg[k] >> 32);
+        if ((uint32_t)hi + below < span) {
+          const double t = (__hiloint2double(max(hi, -(1 << 19)) + F2I_HI, (int)lg[k]) - F2I) * ratio;
           pass &= !(fma(fabs(t), 8.881784197001252e-16, t) + gtab[j] < floor_);
         }
         if (__any_sync(0xffffffffu, pass)) {

@@ -88,3 +88,24 @@ def test_apply_forces_the_integer_token(tmp_path):
     finally:
         S.STASH.active, S.STASH.logits, S.STASH.head, S.STASH.lnt, S.STASH.fr = old
         S.STASH.sampler = None
+
+
+@pytest.mark.parametrize("td,tn", [(10, 7), (1, 1), (100, 3), ((1 << 27) - 1, (1 << 30) - 1), (1 << 27, 5), (0, 4)])
+def test_masked_logits(td, tn):
+    """Entries about and far below -2^51, where the pruning bound changes its form, down to where 2 l td wraps and beyond: few left,
+    all masked alike, all masked to sizes of their own."""
+    from bitexact_llm_b200.exact.consts import ln_table
+    from bitexact_llm_b200.vllm_plugin import sampler as S
+    rng, V, lnt_np = np.random.RandomState(tn), 3000, ox.ln_table()
+    lim = (1 << 62) >> td.bit_length()                           # down to -lim nothing wraps
+    masks = [-(1 << 40), -(1 << 51) + 1, -(1 << 51), -(1 << 51) - 1, -(1 << 55), -lim, -lim - 1, -lim - (1 << 32), -(1 << 62), -(1 << 63), 1 << 51, (lim >> 2) - 1, lim >> 2, lim >> 1]
+    logits = rng.randint(-(20 << 24), 20 << 24, (2 * len(masks) + 1, V)).astype(np.int64)
+    for i, m in enumerate(masks):
+        logits[2 * i] = np.where(rng.rand(V) < 0.05, logits[2 * i], m)
+        logits[2 * i + 1] = m
+    logits[-1] = np.array(masks)[rng.randint(0, len(masks), V)]
+    n = len(logits)
+    with np.errstate(over="ignore"):
+        want = _want(logits, list(range(n)), [5] * n, [(tn, td)] * n, lnt_np, 24)
+    got = S.integer_sample(torch.from_numpy(logits).cuda(), range(n), [5] * n, [(tn, td)] * n, ln_table(device="cuda"))
+    assert got.tolist() == want
