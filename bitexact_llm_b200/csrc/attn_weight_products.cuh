@@ -2,10 +2,11 @@
 //
 // Both weight tables are exponentials, so an entry is the product of two of 128 (exact rule: 2^-f in steps of 2^-7 and 2^-14) or of
 // 512 and 256 (int8 rule: e^z in steps of 2^-4 and 2^-12) doubles in shared memory, 2 and 6 KB for 131 and 524, and a weight
-// is known to 2^-27 (exact rule) or to the 2^-11 that its table was rounded by before (int8 rule). Nearer to a rounding boundary than
-// 2^-21 / 2^-10 the table itself decides. A table is known to be of this kind because every entry was held against the products: by the
-// caller that prepared them (attn_table.py, the kernels that give a pair to a CTA or a cluster), or by the first kernel of the split
-// decode attention, a slice per CTA. A table of another kind takes the general rule.
+// is known to 2^-27 (exact rule) or to the 2^-11 that its table was rounded by before (int8 rule). From 2^-22 below a rounding boundary
+// to 2^-21 above it (exact rule), or within 2^-9 of it (int8 rule), the table itself decides. A table is known to be of this kind
+// because every entry was held against the products: by the caller that prepared them (attn_table.py, the kernels that give a pair to
+// a CTA or a cluster), or by the first kernel of the split decode attention, a slice per CTA. A table of another kind takes the general
+// rule.
 // Measured in the second kernel of the split attention, 32 sequences of 64 .. 8192 keys: 85 us with the 4097 entries of
 // attn_weight_tables.cuh, which leave 1 % of the weights near the maximum undecided (most warps then gather from L2), 66 us so.
 #pragma once

@@ -771,7 +771,8 @@ static StreamPlan stream_plan(int NW, int64_t max_keys, bool chunked, int table)
   if (p.per_sm < 1) return p;
   // The compact weight table where it costs neither a CTA nor the ring: 256 sequences of 512 .. 768 keys 155 -> 133 us; a
   // step that had to give up CTAs for it (and the cluster kernels, five small CTAs to an SM) lost up to 35 %. With
-  // pages of 16 keys that is: tables of up to 64 keys, 592 .. 832, 1360 .. 1888, and all that are chunked.
+  // pages of 16 keys that is: tables of up to 64 keys, 592 .. 832, 1360 .. 1888, and all that are chunked; for the 2 KB of products
+  // up to 512 keys, 592 .. 1280, 1360 .. 2336, and all that are chunked.
   p.table = table && stages(fixed + table) >= 4;
   if (p.table) {
     fixed += table;
@@ -872,9 +873,10 @@ static bool split_can(int64_t R, int64_t HKV, int64_t max_keys, int bs, int sms)
 // Where the automatic choice splits evenly, by what the host knows: pairs and the width of the block tables. The two kernels cost about
 // 9 us more than one on the smallest batches and serve every mix of lengths alike (us, before : split, 8 KV heads: 32 sequences of
 // 64 .. 8192 keys 223 : 110, 64 of 16 .. 4096 145 : 119, 100 of 100 .. 1500 111 : 84, 256 of 500 .. 1400 254 : 184, 256 of
-// 512 .. 768 145 : 138, of 500 .. 620 129 : 119; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27). Narrower tables stay with the kernels that give
-// a pair to a CTA or a cluster (64 of 16 .. 600 37 : 45, 256 of 16 .. 200 59 : 70), and so do few pairs of up to 3072 keys (4 of 2000 25 : 27).
-// Contexts much shorter than wide tables pay for it (64 of 16 .. 100 keys in 4096 25 : 30, 32 of the same 47 : 25).
+// 512 .. 768 145 : 138, of 500 .. 620 129 : 119; 16 of 500 .. 1400 35 : 33; one of 4000 / 8000 keys 27 : 23, 39 : 27; 72 of 64 .. 8192
+// 265 : 224; pages of 64 keys, which the streaming kernel does not take, 200 of 64 .. 8192 968 : 562). Narrower tables stay with the
+// kernels that give a pair to a CTA or a cluster (64 of 16 .. 600 37 : 45, 256 of 16 .. 200 59 : 70), and so do few pairs of up to 3072
+// keys (4 of 2000 25 : 27). Contexts much shorter than wide tables pay for it (64 of 16 .. 100 keys in 4096 23 : 28, 32 of the same 47 : 25).
 // entries: the caller's exact table has a compact form but no products, which leaves every weight of the split to the full table; the
 // streaming kernel has the entries (us, stream : split: 64 sequences of 16 .. 4096 keys 137 : 167, 100 of 100 .. 1500 109 : 122, 256 of
 // 512 .. 768 138 : 175, of 500 .. 1400 254 : 247; 48 of 64 .. 8192 221 : 208).

@@ -600,7 +600,8 @@ __device__ __noinline__ void attn_out_row(const i64* num, const i64* den, int32_
 // One row per CTA; a thread has four consecutive entries of one head (HD is a multiple of four) and Q such groups.
 // o = floor(32 num / den + 1/2): num is one rounding (its halves are exact), 32 / den another and the product a third, so
 // for |o| < 2^29 the quotient is known to 2^-21; nearer to a boundary than 2^-20 the integer division decides.
-// 3750 rows of 2048: 66 -> 26 us (4.5 TB/s), 256 rows 6.7 -> 4.1 us, one row 3.9 -> 2.1 us.
+// 3750 rows of 2048: 66 -> 26 us (4.5 TB/s), 256 rows 6.7 -> 4.1 us, one row 3.9 -> 2.1 us; with an entry from 32 on in every row,
+// which takes the integer rule for the row, 72 -> 106 us.
 template <int NT, int Q>
 __global__ void __launch_bounds__(NT)
 attn_out_kernel(const i64* __restrict__ num, const i64* __restrict__ den, int32_t* __restrict__ q,
@@ -830,7 +831,8 @@ silu_cluster_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int3
 // thread. The table gathers are what the other forms wait for (they miss L1); from shared memory they cost a few cycles, and a
 // CTA fetches the table once for all its rows. 23 bytes and 117 warp instructions per 32 elements. FF % 4 == 0, FF <= 4 GT Q.
 // 3750 rows of 8192: 275 -> 164 us (4.3 TB/s), of 14336 1875 rows 405 -> 155 us; 256 rows of 8192 25.2 -> 17.5 us. ncu: issue 63 %, waits for
-// loads (64 registers hold no second row; asking for the next row's lines in L2 cost 20 %).
+// loads (64 registers hold no second row and spill 124 bytes; asking for the next row's lines in L2 cost 20 %). Arguments beyond 64
+// take the general form one by one: 1875 rows of 8192 98 us, 106 with one in 1000 of them, 150 with one in 100 (148 before).
 constexpr int SILU_P_THREADS = 1024;
 constexpr int SILU_TABLE = (1 << EXP2_BITS) + 1;
 

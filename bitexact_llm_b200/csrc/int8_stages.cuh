@@ -511,7 +511,9 @@ int8_silu_kernel(const i64* __restrict__ y, const i64* __restrict__ lut, int8_t*
 
 // The compact SiLU table (bitexact_llm_b200/int8/consts.py: silu_compact): max(x, 0) - silu(x) of the table's entries for
 // |x| <= 8, 65537 x 16 bits (131 KB instead of 2 MB), which fits beside the rows of an SM. 1875 rows of 8192 (18 bytes an element):
-// 152 -> 84 us, of 14336 405 -> 128 us, 64 rows of 8192 20.8 -> 9.6 us, one row 12.7 -> 4.3 us.
+// 152 -> 84 us (3.3 TB/s), of 14336 405 -> 128 us, 64 rows of 8192 20.8 -> 9.6 us, one row 12.7 -> 4.3 us. With 10 % of the arguments
+// beyond 8, which go to the full table one by one, 1875 rows of 8192 158 -> 139 us. 64 registers a thread spill 192 bytes and load
+// 420 (two rows at a time).
 constexpr int SC_HALF = 8 << FA, SC_N = 2 * SC_HALF + 1, SC_BYTES = (SC_N * 2 + 15) / 16 * 16;
 
 struct SiluAcc {
