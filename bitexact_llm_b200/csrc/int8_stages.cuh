@@ -642,6 +642,7 @@ int8_silu_persistent_kernel(const i64* __restrict__ y, const i64* __restrict__ l
       atomicMax(reinterpret_cast<long long*>(scr + 1), (long long)u);
     }
   }
+  if (!there) mbar_wait(&table_full, 0);                       // a copy that is late lands before the CTA ends
 }
 
 // Decode batches: the columns of a row over the CTAs of a cluster (256 threads, Q groups of four columns each), the compact

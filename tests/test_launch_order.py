@@ -41,6 +41,18 @@ def test_weight_tiles_are_requested_behind_the_wait_unless_asked_for_early():
     assert seen == 3
 
 
+def test_a_late_copy_lands_before_its_cta_ends():
+    """Whoever copies into shared memory without a tensor map waits for the copy once more at its end where the first wait ran out."""
+    src = _integer_sources()
+    kernels = {m.group(1): m.group(0) for f in ("int8_stages.cuh", "paged_attention.cuh")
+               for m in re.finditer(r"__global__ .*?(\w+)\(.*?^}", re.sub(r"__launch_bounds__\([^)]*\)*", "", src[f]), re.S | re.M)
+               if "bulk_load(" in m.group(0) or "fetch_compact(" in m.group(0)}
+    assert sorted(kernels) == ["exact_attention_stream_kernel", "int8_silu_persistent_kernel"]
+    for name, body in kernels.items():
+        again = re.search(r"if \(!(there|table)\) (mbar_wait\(&table_full, 0\)|wait_table\(\));", body[body.rindex("for (int64_t"):])
+        assert again, name
+
+
 def test_only_the_engines_ask_for_weights_early(monkeypatch):
     from bitexact_llm_b200 import _native as nv
     from bitexact_llm_b200.exact.model import Lin
