@@ -25,7 +25,7 @@ def tile_table(pre, G, bm=BM):
 def cut_runs(pre, n):
     """[T, 3] int32 (request, first token, tokens): the runs of pre = [(req, tok0, qlen, seq_len)], any iterable of rows of whole
     numbers, in pieces of n tokens."""
-    run = torch.tensor([(int(r), int(t0), max(int(ql), 0)) for r, t0, ql, _ in pre], dtype=torch.int32).reshape(-1, 3)
+    run = torch.tensor([(r, t0, ql if ql > 0 else 0) for r, t0, ql, _ in pre], dtype=torch.int32).reshape(-1, 3)
     pieces = (run[:, 2] + n - 1) // n
     out = torch.repeat_interleave(run, pieces, dim=0)
     at = n * (torch.arange(out.shape[0], dtype=torch.int32) - torch.repeat_interleave(torch.cumsum(pieces, 0).int() - pieces, pieces))
