@@ -33,6 +33,7 @@ class IntEngine(TokenRowEngine):
         lin = lambda k: (t(k), t(f"{k}.m"), int(c[f"{k}.fm"]) + 8 * (nl - 1) - 24)
         self.layers = [{"ga": t(f"{i}.ga"), "gm": t(f"{i}.gm"), **{n: lin(f"{i}.{n}") for n in ("wqkv", "wo", "wgu", "wd")}}
                        for i in range(self.L)]
+        self.FF = self.layers[0]["wgu"][0].shape[0] // 2 if self.layers else cfg.get("intermediate_size", 8192)
         self.gf, self.lm = t("gf"), lin("lm")
         self.silu_t, self.cos, self.sin, self.ln = t("silu"), t("cos"), t("sin"), t("ln")
         self.silu_c = silu_compact(self.silu_t)              # the stage kernels' form of it

@@ -100,6 +100,7 @@ def test_the_feed_forward_width_is_that_of_the_weights(mode):
         got = []
         for edit in (unnamed, lambda c: c):
             eng = engine(mode, 256, 2, edit)
+            assert mode == "exact" or eng.FF == 1024
             got.append(step(eng, Session(eng, 2, 640, perm_seed=1), [1], [n], n > 500, True))
         assert torch.equal(got[0][0], got[1][0]) and got[0][3] == got[1][3]
 
